@@ -68,51 +68,74 @@ struct AlphaArgs {
 
 // ---- small dense helpers for the projected tridiagonal (double, one CTA) --------------------
 
-// Biased exponent of a double (integer pipe: the recurrences below test signs and magnitudes on
-// the bit pattern, keeping double compares off their dependency chains).
-__device__ __forceinline__ int dexp_bits(double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7FF); }
+// A tridiagonal as its recurrences read it, in shared memory: row i is {a_i, b_{i-1}^2} (b_{-1} = 0),
+// padded to a multiple of kTriBlock rows with {2^60, 0}: such a row multiplies both minors by a
+// positive number and takes no part in a sign count.
+constexpr int kTriBlock = 8;
+constexpr int kTriPad = kNcvMax + kTriBlock;
+__host__ __device__ constexpr int tri_blocks(int m) { return (m + kTriBlock - 1) / kTriBlock; }
 
-// Number of eigenvalues of the tridiagonal (a, b; size m) below x: sign changes of the leading
-// principal minors det(T_k - x I), computed with the three-term recurrence. The pair (p_k, p_k-1) is
-// rescaled by exact powers of two every 4 steps when its exponent leaves [2^-500, 2^500] (four steps
-// of entries bounded by the Gershgorin radius cannot leave the double range from there).
-__device__ inline int sturm_count(const double* a, const double* b, int m, double x) {
-  double pp = 1.0, pc = a[0] - x;
-  bool neg = pc < 0.0;
-  int cnt = neg ? 1 : 0;
-  for (int i = 1; i < m; ++i) {
-    const double pn = (a[i] - x) * pc - b[i - 1] * b[i - 1] * pp;
-    pp = pc;
-    pc = pn;
-    const long long bits = __double_as_longlong(pc);
-    const bool nneg = ((bits << 1) != 0) ? (bits < 0) : !neg;   // a zero minor takes the opposite sign
-    cnt += (nneg != neg);
-    neg = nneg;
-    if ((i & 3) == 0) {
-      const int e = max(dexp_bits(pc), dexp_bits(pp));
-      if (e > 1023 + 500) { pc *= 0x1p-500; pp *= 0x1p-500; }
-      else if (e < 1023 - 500) { pc *= 0x1p500; pp *= 0x1p500; }
+// Stages the tridiagonal (a, b; size m) in `tri` (all threads; the caller synchronises).
+__device__ __forceinline__ void tri_stage(const double* a, const double* b, int m, double2* tri) {
+  for (int i = threadIdx.x; i < tri_blocks(m) * kTriBlock; i += blockDim.x) {
+    const double bb = (i > 0 && i < m) ? b[i - 1] : 0.0;
+    tri[i] = make_double2(i < m ? a[i] : 0x1p60, bb * bb);
+  }
+}
+
+// Power of two that brings the larger of two doubles to [1, 2) (their biased exponent on the integer
+// pipe; two zeros or subnormals are scaled by 2^1022).
+__device__ __forceinline__ double pow2_normaliser(double p, double q) {
+  const int e = max(max((__double2hiint(p) >> 20) & 0x7FF, (__double2hiint(q) >> 20) & 0x7FF), 1);
+  return __hiloint2double((2046 - e) << 20, 0);
+}
+
+// Number of eigenvalues of the tridiagonal below x: sign changes of the leading principal minors
+// det(T_k - x I), computed with the three-term recurrence. What bounds it is one dependent DFMA a row
+// (8.7 cycles), so nothing else may stand on that chain: rows are read kTriBlock at a time ahead of
+// their use, signs are counted on the integer pipe, and the pair of minors is normalised by a power
+// of two once per block without a branch (a block of entries below 2^60 cannot leave the double
+// range). A zero minor counts as positive: the minor after it has the opposite sign of the one before.
+__device__ __forceinline__ int sturm_count(const double2* tri, int blocks, double x) {
+  double pp = 0.0, pc = 1.0;
+  int cnt = 0;
+  for (int k = 0; k < blocks; ++k) {
+    double2 r[kTriBlock];
+#pragma unroll
+    for (int q = 0; q < kTriBlock; ++q) r[q] = tri[k * kTriBlock + q];
+#pragma unroll
+    for (int q = 0; q < kTriBlock; ++q) {
+      const double pn = (r[q].x - x) * pc - r[q].y * pp;
+      cnt += (int)((unsigned)(__double2hiint(pn) ^ __double2hiint(pc)) >> 31);
+      pp = pc;
+      pc = pn;
     }
+    const double f = pow2_normaliser(pc, pp);
+    pc *= f;
+    pp *= f;
   }
   return cnt;
 }
 
-// s_last^2 of the unit eigenvector for eigenvalue x: -det(T_{m-1} - x) / det'(T_m - x) (the same
-// rescaling as sturm_count).
-__device__ inline double last_component_sq(const double* a, const double* b, int m, double x) {
-  double pp = 1.0, pc = a[0] - x, dp = 0.0, dc = -1.0;
-  for (int i = 1; i < m; ++i) {
-    const double bb = b[i - 1] * b[i - 1];
-    const double pn = (a[i] - x) * pc - bb * pp;
-    const double dn = -pc + (a[i] - x) * dc - bb * dp;
-    pp = pc; pc = pn; dp = dc; dc = dn;
-    if ((i & 3) == 0) {
-      const int e = max(max(dexp_bits(pc), dexp_bits(dc)), max(dexp_bits(pp), dexp_bits(dp)));
-      if (e > 1023 + 500) { pc *= 0x1p-500; pp *= 0x1p-500; dc *= 0x1p-500; dp *= 0x1p-500; }
-      else if (e < 1023 - 500 && e > 0) { pc *= 0x1p500; pp *= 0x1p500; dc *= 0x1p500; dp *= 0x1p500; }
+// s_last^2 of the unit eigenvector for eigenvalue x of the leading m rows:
+// -det(T_{m-1} - x) / det'(T_m - x), the minors and their derivatives by the same recurrence.
+__device__ __forceinline__ double last_component_sq(const double2* tri, int m, double x) {
+  double pp = 0.0, pc = 1.0, dp = 0.0, dc = 0.0;
+  for (int k = 0; k < m; k += kTriBlock) {
+    double2 r[kTriBlock];
+#pragma unroll
+    for (int q = 0; q < kTriBlock; ++q) r[q] = tri[k + q];
+#pragma unroll
+    for (int q = 0; q < kTriBlock; ++q) {
+      if (k + q < m) {
+        const double pn = (r[q].x - x) * pc - r[q].y * pp;
+        const double dn = (r[q].x - x) * dc - (r[q].y * dp + pc);
+        pp = pc; pc = pn; dp = dc; dc = dn;
+      }
     }
+    const double f = fmin(pow2_normaliser(pc, pp), pow2_normaliser(dc, dp));
+    pc *= f; pp *= f; dc *= f; dp *= f;
   }
-  // pp = det(T_{m-1} - x) (1 for m = 1), dc = det'(T_m - x)
   if (dc == 0.0) return 1.0;
   double s2 = -pp / dc;
   if (!(s2 >= 0.0)) s2 = 0.0;
@@ -120,65 +143,96 @@ __device__ inline double last_component_sq(const double* a, const double* b, int
   return s2;
 }
 
-// Smallest eigenvalue by multisection over the whole CTA (blockDim.x points per round), and the
-// squared last component of its unit eigenvector in *s2 (every thread gets both). The tridiagonal
-// is first copied from the control block to shared memory: every Sturm count walks it
-// sequentially, so its loads must be short.
+// Gershgorin interval of the staged tridiagonal, widened by its rounding (one full warp).
+__device__ __forceinline__ void tri_interval(const double2* tri, int m, double* lo_out, double* hi_out) {
+  const int lane = threadIdx.x & 31;
+  double lo = 1e300, hi = -1e300;
+  for (int i = lane; i < m; i += 32) {
+    const double r = sqrt(tri[i].y) + (i + 1 < m ? sqrt(tri[i + 1].y) : 0.0);
+    lo = fmin(lo, tri[i].x - r);
+    hi = fmax(hi, tri[i].x + r);
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  const double pad = 1e-12 * fmax(1.0, fmax(fabs(lo), fabs(hi)));
+  *lo_out = lo - pad;
+  *hi_out = hi + pad;
+}
+
+// Threads of the multisection below, their barrier, and how many of them hold `p`. Four warps, one per
+// scheduler, keep a row of the Sturm recurrence at its DFMA latency (about 13 cycles); with sixteen
+// warps the FP64 pipe bounds it (about 38 cycles a row) for only two more bits a round.
+constexpr int kRitzThreads = 128;
+__device__ __forceinline__ int ritz_sync_count(bool p) {
+  int c;
+  asm volatile(
+      "{\n .reg .pred q;\n setp.ne.s32 q, %1, 0;\n barrier.cta.red.popc.aligned.u32 %0, 1, %2, q;\n}"
+      : "=r"(c)
+      : "r"((int)p), "n"(kRitzThreads)
+      : "memory");
+  return c;
+}
+
+// Smallest eigenvalue of the tridiagonal (a, b; size m) by multisection with kRitzThreads points per
+// round, and the squared last component of its unit eigenvector in *s2 (every thread of the CTA gets
+// both). The threads whose point lies below the eigenvalue form a prefix, so their number, from one
+// barrier, is the new bracket in every thread's registers.
 // hint_lo < hint_hi: a bracket to try first (from the previous step: by interlacing the smallest
 // eigenvalue of T_m is at most the previous smallest Ritz value, and the previous residual bounds how
-// far below it can be unless a new, lower eigenvalue appears); it is used only if the Sturm counts
-// confirm no eigenvalue below hint_lo and at least one below hint_hi, else the Gershgorin interval.
-__device__ inline double smallest_eig_block(const double* ag, const double* bg, int m, double* s2,
+// far below it can be unless a new, lower eigenvalue appears). Its points halve the distance to
+// hint_hi every second point, since near convergence the Ritz value moves by about the residual
+// squared; the round itself shows whether the bracket holds the eigenvalue, else the Gershgorin
+// interval is taken. Against a branching recurrence with its loads on the chain, on all sixteen warps,
+// and one bulge chase after the other, one alpha on ER(1024) went from 2.33 to 1.69 ms and on BA(2^16)
+// in FP64 from 6.13 to 4.94 ms (both this and the restart below).
+// scratch: 2 kTriPad doubles of shared memory, 16-byte aligned.
+__device__ inline double smallest_eig_block(const double* ag, const double* bg, int m, double* s2, double* scratch,
                                             double hint_lo = 0.0, double hint_hi = -1.0) {
-  __shared__ double s_lo, s_hi, s_s2;
-  __shared__ int s_first, s_cnt_lo, s_cnt_hi;
-  __shared__ double a[kNcvMax], b[kNcvMax];
-  for (int i = threadIdx.x; i < m; i += blockDim.x) {
-    a[i] = ag[i];
-    b[i] = (i + 1 < m) ? bg[i] : 0.0;
-  }
+  __shared__ double s_r, s_s2;
+  double2* tri = (double2*)scratch;
+  tri_stage(ag, bg, m, tri);
   __syncthreads();
-  const bool hint = hint_lo < hint_hi;
-  if (hint && threadIdx.x == 1) s_cnt_lo = sturm_count(a, b, m, hint_lo);
-  if (hint && threadIdx.x == 2) s_cnt_hi = sturm_count(a, b, m, hint_hi);
-  if (threadIdx.x == 0) {
-    double lo = 1e300, hi = -1e300;
-    for (int i = 0; i < m; ++i) {
-      const double r = (i > 0 ? fabs(b[i - 1]) : 0.0) + (i + 1 < m ? fabs(b[i]) : 0.0);
-      lo = fmin(lo, a[i] - r);
-      hi = fmax(hi, a[i] + r);
+  if (threadIdx.x < kRitzThreads) {
+    constexpr int P = kRitzThreads;
+    const int t = threadIdx.x, blocks = tri_blocks(m);
+    double lo = 0.0, hi = 0.0;
+    bool have = false;
+    if (hint_lo < hint_hi) {
+      const double w = hint_hi - hint_lo;
+      // point t: hint_hi - w 2^(-t / 2), the last one hint_hi itself
+      auto point = [&](int k) {
+        if (k == P - 1) return hint_hi;
+        return hint_hi - w * ((k & 1) ? 0.70710678118654752 : 1.0) * __hiloint2double((1023 - (k >> 1)) << 20, 0);
+      };
+      const int f = ritz_sync_count(sturm_count(tri, blocks, point(t)) == 0);
+      if (f > 0 && f < P) {
+        lo = point(f - 1);
+        hi = point(f);
+        have = true;
+      }
     }
-    const double pad = 1e-12 * fmax(1.0, fmax(fabs(lo), fabs(hi)));
-    s_lo = lo - pad;
-    s_hi = hi + pad;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0 && hint && s_cnt_lo == 0 && s_cnt_hi >= 1 && hint_lo > s_lo && hint_hi < s_hi) {
-    s_lo = hint_lo;
-    s_hi = hint_hi;
-  }
-  __syncthreads();
-  const int P = blockDim.x;
-  for (int round = 0; round < 7; ++round) {
-    const double lo = s_lo, hi = s_hi;
-    if (threadIdx.x == 0) s_first = P;
-    __syncthreads();
-    const double x = lo + (hi - lo) * (double)(threadIdx.x + 1) / (double)(P + 1);
-    if (sturm_count(a, b, m, x) >= 1) atomicMin(&s_first, (int)threadIdx.x);
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      const int f = s_first;
-      const double nlo = (f == 0) ? lo : lo + (hi - lo) * (double)f / (double)(P + 1);
-      const double nhi = (f >= P) ? hi : lo + (hi - lo) * (double)(f + 1) / (double)(P + 1);
-      s_lo = nlo;
-      s_hi = nhi;
+    if (!have) tri_interval(tri, m, &lo, &hi);
+    for (int round = 0; round < 9 && hi - lo > 1e-15 * fmax(1.0, fabs(hi)); ++round) {
+      const double w = (hi - lo) * (1.0 / (P + 1));
+      const int f = ritz_sync_count(sturm_count(tri, blocks, lo + w * (double)(t + 1)) == 0);
+      const double nlo = f > 0 ? lo + w * (double)f : lo;
+      if (f < P) hi = lo + w * (double)(f + 1);
+      lo = nlo;
     }
-    __syncthreads();
-    if (s_hi - s_lo <= 1e-15 * fmax(1.0, fabs(s_hi))) break;
+    const double r = 0.5 * (lo + hi);
+    if (t < 32) {
+      const double c2 = last_component_sq(tri, m, r);
+      if (t == 0) {
+        s_r = r;
+        s_s2 = c2;
+      }
+    }
   }
-  const double r = 0.5 * (s_lo + s_hi);
-  if (threadIdx.x == 0) s_s2 = last_component_sq(a, b, m, r);
   __syncthreads();
+  const double r = s_r;
   *s2 = s_s2;
   __syncthreads();
   return r;
@@ -245,82 +299,95 @@ __device__ inline void tridiag_eigvec(const double* a, const double* b, int m, d
   }
 }
 
-// The (q+1)-th smallest eigenvalue of the tridiagonal by bisection on the Sturm count.
-__device__ inline double kth_eig(const double* a, const double* b, int m, int q) {
-  double lo = 1e300, hi = -1e300;
-  for (int i = 0; i < m; ++i) {
-    const double r = (i > 0 ? fabs(b[i - 1]) : 0.0) + (i + 1 < m ? fabs(b[i]) : 0.0);
-    lo = fmin(lo, a[i] - r);
-    hi = fmax(hi, a[i] + r);
+// All eigenvalues of the staged tridiagonal in ascending order into out[m] (the CTA): four lanes per
+// eigenvalue, three of them probing the quarters of its bracket in each of 27 rounds.
+__device__ inline void all_eigs_block(const double2* tri, int m, double* out) {
+  const int sub = threadIdx.x & 3, blocks = tri_blocks(m);
+  double lo0, hi0;
+  tri_interval(tri, m, &lo0, &hi0);
+  for (int base = 0; base < m; base += blockDim.x >> 2) {
+    const int q = min(base + (int)(threadIdx.x >> 2), m - 1);
+    if (base + (int)((threadIdx.x & ~31) >> 2) >= m) break;   // a warp without an eigenvalue of its own
+    double lo = lo0, hi = hi0;
+    for (int it = 0; it < 27; ++it) {
+      const double w = 0.25 * (hi - lo);
+      // points whose count leaves eigenvalue q above them form a prefix of the three
+      const bool above = sub < 3 && sturm_count(tri, blocks, lo + w * (double)(sub + 1)) <= q;
+      const unsigned g = (__ballot_sync(0xffffffffu, above) >> (threadIdx.x & 28)) & 7u;
+      const int k = __popc(g);
+      if (k < 3) hi = lo + w * (double)(k + 1);
+      lo += w * (double)k;
+    }
+    if (sub == 0) out[q] = 0.5 * (lo + hi);
   }
-  lo -= 1e-12 * fmax(1.0, fabs(lo));
-  hi += 1e-12 * fmax(1.0, fabs(hi));
-  for (int it = 0; it < 80 && hi - lo > 1e-15 * fmax(1.0, fabs(hi)); ++it) {
-    const double mid = 0.5 * (lo + hi);
-    if (sturm_count(a, b, m, mid) >= q + 1) hi = mid;
-    else lo = mid;
-  }
-  return 0.5 * (lo + hi);
 }
 
 // Implicit restart with exact shifts (the CTA): the m - kk largest Ritz values of the tridiagonal
 // (a, b; size m) are the shifts of implicit QR steps. Each step is a bulge chase on the tridiagonal
-// itself (diagonal d, off-diagonal e and the one bulge entry, O(m) work by one thread: rotation r
-// acts on rows and columns r, r + 1 as T <- G T G^T with G = [[c, s], [-s, c]]); its m - 1 rotations
-// are then applied to the rows of Q (Qd, m x m row-major, Q <- Q G^T) by all threads, one row each,
-// with the row's moving entry kept in a register. Afterwards Q^T T Q has a leading kk x kk
-// tridiagonal, written back to a and b, and the residual of the kept basis is
-// V Q[:, kk] T+[kk][kk-1] + w Q[m-1][kk-1] (w: the pending unnormalised Lanczos vector).
-// scratch: 5 kNcvMax doubles of shared memory.
+// itself (diagonal d, off-diagonal e and the one bulge entry): rotation r acts on rows and columns
+// r, r + 1 as T <- G T G^T with G = [[c, s], [-s, c]], and on the rows of Q (Qd, m x m row-major,
+// Q <- Q G^T). Rotation r of a shift touches d[r], d[r + 1] and e[r - 1 .. r + 1], so the next shift
+// follows three rotations behind: thread s chases shift s and all chases advance together, m - 1 + 3
+// (m - kk - 1) steps instead of (m - kk)(m - 1), each of them a square root's latency; the other
+// threads apply the rotations of the step before to Q meanwhile. The values are those of one chase after
+// the other. Afterwards Q^T T Q has a leading kk x kk tridiagonal, written back to a and b, and the
+// residual of the kept basis is V Q[:, kk] T+[kk][kk-1] + w Q[m-1][kk-1] (w: the pending unnormalised
+// Lanczos vector). scratch: 2 kTriPad + 7 kNcvMax doubles of shared memory, 16-byte aligned.
 __device__ inline void implicit_restart(AlphaCtrl* C, double* Qd, int m, int kk, double* scratch) {
-  double* d = scratch;
-  double* e = scratch + kNcvMax;
-  double* ritz = scratch + 2 * kNcvMax;
-  double* rc = scratch + 3 * kNcvMax;
-  double* rs = scratch + 4 * kNcvMax;
+  double2* tri = (double2*)scratch;
+  double* d = scratch + 2 * kTriPad;
+  double* e = d + kNcvMax;
+  double* ritz = e + kNcvMax;
+  double2* rot = (double2*)(ritz + kNcvMax);   // two steps' rotations, one per shift
   const int t = threadIdx.x;
+  tri_stage(C->a, C->b, m, tri);
   for (int i = t; i < m; i += blockDim.x) {
     d[i] = C->a[i];
     e[i] = (i + 1 < m) ? C->b[i] : 0.0;
   }
-  __syncthreads();
-  if (t < m) ritz[t] = kth_eig(d, e, m, t);
   for (int idx = t; idx < m * m; idx += blockDim.x) Qd[idx] = (idx / m == idx % m) ? 1.0 : 0.0;
   __syncthreads();
-  for (int sft = m - 1; sft >= kk; --sft) {
-    if (t == 0) {
-      const double mu = ritz[sft];
-      double g = 0.0;                          // bulge T[r+1][r-1]
-      for (int r = 0; r < m - 1; ++r) {
-        const double x = (r == 0) ? d[0] - mu : e[r - 1];
-        const double z = (r == 0) ? e[0] : g;
-        const double rr = hypot(x, z);
-        const double c = (rr == 0.0) ? 1.0 : x / rr;
-        const double sn = (rr == 0.0) ? 0.0 : z / rr;
-        if (r > 0) e[r - 1] = rr;
-        const double dr = d[r], dn = d[r + 1], er = e[r];
-        d[r] = c * c * dr + 2.0 * c * sn * er + sn * sn * dn;
-        d[r + 1] = sn * sn * dr - 2.0 * c * sn * er + c * c * dn;
-        e[r] = c * sn * (dn - dr) + (c * c - sn * sn) * er;
-        if (r + 2 < m) {
-          g = sn * e[r + 1];
-          e[r + 1] = c * e[r + 1];
-        }
-        rc[r] = c;
-        rs[r] = sn;
+  all_eigs_block(tri, m, ritz);
+  __syncthreads();
+  const int ns = m - kk, steps = (m - 1) + 3 * (ns - 1);
+  double g = 0.0;                              // this chase's bulge T[r+1][r-1]
+  for (int step = 0; step <= steps; ++step) {
+    // rotation r = step - 3 s of shift s (the largest Ritz value first)
+    const int r = step - 3 * t;
+    if (t < ns && r >= 0 && r < m - 1) {
+      const double x = (r == 0) ? d[0] - ritz[m - 1 - t] : e[r - 1];
+      const double z = (r == 0) ? e[0] : g;
+      const double h = x * x + z * z;
+      const double inv = (h == 0.0) ? 0.0 : rsqrt(h);
+      const double c = (h == 0.0) ? 1.0 : x * inv;
+      const double sn = z * inv;
+      if (r > 0) e[r - 1] = h * inv;
+      const double dr = d[r], dn = d[r + 1], er = e[r];
+      d[r] = c * c * dr + 2.0 * c * sn * er + sn * sn * dn;
+      d[r + 1] = sn * sn * dr - 2.0 * c * sn * er + c * c * dn;
+      e[r] = c * sn * (dn - dr) + (c * c - sn * sn) * er;
+      if (r + 2 < m) {
+        g = sn * e[r + 1];
+        e[r + 1] = c * e[r + 1];
       }
+      rot[(step & 1) * kNcvMax + t] = make_double2(c, sn);
     }
-    __syncthreads();
-    for (int q = t; q < m; q += blockDim.x) {
-      double* row = Qd + (long long)q * m;
-      double pv = row[0];
-      for (int r = 0; r < m - 1; ++r) {
-        const double qv = row[r + 1];
-        const double c = rc[r], sn = rs[r];
-        row[r] = c * pv + sn * qv;
-        pv = -sn * pv + c * qv;
+    // the rotations of the step before, on every row of Q (disjoint pairs of columns)
+    const int prev = step - 1;
+    if (prev >= 0) {
+      const int s_lo = max(0, (prev - (m - 2) + 2) / 3), s_hi = min(ns - 1, prev / 3);
+      const int cnt = s_hi - s_lo + 1;
+      // the chasing warps come last in the order of the work on Q
+      const int tt = (int)blockDim.x - 1 - t;
+      for (int idx = tt; idx < cnt * m; idx += blockDim.x) {
+        const int s = s_lo + idx % cnt, q = idx / cnt;
+        const int pr = prev - 3 * s;
+        const double2 cs = rot[(prev & 1) * kNcvMax + s];
+        double* row = Qd + (long long)q * m + pr;
+        const double pv = row[0], qv = row[1];
+        row[0] = cs.x * pv + cs.y * qv;
+        row[1] = -cs.y * pv + cs.x * qv;
       }
-      row[m - 1] = pv;
     }
     __syncthreads();
   }
@@ -452,12 +519,13 @@ constexpr int kRedCols = 2 * kNcvMax + kDotBatch + 8;
 // (the batch kernel, whose register budget the other paths would spill).
 template <typename T, typename RP, class Pol, int NW = kWarps, bool kLayouts = true>
 __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol& pol) {
+  static_assert(2 * kTriPad + 7 * kNcvMax <= kNcvMax * (kRestartMax + 1), "restart scratch too small");
   static_assert(NW * (kDotBatch + 1) <= kRedCols, "reduction scratch too small");
   __shared__ double sm[kRedCols];
   __shared__ double sh[kNcvMax];
   __shared__ double s_theta, s_s2;
   __shared__ SpmvSmem<T, NW> ssp;
-  __shared__ double sq[kNcvMax * (kRestartMax + 1)];
+  __shared__ __align__(16) double sq[kNcvMax * (kRestartMax + 1)];
   __shared__ unsigned long long pbars[kPanelBufs];
   extern __shared__ __align__(128) char panel_smem[];
   AlphaCtrl* C = A.ctrl;
@@ -847,7 +915,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
                 hlo = th0 - 2.0 * r0 - pad;
                 hhi = th0 + pad;
               }
-              const double th = smallest_eig_block(C->a, C->b, m, &s2, hlo, hhi);
+              const double th = smallest_eig_block(C->a, C->b, m, &s2, sq, hlo, hhi);
               if (threadIdx.x == 0) {
                 s_theta = th;
                 s_s2 = s2;
@@ -928,13 +996,15 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
         block_store_partials<1>(v, A.part, A.pw, 0, sm, pol.block());
         if (!pol.sync(&C->gs, [&] {
               reduce_partials(A.part, A.pw, pol.nblocks(), 1, sm);
+              const double nf = sqrt(sm[0]);
+              const bool invariant = !(nf > 1e-14 * bound) || !isfinite(nf);
+              double th = 0.0, s2 = 0.0;
+              if (invariant) th = smallest_eig_block(C->a, C->b, kk, &s2, sq);
               if (threadIdx.x == 0) {
-                const double nf = sqrt(sm[0]);
                 C->pass2 = 0;
                 C->bytes += (double)n * sizeof(T) * (double)(m + kk + 3);
-                if (!(nf > 1e-14 * bound) || !isfinite(nf)) {
+                if (invariant) {
                   // the kept basis spans an invariant subspace: finish with its Ritz vector
-                  const double th = kth_eig(C->a, C->b, kk, 0);
                   C->theta = th;
                   tridiag_eigvec(C->a, C->b, kk, th, C->s);
                   C->j = kk - 1;
