@@ -21,6 +21,7 @@
 namespace sa {
 
 constexpr int kAdjWindow = 50;          // MINRES iterations between stagnation checks
+constexpr int kAdjCols = 8;             // columns of partial sums (PhaseSums)
 constexpr double kAdjStallOk = 1e-3;    // a stalled solve counts as converged below this residual
 
 struct AdjCtrl {
@@ -52,8 +53,7 @@ struct AdjArgs {
   T* G;
   double* grad;
   T* out;
-  double* part;
-  int pw;
+  double* part;      // two buffers of kAdjCols columns x CTAs
   AdjCtrl* ctrl;
   PanelArgs panel;   // column-panel layout of the operator (use_panel = 1, with
   int use_panel;     // panel_smem_bytes(sizeof(T)) of dynamic shared memory), else the work list
@@ -71,13 +71,15 @@ __device__ __forceinline__ double dlog_of(const AdjArgs<T, RP>& A, long long i) 
 
 template <typename T, typename RP>
 __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) {
-  __shared__ double sm[kWarps * 4];
-  __shared__ double sh[8];
+  __shared__ double sm[kWarps * 3];
+  __shared__ double sh[kAdjCols];
+  __shared__ AdjCtrl ctl;   // this CTA's copy of the control block; every CTA computes the same one
   __shared__ SpmvSmem<T> ssp;
   __shared__ unsigned long long pbars[kPanelBufs];
   extern __shared__ __align__(128) char panel_smem[];
   const GridPolicy pol;
-  AdjCtrl* C = A.ctrl;
+  AdjCtrl* const C = &ctl;
+  PhaseSums<GridPolicy, kAdjCols> sums(pol, &A.ctrl->gs, A.part, sm, sh);
   const long long n = A.n;
   const long long gtid = pol.tid(), nthreads = pol.nthr();
   const long long gwarp = gtid >> 5, nwarps = nthreads >> 5;
@@ -86,14 +88,26 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
   // one operator application: fin(row, sum_j val_ij u_j) once per row; false on a timed-out wait
   auto apply = [&](auto&& fin) -> bool {
     if (A.use_panel)
-      return panel_spmv<T>(A.panel, A.u, pol.block(), pol.nblocks(), panel_smem, pbars, ppar, &C->gs.error, fin);
+      return panel_spmv<T>(A.panel, A.u, pol.block(), pol.nblocks(), panel_smem, pbars, ppar, &A.ctrl->gs.error,
+                           [](long long) { return 0; }, [&](long long r, T acc, int) { fin(r, acc); });
     spmv_items<T, RP>(A.S, A.u, gwarp, nwarps, ssp, fin);
     return true;
   };
   const T tlam = (T)A.lambda;
+  // the results as the host reads them
+  auto publish = [&] {
+    if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    A.ctrl->beta1 = C->beta1;
+    A.ctrl->phibar = C->phibar;
+    A.ctrl->loss = C->loss;
+    A.ctrl->dalpha = C->dalpha;
+    A.ctrl->itn = C->itn;
+    A.ctrl->spmvs = C->spmvs;
+    A.ctrl->status = C->status;
+  };
 
   // ---- P0: scaling for the exponents, zero the recurrences' vectors, mode set-up ------------
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
     C->status = SA_OK;
     C->spmvs = 0;
     C->itn = 0;
@@ -119,7 +133,7 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
       A.u[i] = sg * yh;
     }
   }
-  if (!grid_barrier(&C->gs)) return;
+  if (!sums.meet()) return;
 
   // ---- P1: right-hand side G (and the loss) ---------------------------------------------------
   if (A.mode == 0) {
@@ -133,34 +147,32 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
       v[0] += t * jt;
       v[1] += (double)__ldg(A.yhat + r) * (double)gy;
     })) return;
-    block_store_partials<2>(v, A.part, A.pw, 0, sm, blockIdx.x);
-    if (!grid_barrier(&C->gs, [&] {
-          reduce_partials(A.part, A.pw, gridDim.x, 2, sh);
-          if (threadIdx.x == 0) {
-            C->loss = -0.5 * sh[0];
-            C->rhs_dot = sh[1];
-            C->spmvs += 1;
-          }
-        })) return;
+    sums.block_put(v);
+    if (!sums.all_sum(2)) return;
+    if (threadIdx.x == 0) {
+      C->loss = -0.5 * sh[0];
+      C->rhs_dot = sh[1];
+      C->spmvs += 1;
+    }
+    __syncthreads();
   } else if (A.mode == 1) {
     if (!apply([&](long long r, T acc) {
       A.Z[r] = __ldcg(A.sigma + r) * acc;                     // (M y)_r
     })) return;
-    if (!grid_barrier(&C->gs)) return;
+    if (!sums.meet()) return;
     for (long long i = gtid; i < n; i += nthreads)
       A.u[i] = (T)((double)__ldcg(A.sigma + i) * dlog_of(A, i) * (double)__ldg(A.yhat + i));
-    if (!grid_barrier(&C->gs)) return;
+    if (!sums.meet()) return;
     double v[1] = {0.0};
     if (!apply([&](long long r, T acc) {
       const T g = (T)(dlog_of(A, r) * (double)__ldcg(A.Z + r) + (double)__ldcg(A.sigma + r) * (double)acc);
       A.G[r] = g;
       v[0] += (double)__ldg(A.yhat + r) * (double)g;
     })) return;
-    block_store_partials<1>(v, A.part, A.pw, 0, sm, blockIdx.x);
-    if (!grid_barrier(&C->gs, [&] {
-          reduce_partials(A.part, A.pw, gridDim.x, 1, sh);
-          if (threadIdx.x == 0) { C->rhs_dot = sh[0]; C->spmvs += 2; }
-        })) return;
+    sums.block_put(v);
+    if (!sums.all_sum(1)) return;
+    if (threadIdx.x == 0) { C->rhs_dot = sh[0]; C->spmvs += 2; }
+    __syncthreads();
   } else {
     double v[1] = {0.0};
     for (long long i = gtid; i < n; i += nthreads) {
@@ -168,16 +180,15 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
       A.G[i] = g;
       v[0] += (double)__ldg(A.yhat + i) * (double)g;
     }
-    block_store_partials<1>(v, A.part, A.pw, 0, sm, blockIdx.x);
-    if (!grid_barrier(&C->gs, [&] {
-          reduce_partials(A.part, A.pw, gridDim.x, 1, sh);
-          if (threadIdx.x == 0) C->rhs_dot = sh[0];
-        })) return;
+    sums.block_put(v);
+    if (!sums.all_sum(1)) return;
+    if (threadIdx.x == 0) C->rhs_dot = sh[0];
+    __syncthreads();
   }
 
   // ---- P2: b = (I - y y^T) G; r1 = r2 = b; explicit gradient term ----------------------------
   {
-    const double rd = vload(&C->rhs_dot);
+    const double rd = C->rhs_dot;
     double v[1] = {0.0};
     for (long long i = gtid; i < n; i += nthreads) {
       const double g = (double)__ldcg(A.G + i);
@@ -188,43 +199,42 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
       v[0] += (double)bi * (double)bi;
       if (A.mode == 0) A.grad[i] = dlog_of(A, i) * g * yh;   // g_x,i x_i l_i with g_y = D^{-1/2} g_x
     }
-    block_store_partials<1>(v, A.part, A.pw, 0, sm, blockIdx.x);
-    if (!grid_barrier(&C->gs, [&] {
-          reduce_partials(A.part, A.pw, gridDim.x, 1, sh);
-          if (threadIdx.x == 0) {
-            const double b1 = sqrt(sh[0]);
-            C->beta1 = b1;
-            C->beta = b1;
-            C->oldb = 0.0;
-            C->dbar = 0.0;
-            C->epsln = 0.0;
-            C->phibar = b1;
-            C->cs = -1.0;
-            C->sn = 0.0;
-            C->chk_phibar = b1;
-            C->ir1 = 0; C->ir2 = 1; C->iy = 2;
-            C->iw = 0; C->iw1 = 1; C->iw2 = 2;
-            C->done = (b1 > 0.0 && isfinite(b1)) ? 0 : 1;
-            if (!isfinite(b1)) C->status = SA_ERR_NONFINITE;
-          }
-        })) return;
+    sums.block_put(v);
+    if (!sums.all_sum(1)) return;
+    if (threadIdx.x == 0) {
+      const double b1 = sqrt(sh[0]);
+      C->beta1 = b1;
+      C->beta = b1;
+      C->oldb = 0.0;
+      C->dbar = 0.0;
+      C->epsln = 0.0;
+      C->phibar = b1;
+      C->cs = -1.0;
+      C->sn = 0.0;
+      C->chk_phibar = b1;
+      C->ir1 = 0; C->ir2 = 1; C->iy = 2;
+      C->iw = 0; C->iw1 = 1; C->iw2 = 2;
+      C->done = (b1 > 0.0 && isfinite(b1)) ? 0 : 1;
+      if (!isfinite(b1)) C->status = SA_ERR_NONFINITE;
+    }
+    __syncthreads();
   }
   // first Lanczos vector v = r2 / beta and its scaled copy for the SpMV gather
-  if (!vload(&C->done)) {
-    const double ib = 1.0 / vload(&C->beta);
+  if (!C->done) {
+    const double ib = 1.0 / C->beta;
     for (long long i = gtid; i < n; i += nthreads) {
       const T vi = (T)((double)__ldcg(A.R[1] + i) * ib);
       A.V[i] = vi;
       A.u[i] = __ldcg(A.sigma + i) * vi;
     }
   }
-  if (!grid_barrier(&C->gs)) return;
+  if (!sums.meet()) return;
 
   // ---- MINRES on (lambda I - M) restricted to y's complement ----------------------------------
-  while (!vload(&C->done)) {
-    const int ir1 = vload(&C->ir1), ir2 = vload(&C->ir2), iy = vload(&C->iy);
-    const double beta = vload(&C->beta), oldb = vload(&C->oldb);
-    const int itn = vload(&C->itn);
+  while (!C->done) {
+    const int ir1 = C->ir1, ir2 = C->ir2, iy = C->iy;
+    const double beta = C->beta, oldb = C->oldb;
+    const int itn = C->itn;
     // PS: y = (lambda I - M) v - (beta / oldb) r1; alfa = v.y. The Krylov vectors are not
     // re-projected: applying (I - y y^T) after the operator alone would make it unsymmetric and
     // break the short recurrence; the right-hand side is orthogonal to y and the operator maps y's
@@ -242,19 +252,18 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
         yv[r] = yt;
         v[0] += (double)vr * (double)yt;
       })) return;
-      block_store_partials<1>(v, A.part, A.pw, 0, sm, blockIdx.x);
-      if (!grid_barrier(&C->gs, [&] {
-            reduce_partials(A.part, A.pw, gridDim.x, 1, sh);
-            if (threadIdx.x == 0) {
-              C->alfa = sh[0];
-              C->itn = itn + 1;
-              C->spmvs += 1;
-            }
-          })) return;
+      sums.block_put(v);
+      if (!sums.all_sum(1)) return;
+      if (threadIdx.x == 0) {
+        C->alfa = sh[0];
+        C->itn = itn + 1;
+        C->spmvs += 1;
+      }
+      __syncthreads();
     }
     // PU: y <- y - (alfa / beta) r2 ; |y|^2
     {
-      const double fa = vload(&C->alfa) / beta;
+      const double fa = C->alfa / beta;
       const T* r2 = A.R[ir2];
       T* yv = A.R[iy];
       double v[1] = {0.0};
@@ -264,57 +273,56 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
         yv[i] = yt;
         v[0] += (double)yt * (double)yt;
       }
-      block_store_partials<1>(v, A.part, A.pw, 0, sm, blockIdx.x);
-      if (!grid_barrier(&C->gs, [&] {
-            reduce_partials(A.part, A.pw, gridDim.x, 1, sh);
-            if (threadIdx.x == 0) {
-              // r1 <- r2, r2 <- y (index rotation); Givens update of the QR factor of T_k
-              C->ir1 = ir2;
-              C->ir2 = iy;
-              C->iy = ir1;
-              C->oldb = beta;
-              const double nb = sqrt(sh[0]);
-              C->beta = nb;
-              const double alfa = C->alfa;
-              C->oldeps = C->epsln;
-              C->delta = C->cs * C->dbar + C->sn * alfa;
-              const double gbar = C->sn * C->dbar - C->cs * alfa;
-              C->epsln = C->sn * nb;
-              C->dbar = -C->cs * nb;
-              const double gamma = fmax(hypot(gbar, nb), 1e-300);
-              C->cs = gbar / gamma;
-              C->sn = nb / gamma;
-              C->phi = C->cs * C->phibar;
-              C->phibar = C->sn * C->phibar;
-              C->denom = 1.0 / gamma;
-              const bool conv = C->phibar <= A.tol * C->beta1 || !(nb > 0.0);
-              // stagnation: the right-hand side keeps a component along the true eigenvector as
-              // large as the eigenpair's error, which the projected operator cannot resolve; the
-              // residual estimate then stops decreasing and further iterations change nothing
-              bool stalled = false;
-              if (C->itn % kAdjWindow == 0) {
-                stalled = C->phibar > 0.99 * C->chk_phibar;
-                C->chk_phibar = C->phibar;
-              }
-              if (!isfinite(nb) || !isfinite(alfa)) {
-                C->status = SA_ERR_NONFINITE;
-                C->done = 1;
-              } else if (conv || stalled || C->itn >= A.maxiter) {
-                C->status = (conv || (stalled && C->phibar <= kAdjStallOk * C->beta1)) ? SA_OK : SA_ERR_NOT_CONVERGED;
-                C->done = 1;
-              }
-            }
-          })) return;
+      sums.block_put(v);
+      if (!sums.all_sum(1)) return;
+      if (threadIdx.x == 0) {
+        // r1 <- r2, r2 <- y (index rotation); Givens update of the QR factor of T_k
+        C->ir1 = ir2;
+        C->ir2 = iy;
+        C->iy = ir1;
+        C->oldb = beta;
+        const double nb = sqrt(sh[0]);
+        C->beta = nb;
+        const double alfa = C->alfa;
+        C->oldeps = C->epsln;
+        C->delta = C->cs * C->dbar + C->sn * alfa;
+        const double gbar = C->sn * C->dbar - C->cs * alfa;
+        C->epsln = C->sn * nb;
+        C->dbar = -C->cs * nb;
+        const double gamma = fmax(hypot(gbar, nb), 1e-300);
+        C->cs = gbar / gamma;
+        C->sn = nb / gamma;
+        C->phi = C->cs * C->phibar;
+        C->phibar = C->sn * C->phibar;
+        C->denom = 1.0 / gamma;
+        const bool conv = C->phibar <= A.tol * C->beta1 || !(nb > 0.0);
+        // stagnation: the right-hand side keeps a component along the true eigenvector as
+        // large as the eigenpair's error, which the projected operator cannot resolve; the
+        // residual estimate then stops decreasing and further iterations change nothing
+        bool stalled = false;
+        if (C->itn % kAdjWindow == 0) {
+          stalled = C->phibar > 0.99 * C->chk_phibar;
+          C->chk_phibar = C->phibar;
+        }
+        if (!isfinite(nb) || !isfinite(alfa)) {
+          C->status = SA_ERR_NONFINITE;
+          C->done = 1;
+        } else if (conv || stalled || C->itn >= A.maxiter) {
+          C->status = (conv || (stalled && C->phibar <= kAdjStallOk * C->beta1)) ? SA_OK : SA_ERR_NOT_CONVERGED;
+          C->done = 1;
+        }
+      }
+      __syncthreads();
     }
     // PW: w = (v - oldeps w1 - delta w2) / gamma into the oldest buffer; x += phi w; next v
     {
-      const int iw = vload(&C->iw), iw1 = vload(&C->iw1), iw2 = vload(&C->iw2);
-      const double oldeps = vload(&C->oldeps), delta = vload(&C->delta), denom = vload(&C->denom);
-      const double phi = vload(&C->phi);
-      const int done = vload(&C->done);
-      const double nb = vload(&C->beta);
+      const int iw = C->iw, iw1 = C->iw1, iw2 = C->iw2;
+      const double oldeps = C->oldeps, delta = C->delta, denom = C->denom;
+      const double phi = C->phi;
+      const int done = C->done;
+      const double nb = C->beta;
       const double ib = done ? 0.0 : 1.0 / nb;
-      const int nr2 = vload(&C->ir2);
+      const int nr2 = C->ir2;
       for (long long i = gtid; i < n; i += nthreads) {
         const double vi = (double)__ldcg(A.V + i);
         const double w = (vi - oldeps * (double)__ldcg(A.Wb[iw2] + i) - delta * (double)__ldcg(A.Wb[iw] + i)) * denom;
@@ -326,13 +334,13 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
           A.u[i] = __ldcg(A.sigma + i) * vn;
         }
       }
-      if (!grid_barrier(&C->gs, [&] {
-            if (threadIdx.x == 0) {
-              C->iw = iw1;
-              C->iw1 = iw2;
-              C->iw2 = iw;
-            }
-          })) return;
+      if (!sums.meet()) return;
+      if (threadIdx.x == 0) {
+        C->iw = iw1;
+        C->iw1 = iw2;
+        C->iw2 = iw;
+      }
+      __syncthreads();
     }
   }
 
@@ -340,14 +348,13 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
   {
     double v[1] = {0.0};
     for (long long i = gtid; i < n; i += nthreads) v[0] += (double)__ldg(A.yhat + i) * (double)__ldcg(A.X + i);
-    block_store_partials<1>(v, A.part, A.pw, 0, sm, blockIdx.x);
-    if (!grid_barrier(&C->gs, [&] {
-          reduce_partials(A.part, A.pw, gridDim.x, 1, sh);
-          if (threadIdx.x == 0) C->xproj = sh[0];
-        })) return;
+    sums.block_put(v);
+    if (!sums.all_sum(1)) return;
+    if (threadIdx.x == 0) C->xproj = sh[0];
+    __syncthreads();
   }
   {
-    const double xp = vload(&C->xproj);
+    const double xp = C->xproj;
     for (long long i = gtid; i < n; i += nthreads) {
       const T xi = (T)((double)__ldcg(A.X + i) - xp * (double)__ldg(A.yhat + i));
       A.X[i] = xi;
@@ -355,16 +362,19 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
       else A.out[i] = xi;
     }
   }
-  if (A.mode != 0) return;
-  if (!grid_barrier(&C->gs)) return;
+  if (A.mode != 0) {
+    publish();
+    return;
+  }
+  if (!sums.meet()) return;
 
   // ---- gradient: M w, then M y and the assembly --------------------------------------------------
   if (!apply([&](long long r, T acc) {
     A.Z[r] = __ldcg(A.sigma + r) * acc;
   })) return;
-  if (!grid_barrier(&C->gs)) return;
+  if (!sums.meet()) return;
   for (long long i = gtid; i < n; i += nthreads) A.u[i] = __ldcg(A.sigma + i) * __ldg(A.yhat + i);
-  if (!grid_barrier(&C->gs)) return;
+  if (!sums.meet()) return;
   {
     double v[1] = {0.0};
     if (!apply([&](long long r, T acc) {
@@ -374,17 +384,16 @@ __global__ void __launch_bounds__(kThreads, 1) adjoint_kernel(AdjArgs<T, RP> A) 
       A.grad[r] = g;
       v[0] += g;
     })) return;
-    block_store_partials<1>(v, A.part, A.pw, 0, sm, blockIdx.x);
-    grid_barrier(&C->gs, [&] {
-      reduce_partials(A.part, A.pw, gridDim.x, 1, sh);
-      if (threadIdx.x == 0) { C->dalpha = sh[0]; C->spmvs += 2; }
-    });
+    sums.block_put(v);
+    if (!sums.all_sum(1)) return;
+    if (threadIdx.x == 0) { C->dalpha = sh[0]; C->spmvs += 2; }
   }
+  publish();
 }
 
 // ---- host side ------------------------------------------------------------------------------
 
-constexpr int kAdjPartWidth = 8;
+constexpr int kAdjPartWidth = 2 * kAdjCols;
 
 struct AdjCarve {
   size_t sigma, u, V, R[3], W[3], X, Z, G, part, ctrl, total;
@@ -441,7 +450,6 @@ static int launch_adjoint(sa_handle* h, const sa_adjoint_params* p, char* ws, in
   A.grad = p->grad;
   A.out = (T*)p->out;
   A.part = (double*)(ws + c.part);
-  A.pw = kAdjPartWidth;
   A.ctrl = (AdjCtrl*)(ws + c.ctrl);
   if (cudaMemsetAsync(A.ctrl, 0, sizeof(GridSync), h->stream) != cudaSuccess) return SA_ERR_CUDA;
   if (h->n_mc && cudaMemsetAsync(h->mc_count, 0, 4 * h->n_mc, h->stream) != cudaSuccess) return SA_ERR_CUDA;

@@ -8,9 +8,10 @@
 //
 // Vectors (basis V, w, u, y) are in T (float or double); every inner product and norm is
 // accumulated in double; the projected tridiagonal T_j lives in double in the control block.
-// Between phases the CTAs meet at grid_barrier, whose epilogue (run by the last CTA to arrive)
-// reduces the per-CTA partial sums in CTA order and takes the Lanczos decisions, so every CTA
-// follows the same control path and results do not depend on timing.
+// Between phases the CTAs meet at a barrier; then every CTA reduces the per-CTA partial sums itself, in
+// CTA order, and takes the Lanczos decisions in its own copy of the control block. All copies are the
+// same, so every CTA follows the same control path, results do not depend on timing, and no CTA waits
+// for another one's decision.
 #pragma once
 #include <cmath>
 #include <cstdio>
@@ -24,6 +25,8 @@
 namespace sa {
 
 void count_launches(int k);
+
+constexpr int kPartCols = kNcvMax + 8;   // columns of partial sums that a phase reduces at most
 
 enum Action : int { ACT_NEXT = 0, ACT_REPASS = 1, ACT_RESTART = 2, ACT_REJECT = 3, ACT_DONE = 4, ACT_ERROR = 5,
                     ACT_P0_AGAIN = 6 };
@@ -47,8 +50,7 @@ struct AlphaArgs {
   const T* yprev;
   T* yout;
   const T* v0;
-  double* part;          // per-CTA partial sums, blocks x pw
-  int pw;
+  double* part;          // per-CTA partial sums: two buffers of kPartCols columns x CTAs
   AlphaCtrl* ctrl;
   uint32_t* bits;        // scratch candidate (W words)
   long long W;
@@ -59,11 +61,12 @@ struct AlphaArgs {
   int group;
   double spmv_bytes;     // algorithmic bytes of one fused SpMV
   double* dense;         // implicit-restart scratch (dense T, then dense Q)
-  PanelArgs panel;       // column-panel layout of the operator (use_panel = 1; needs
-  int use_panel;         // panel_smem_bytes(sizeof(T)) of dynamic shared memory), else the work list
+  PanelArgs panel;       // column-panel layout of the operator (ALPHA_PANEL; panel_smem_bytes(sizeof(T)) and
+                         // at least stream_smem_bytes(sizeof(T)) of dynamic shared memory)
   SpmvArgs<T, RP> split[kMaxSplits];   // L2 column splits of the operator (n_splits > 0): one
   int n_splits;                        // work-list pass per split, partial row sums in split_part
   T* split_part;
+  int cluster;           // the grid is one cluster (GridPolicy)
 };
 
 // ---- small dense helpers for the projected tridiagonal (double, one CTA) --------------------
@@ -72,7 +75,7 @@ struct AlphaArgs {
 // padded to a multiple of kTriBlock rows with {2^60, 0}: such a row multiplies both minors by a
 // positive number and takes no part in a sign count.
 constexpr int kTriBlock = 8;
-constexpr int kTriPad = kNcvMax + kTriBlock;
+constexpr int kTriPad = kNcvMax + 2 * kTriBlock;
 __host__ __device__ constexpr int tri_blocks(int m) { return (m + kTriBlock - 1) / kTriBlock; }
 
 // Stages the tridiagonal (a, b; size m) in `tri` (all threads; the caller synchronises).
@@ -92,61 +95,83 @@ __device__ __forceinline__ double pow2_normaliser(double p, double q) {
 
 // Number of eigenvalues of the tridiagonal below x: sign changes of the leading principal minors
 // det(T_k - x I), computed with the three-term recurrence. What bounds it is one dependent DFMA a row
-// (8.7 cycles), so nothing else may stand on that chain: rows are read kTriBlock at a time ahead of
-// their use, signs are counted on the integer pipe, and the pair of minors is normalised by a power
-// of two once per block without a branch (a block of entries below 2^60 cannot leave the double
-// range). A zero minor counts as positive: the minor after it has the opposite sign of the one before.
+// (8.7 cycles), so nothing else may stand on that chain: a block of kTriBlock rows is read while the one
+// before it is worked on, signs are counted on the integer pipe, and the pair of minors is scaled
+// once per block by a power of two taken from the middle of the block, without a branch (entries
+// below 2^60 cannot leave the double range in between). A zero minor counts as positive: the minor
+// after it has the opposite sign of the one before.
 __device__ __forceinline__ int sturm_count(const double2* tri, int blocks, double x) {
-  double pp = 0.0, pc = 1.0;
+  double pp = 0.0, pc = 1.0, f = 1.0;
   int cnt = 0;
-  for (int k = 0; k < blocks; ++k) {
-    double2 r[kTriBlock];
+  double2 r[kTriBlock];
 #pragma unroll
-    for (int q = 0; q < kTriBlock; ++q) r[q] = tri[k * kTriBlock + q];
+  for (int q = 0; q < kTriBlock; ++q) r[q] = tri[q];
+#pragma unroll 1
+  for (int k = 1; k <= blocks; ++k) {
+    double2 nx[kTriBlock];
+    const double2* next = tri + (k < blocks ? k : 0) * kTriBlock;
+#pragma unroll
+    for (int q = 0; q < kTriBlock; ++q) nx[q] = next[q];
 #pragma unroll
     for (int q = 0; q < kTriBlock; ++q) {
-      const double pn = (r[q].x - x) * pc - r[q].y * pp;
+      const double pn = fma(r[q].x - x, pc, -__dmul_rn(r[q].y, pp));   // (the product is off the chain)
       cnt += (int)((unsigned)(__double2hiint(pn) ^ __double2hiint(pc)) >> 31);
       pp = pc;
       pc = pn;
+      if (q == kTriBlock / 2 - 1) f = pow2_normaliser(pc, pp);
     }
-    const double f = pow2_normaliser(pc, pp);
     pc *= f;
     pp *= f;
+#pragma unroll
+    for (int q = 0; q < kTriBlock; ++q) r[q] = nx[q];
   }
   return cnt;
 }
 
-// s_last^2 of the unit eigenvector for eigenvalue x of the leading m rows:
-// -det(T_{m-1} - x) / det'(T_m - x), the minors and their derivatives by the same recurrence.
-__device__ __forceinline__ double last_component_sq(const double2* tri, int m, double x) {
-  double pp = 0.0, pc = 1.0, dp = 0.0, dc = 0.0;
-  for (int k = 0; k < m; k += kTriBlock) {
-    double2 r[kTriBlock];
+// The minors det(T_{m-1} - x), det(T_m - x) and the derivative of the latter by x, up to one common
+// power of two, by the same recurrence (pad rows are left out: they are no factor of a derivative).
+struct Minors {
+  double pm1, p, dp;
+};
+
+__device__ __forceinline__ void minor_step(const double2& r, double x, double& pp, double& pc, double& dp, double& dc) {
+  const double d = r.x - x;
+  const double pn = fma(d, pc, -__dmul_rn(r.y, pp));
+  const double dn = fma(d, dc, -fma(r.y, dp, pc));
+  pp = pc; pc = pn; dp = dc; dc = dn;
+}
+
+__device__ __forceinline__ Minors last_minors(const double2* tri, int m, double x) {
+  double pp = 0.0, pc = 1.0, dp = 0.0, dc = 0.0, f = 1.0;
+  int k = 0;
+  double2 r[kTriBlock];
 #pragma unroll
-    for (int q = 0; q < kTriBlock; ++q) r[q] = tri[k + q];
+  for (int q = 0; q < kTriBlock; ++q) r[q] = tri[q];
+#pragma unroll 1
+  for (; k + kTriBlock <= m; k += kTriBlock) {
+    double2 nx[kTriBlock];   // (the staging is padded, so a block past the last one can be read)
+#pragma unroll
+    for (int q = 0; q < kTriBlock; ++q) nx[q] = tri[k + kTriBlock + q];
 #pragma unroll
     for (int q = 0; q < kTriBlock; ++q) {
-      if (k + q < m) {
-        const double pn = (r[q].x - x) * pc - r[q].y * pp;
-        const double dn = (r[q].x - x) * dc - (r[q].y * dp + pc);
-        pp = pc; pc = pn; dp = dc; dc = dn;
-      }
+      minor_step(r[q], x, pp, pc, dp, dc);
+      if (q == kTriBlock / 2 - 1) f = fmin(pow2_normaliser(pc, pp), pow2_normaliser(dc, dp));
     }
-    const double f = fmin(pow2_normaliser(pc, pp), pow2_normaliser(dc, dp));
     pc *= f; pp *= f; dc *= f; dp *= f;
+#pragma unroll
+    for (int q = 0; q < kTriBlock; ++q) r[q] = nx[q];
   }
-  if (dc == 0.0) return 1.0;
-  double s2 = -pp / dc;
-  if (!(s2 >= 0.0)) s2 = 0.0;
-  if (s2 > 1.0) s2 = 1.0;
-  return s2;
+#pragma unroll
+  for (int q = 0; q < kTriBlock - 1; ++q)
+    if (k + q < m) minor_step(r[q], x, pp, pc, dp, dc);
+  return Minors{pp, pc, dc};
 }
 
 // Gershgorin interval of the staged tridiagonal, widened by its rounding (one full warp).
 __device__ __forceinline__ void tri_interval(const double2* tri, int m, double* lo_out, double* hi_out) {
   const int lane = threadIdx.x & 31;
   double lo = 1e300, hi = -1e300;
+#pragma unroll 1
   for (int i = lane; i < m; i += 32) {
     const double r = sqrt(tri[i].y) + (i + 1 < m ? sqrt(tri[i + 1].y) : 0.0);
     lo = fmin(lo, tri[i].x - r);
@@ -176,59 +201,79 @@ __device__ __forceinline__ int ritz_sync_count(bool p) {
   return c;
 }
 
-// Smallest eigenvalue of the tridiagonal (a, b; size m) by multisection with kRitzThreads points per
-// round, and the squared last component of its unit eigenvector in *s2 (every thread of the CTA gets
-// both). The threads whose point lies below the eigenvalue form a prefix, so their number, from one
-// barrier, is the new bracket in every thread's registers.
-// hint_lo < hint_hi: a bracket to try first (from the previous step: by interlacing the smallest
-// eigenvalue of T_m is at most the previous smallest Ritz value, and the previous residual bounds how
-// far below it can be unless a new, lower eigenvalue appears). Its points halve the distance to
-// hint_hi every second point, since near convergence the Ritz value moves by about the residual
-// squared; the round itself shows whether the bracket holds the eigenvalue, else the Gershgorin
-// interval is taken. Against a branching recurrence with its loads on the chain, on all sixteen warps,
-// and one bulge chase after the other, one alpha on ER(1024) went from 2.33 to 1.69 ms and on BA(2^16)
-// in FP64 from 6.13 to 4.94 ms (both this and the restart below).
-// scratch: 2 kTriPad doubles of shared memory, 16-byte aligned.
-__device__ inline double smallest_eig_block(const double* ag, const double* bg, int m, double* s2, double* scratch,
-                                            double hint_lo = 0.0, double hint_hi = -1.0) {
+// Smallest eigenvalue of the tridiagonal (a, b; size m), and the squared last component of its unit
+// eigenvector, -det(T_{m-1} - x) / det'(T_m - x), in *s2 (every thread of the CTA gets both).
+//   1. A bracket, from Sturm counts at kRitzThreads points at a time: the threads whose point lies below
+//      the eigenvalue form a prefix, so their number, from one barrier, is the bracket in every thread's
+//      registers. hint_lo < hint_hi is a bracket to try first (from the previous step: by interlacing
+//      the smallest eigenvalue of T_m is at most the previous smallest Ritz value, and the previous
+//      residual bounds how far below it can be unless a new, lower eigenvalue appears). Its points
+//      halve the distance to hint_hi every second point, since near convergence the Ritz value moves
+//      by about the residual squared; the round itself shows whether the bracket holds the eigenvalue,
+//      else the Gershgorin interval is cut twice into kRitzThreads + 1 parts.
+//   2. Newton's iteration on det(T_m - x) from the bracket's lower end, by one warp: to the left of the
+//      smallest root of a polynomial with only real roots it increases to that root, quadratically
+//      (two to four evaluations here). It ends when the step no longer changes x, and the last
+//      evaluation gives *s2 too.
+//   3. If Newton leaves the bracket or takes too long (clustered roots), multisection to the end.
+// One test costs about DFMA latency x rows x evaluations. Each recurrence has one call site: the code
+// of a Lanczos step is read again at every step, and what does not stay in the instruction cache costs
+// as much as the arithmetic.
+__device__ __forceinline__ double smallest_eig_block(const double* ag, const double* bg, int m, double* s2,
+                                                  double hint_lo = 0.0, double hint_hi = -1.0) {
   __shared__ double s_r, s_s2;
-  double2* tri = (double2*)scratch;
+  __shared__ double2 tri[kTriPad];
+  const int t = tid_here();
   tri_stage(ag, bg, m, tri);
   __syncthreads();
-  if (threadIdx.x < kRitzThreads) {
+  if (t < kRitzThreads) {
     constexpr int P = kRitzThreads;
-    const int t = threadIdx.x, blocks = tri_blocks(m);
-    double lo = 0.0, hi = 0.0;
-    bool have = false;
-    if (hint_lo < hint_hi) {
-      const double w = hint_hi - hint_lo;
-      // point t: hint_hi - w 2^(-t / 2), the last one hint_hi itself
-      auto point = [&](int k) {
-        if (k == P - 1) return hint_hi;
-        return hint_hi - w * ((k & 1) ? 0.70710678118654752 : 1.0) * __hiloint2double((1023 - (k >> 1)) << 20, 0);
-      };
-      const int f = ritz_sync_count(sturm_count(tri, blocks, point(t)) == 0);
-      if (f > 0 && f < P) {
-        lo = point(f - 1);
-        hi = point(f);
-        have = true;
+    const int blocks = tri_blocks(m);
+    double lo = 0.0, hi = 0.0, x = 0.0, c2 = 1.0;
+    bool hint = hint_lo < hint_hi, newton = true;
+    if (!hint) tri_interval(tri, m, &lo, &hi);
+    // rounds to go before Newton's iteration; on its failure, rounds to the end
+    int rounds = hint ? 1 : 2;
+    while (true) {
+      for (; rounds > 0 && (newton || hi - lo > 1e-15 * fmax(1.0, fabs(hi))); --rounds) {
+        // hint: point k is hint_hi - w 2^(-k / 2), the last one hint_hi; else P cuts of [lo, hi]
+        const double w = hint ? hint_hi - hint_lo : (hi - lo) * (1.0 / (P + 1));
+        auto point = [&](int k) {
+          if (!hint) return lo + w * (double)(k + 1);
+          if (k == P - 1) return hint_hi;
+          return hint_hi - w * ((k & 1) ? 0.70710678118654752 : 1.0) * __hiloint2double((1023 - (k >> 1)) << 20, 0);
+        };
+        const int f = ritz_sync_count(sturm_count(tri, blocks, point(t)) == 0);
+        if (hint && (f == 0 || f == P)) {
+          hint = false;
+          tri_interval(tri, m, &lo, &hi);
+          rounds = 3;
+          continue;
+        }
+        const double nlo = f > 0 ? point(f - 1) : lo;
+        if (f < P) hi = point(f);
+        lo = nlo;
+        hint = false;
       }
-    }
-    if (!have) tri_interval(tri, m, &lo, &hi);
-    for (int round = 0; round < 9 && hi - lo > 1e-15 * fmax(1.0, fabs(hi)); ++round) {
-      const double w = (hi - lo) * (1.0 / (P + 1));
-      const int f = ritz_sync_count(sturm_count(tri, blocks, lo + w * (double)(t + 1)) == 0);
-      const double nlo = f > 0 ? lo + w * (double)f : lo;
-      if (f < P) hi = lo + w * (double)(f + 1);
-      lo = nlo;
-    }
-    const double r = 0.5 * (lo + hi);
-    if (t < 32) {
-      const double c2 = last_component_sq(tri, m, r);
-      if (t == 0) {
-        s_r = r;
-        s_s2 = c2;
+      // every warp iterates alike (no exchange); without Newton one evaluation, for c2
+      x = newton ? lo : 0.5 * (lo + hi);
+      const double tiny = 1e-16 * fmax(1.0, fabs(hi));
+      bool done = false;
+      for (int it = 0; it < (newton ? 16 : 1) && !done; ++it) {
+        const Minors q = last_minors(tri, m, x);
+        const double inv = -1.0 / q.dp;
+        const double step = q.p * inv;
+        c2 = q.pm1 * inv;
+        done = !newton || !(step > tiny);
+        if (!done) x += step;
       }
+      if (!newton || (done && x <= hi + tiny && isfinite(c2))) break;
+      newton = false;
+      rounds = 9;
+    }
+    if (t == 0) {
+      s_r = x;
+      s_s2 = isnan(c2) ? 1.0 : fmin(fmax(c2, 0.0), 1.0);
     }
   }
   __syncthreads();
@@ -238,65 +283,78 @@ __device__ inline double smallest_eig_block(const double* ag, const double* bg, 
   return r;
 }
 
-// Unit eigenvector of the tridiagonal for eigenvalue theta by inverse iteration (one thread):
-// LU with partial pivoting of (T - theta I), two solves from a constant start.
-__device__ inline void tridiag_eigvec(const double* a, const double* b, int m, double theta, double* s) {
-  if (m == 1) { s[0] = 1.0; return; }
-  double dl[kNcvMax], d[kNcvMax], du[kNcvMax], du2[kNcvMax];
-  int ipiv[kNcvMax];
-  double anorm = 0.0;
-  for (int i = 0; i < m; ++i) {
-    d[i] = a[i] - theta;
-    if (i + 1 < m) { dl[i] = b[i]; du[i] = b[i]; }
-    anorm = fmax(anorm, fabs(a[i]) + (i > 0 ? fabs(b[i - 1]) : 0.0) + (i + 1 < m ? fabs(b[i]) : 0.0));
-  }
-  const double tiny = fmax(anorm, 1e-300) * 1e-15;
-  for (int i = 0; i < m; ++i) du2[i] = 0.0;
-  for (int i = 0; i < m - 1; ++i) {
-    if (fabs(d[i]) >= fabs(dl[i])) {
-      ipiv[i] = i;
-      if (d[i] == 0.0) d[i] = tiny;
-      const double f = dl[i] / d[i];
-      dl[i] = f;
-      d[i + 1] -= f * du[i];
-    } else {
-      ipiv[i] = i + 1;
-      const double f = d[i] / dl[i];
-      d[i] = dl[i];
-      dl[i] = f;
-      const double t = du[i];
-      du[i] = d[i + 1];
-      d[i + 1] = t - f * d[i + 1];
-      if (i < m - 2) {
-        du2[i] = du[i + 1];
-        du[i + 1] = -f * du[i + 1];
-      }
+// The same as a call, for the rare invariant subspace at a restart.
+static __device__ __noinline__ double smallest_eig_call(const double* a, const double* b, int m) {
+  double s2;
+  return smallest_eig_block(a, b, m, &s2);
+}
+
+// Unit eigenvector of the tridiagonal (a, b; size m) for its smallest eigenvalue theta into s (the first
+// warp). With T - theta I factored from the top (pivots u_k) and from the bottom (pivots l_k), the
+// vector is 1 at the row r where the two meet with the smallest gamma_r = u_r + l_r - (a_r - theta) and
+// follows from the pivots' ratios on both sides; gamma_r / |z| is its residual. T - theta I is
+// semidefinite, so neither factorisation needs pivoting. The two chains of divisions run in two
+// lanes at once: 33 rows take about 6 k cycles where inverse iteration in one thread took 52 k.
+// scratch: 4 kNcvMax doubles of shared memory.
+static __device__ __noinline__ void tridiag_eigvec(const double* a, const double* b, int m, double theta, double* s,
+                                                   double* scratch) {
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x;
+  double* u = scratch;
+  double* l = scratch + kNcvMax;
+  double* fu = scratch + 2 * kNcvMax;   // s_k / s_{k+1} above the meeting row
+  double* fl = scratch + 3 * kNcvMax;   // s_k / s_{k-1} below it
+  double big = 0.0;
+  for (int i = lane; i < m; i += 32) big = fmax(big, fmax(fabs(a[i]), i + 1 < m ? fabs(b[i]) : 0.0));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) big = fmax(big, __shfl_xor_sync(0xffffffffu, big, o));
+  const double tiny = fmax(big, 1e-300) * 1e-20;
+  if (lane < 2) {
+    double p = 0.0;
+    for (int i = 0; i < m; ++i) {
+      const int k = lane == 0 ? i : m - 1 - i;
+      const double bb = i == 0 ? 0.0 : b[lane == 0 ? k - 1 : k];
+      const double f = i == 0 ? 0.0 : bb / p;
+      p = (a[k] - theta) - bb * f;
+      if (fabs(p) < tiny) p = tiny;
+      (lane == 0 ? u : l)[k] = p;
+      if (i > 0) (lane == 0 ? fu : fl)[lane == 0 ? k - 1 : k + 1] = -f;
     }
   }
-  ipiv[m - 1] = m - 1;
-  if (d[m - 1] == 0.0) d[m - 1] = tiny;
-  for (int i = 0; i < m; ++i) s[i] = 1.0;
-  for (int iter = 0; iter < 3; ++iter) {
-    // forward: L
-    for (int i = 0; i < m - 1; ++i) {
-      if (ipiv[i] == i) {
-        s[i + 1] -= dl[i] * s[i];
-      } else {
-        const double t = s[i];
-        s[i] = s[i + 1];
-        s[i + 1] = t - dl[i] * s[i];
-      }
+  __syncwarp();
+  // the meeting row
+  double g = 1e300;
+  int r = 0;
+  for (int i = lane; i < m; i += 32) {
+    const double gi = fabs(u[i] + l[i] - (a[i] - theta));
+    if (gi < g) {
+      g = gi;
+      r = i;
     }
-    // backward: U
-    s[m - 1] /= d[m - 1];
-    if (m > 1) s[m - 2] = (s[m - 2] - du[m - 2] * s[m - 1]) / d[m - 2];
-    for (int i = m - 3; i >= 0; --i) s[i] = (s[i] - du[i] * s[i + 1] - du2[i] * s[i + 2]) / d[i];
-    double nrm = 0.0;
-    for (int i = 0; i < m; ++i) nrm += s[i] * s[i];
-    nrm = sqrt(nrm);
-    if (!(nrm > 0.0) || !isfinite(nrm)) { for (int i = 0; i < m; ++i) s[i] = (i == 0) ? 1.0 : 0.0; return; }
-    for (int i = 0; i < m; ++i) s[i] /= nrm;
   }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    const double og = __shfl_xor_sync(0xffffffffu, g, o);
+    const int orow = __shfl_xor_sync(0xffffffffu, r, o);
+    if (og < g || (og == g && orow < r)) {
+      g = og;
+      r = orow;
+    }
+  }
+  if (lane == 0) {
+    s[r] = 1.0;
+    double z = 1.0;
+    for (int k = r - 1; k >= 0; --k) s[k] = z = z * fu[k];
+  } else if (lane == 1) {
+    double z = 1.0;
+    for (int k = r + 1; k < m; ++k) s[k] = z = z * fl[k];
+  }
+  __syncwarp();
+  double nrm = 0.0;
+  for (int i = lane; i < m; i += 32) nrm += s[i] * s[i];
+  nrm = sqrt(warp_sum(nrm));
+  for (int i = lane; i < m; i += 32) s[i] /= nrm;
+  __syncwarp();
 }
 
 // All eigenvalues of the staged tridiagonal in ascending order into out[m] (the CTA): four lanes per
@@ -325,15 +383,22 @@ __device__ inline void all_eigs_block(const double2* tri, int m, double* out) {
 // Implicit restart with exact shifts (the CTA): the m - kk largest Ritz values of the tridiagonal
 // (a, b; size m) are the shifts of implicit QR steps. Each step is a bulge chase on the tridiagonal
 // itself (diagonal d, off-diagonal e and the one bulge entry): rotation r acts on rows and columns
-// r, r + 1 as T <- G T G^T with G = [[c, s], [-s, c]], and on the rows of Q (Qd, m x m row-major,
-// Q <- Q G^T). Rotation r of a shift touches d[r], d[r + 1] and e[r - 1 .. r + 1], so the next shift
-// follows three rotations behind: thread s chases shift s and all chases advance together, m - 1 + 3
+// r, r + 1 as T <- G T G^T with G = [[c, s], [-s, c]], and on the rows of Q (Qg, m x m row-major,
+// Q <- Q G^T). Rotation r of a shift touches d[r], d[r + 1] and e[r - 1 .. r + 1] (the entries that
+// the next rotation changes again stay in registers), so the next shift follows three rotations
+// behind: thread s chases shift s and all chases advance together, m - 1 + 3
 // (m - kk - 1) steps instead of (m - kk)(m - 1), each of them a square root's latency; the other
 // threads apply the rotations of the step before to Q meanwhile. The values are those of one chase after
 // the other. Afterwards Q^T T Q has a leading kk x kk tridiagonal, written back to a and b, and the
 // residual of the kept basis is V Q[:, kk] T+[kk][kk-1] + w Q[m-1][kk-1] (w: the pending unnormalised
-// Lanczos vector). scratch: 2 kTriPad + 7 kNcvMax doubles of shared memory, 16-byte aligned.
-__device__ inline void implicit_restart(AlphaCtrl* C, double* Qd, int m, int kk, double* scratch) {
+// Lanczos vector). scratch: scratch_len >= 2 kTriPad + 7 kNcvMax doubles of shared memory, 16-byte
+// aligned.
+static __device__ __noinline__ void implicit_restart(AlphaCtrl* C, double* Qg, int m, int kk, double* scratch,
+                                                     int scratch_len) {
+  // Q is built in the rest of the scratch when it fits there
+  constexpr int kFixed = 2 * kTriPad + 7 * kNcvMax;
+  const bool inside = kFixed + m * m <= scratch_len;
+  double* Qd = inside ? scratch + kFixed : Qg;
   double2* tri = (double2*)scratch;
   double* d = scratch + 2 * kTriPad;
   double* e = d + kNcvMax;
@@ -350,43 +415,54 @@ __device__ inline void implicit_restart(AlphaCtrl* C, double* Qd, int m, int kk,
   all_eigs_block(tri, m, ritz);
   __syncthreads();
   const int ns = m - kk, steps = (m - 1) + 3 * (ns - 1);
-  double g = 0.0;                              // this chase's bulge T[r+1][r-1]
+  const int nw = blockDim.x >> 5, wid = t >> 5;
+  const int cw = (ns + 31) >> 5;               // warps that chase; the others work on Q (all, if too few)
+  const int qw = nw > cw ? nw - cw : nw, q0 = nw > cw ? wid - cw : wid;
+  // what this chase carries from rotation to rotation: T[r+1][r-1] (the bulge), T[r][r-1], T[r][r] and
+  // T[r+1][r] as the rotation before left them
+  double g = 0.0, xe = 0.0, dr = 0.0, er = 0.0;
   for (int step = 0; step <= steps; ++step) {
     // rotation r = step - 3 s of shift s (the largest Ritz value first)
     const int r = step - 3 * t;
     if (t < ns && r >= 0 && r < m - 1) {
-      const double x = (r == 0) ? d[0] - ritz[m - 1 - t] : e[r - 1];
-      const double z = (r == 0) ? e[0] : g;
-      const double h = x * x + z * z;
-      const double inv = (h == 0.0) ? 0.0 : rsqrt(h);
-      const double c = (h == 0.0) ? 1.0 : x * inv;
-      const double sn = z * inv;
-      if (r > 0) e[r - 1] = h * inv;
-      const double dr = d[r], dn = d[r + 1], er = e[r];
-      d[r] = c * c * dr + 2.0 * c * sn * er + sn * sn * dn;
-      d[r + 1] = sn * sn * dr - 2.0 * c * sn * er + c * c * dn;
-      e[r] = c * sn * (dn - dr) + (c * c - sn * sn) * er;
-      if (r + 2 < m) {
-        g = sn * e[r + 1];
-        e[r + 1] = c * e[r + 1];
+      if (r == 0) {
+        dr = d[0];
+        er = e[0];
+        xe = dr - ritz[m - 1 - t];
+        g = er;
       }
+      const double dn = d[r + 1], en = (r + 2 < m) ? e[r + 1] : 0.0;
+      const double h = fma(xe, xe, g * g);
+      const double inv = (h == 0.0) ? 0.0 : rsqrt(h);
+      const double c = (h == 0.0) ? 1.0 : xe * inv;
+      const double sn = g * inv;
       rot[(step & 1) * kNcvMax + t] = make_double2(c, sn);
+      if (r > 0) e[r - 1] = h * inv;
+      const double cc = c * c, ss = sn * sn, cs = c * sn, t2 = 2.0 * cs * er;
+      d[r] = cc * dr + t2 + ss * dn;
+      xe = fma(cs, dn - dr, (cc - ss) * er);
+      dr = ss * dr - t2 + cc * dn;
+      g = sn * en;
+      er = c * en;
+      if (r == m - 2) {
+        d[m - 1] = dr;
+        e[m - 2] = xe;
+      }
     }
-    // the rotations of the step before, on every row of Q (disjoint pairs of columns)
+    // the rotations of the step before, on every row of Q (disjoint pairs of columns): a warp per row,
+    // a lane per shift
     const int prev = step - 1;
-    if (prev >= 0) {
+    if (prev >= 0 && q0 >= 0) {
       const int s_lo = max(0, (prev - (m - 2) + 2) / 3), s_hi = min(ns - 1, prev / 3);
-      const int cnt = s_hi - s_lo + 1;
-      // the chasing warps come last in the order of the work on Q
-      const int tt = (int)blockDim.x - 1 - t;
-      for (int idx = tt; idx < cnt * m; idx += blockDim.x) {
-        const int s = s_lo + idx % cnt, q = idx / cnt;
-        const int pr = prev - 3 * s;
+      for (int s = s_lo + (t & 31); s <= s_hi; s += 32) {
         const double2 cs = rot[(prev & 1) * kNcvMax + s];
-        double* row = Qd + (long long)q * m + pr;
-        const double pv = row[0], qv = row[1];
-        row[0] = cs.x * pv + cs.y * qv;
-        row[1] = -cs.y * pv + cs.x * qv;
+        double* col = Qd + prev - 3 * s;
+#pragma unroll 4
+        for (int q = q0; q < m; q += qw) {
+          const double pv = col[q * m], qv = col[q * m + 1];
+          col[q * m] = cs.x * pv + cs.y * qv;
+          col[q * m + 1] = -cs.y * pv + cs.x * qv;
+        }
       }
     }
     __syncthreads();
@@ -400,6 +476,8 @@ __device__ inline void implicit_restart(AlphaCtrl* C, double* Qd, int m, int kk,
     C->irl_sigma = Qd[(m - 1) * m + (kk - 1)];
     C->irl_k = kk;
   }
+  if (inside)
+    for (int idx = t; idx < m * m; idx += blockDim.x) Qg[idx] = Qd[idx];
   __syncthreads();
 }
 
@@ -408,6 +486,7 @@ __device__ inline void implicit_restart(AlphaCtrl* C, double* Qd, int m, int kk,
 template <typename T>
 __device__ __forceinline__ double basis_combine(const T* V, long long ldv, long long i, int jmax, const double* coef) {
   double acc = 0.0;
+#pragma unroll 1
   for (int kb = 0; kb <= jmax; kb += 8) {
     T vv[8];
 #pragma unroll
@@ -434,6 +513,15 @@ __device__ __forceinline__ void ld16(const T* p, T* out) {
   for (int r = 0; r < (int)(16 / sizeof(T)); ++r) out[r] = c[r];
 }
 
+// (from shared memory)
+template <typename T>
+__device__ __forceinline__ void lds16(const T* p, T* out) {
+  const typename Vec16<T>::type v = *reinterpret_cast<const typename Vec16<T>::type*>(p);
+  const T* c = reinterpret_cast<const T*>(&v);
+#pragma unroll
+  for (int r = 0; r < (int)(16 / sizeof(T)); ++r) out[r] = c[r];
+}
+
 template <typename T>
 __device__ __forceinline__ void st16(T* p, const T* in) {
   typename Vec16<T>::type v;
@@ -445,60 +533,518 @@ __device__ __forceinline__ void st16(T* p, const T* in) {
 
 // ---- reductions of per-CTA partials --------------------------------------------------------
 
-// Sum part[blk * pw + col] over blocks for cols [0, ncols) into out[col] (fixed order).
-__device__ inline void reduce_partials(const double* part, int pw, int nblocks, int ncols, double* out) {
-  // a warp takes kCols adjacent columns and puts all their loads in flight at once (one L2 round trip
-  // per 256 blocks instead of one per column); each column is summed in the same order as alone
+// Sum part[col * nblocks + blk] over blocks for cols [0, ncols) into out[col] (fixed order; not inlined:
+// one copy serves every phase).
+static __device__ __noinline__ void reduce_partials(const double* part, int nblocks, int ncols, double* out) {
+  // a warp takes up to kCols columns (nw apart) and puts the loads of all of them in flight at once
   constexpr int kCols = 3;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int c0 = wid * kCols; c0 < ncols; c0 += nw * kCols) {
+  for (int c0 = wid; c0 < ncols; c0 += nw * kCols) {
     double acc[kCols];
 #pragma unroll
     for (int cc = 0; cc < kCols; ++cc) acc[cc] = 0.0;
-    for (int b0 = 0; b0 < nblocks; b0 += 32 * 8) {
-      double pv[kCols][8];
+    for (int b0 = lane; b0 < nblocks; b0 += 32 * 5) {
+      double pv[kCols][5];
 #pragma unroll
       for (int cc = 0; cc < kCols; ++cc) {
+        const int c = c0 + cc * nw;
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int bk = b0 + lane + 32 * q;
-          pv[cc][q] = (bk < nblocks && c0 + cc < ncols) ? __ldcg(part + (long long)bk * pw + c0 + cc) : 0.0;
+        for (int q = 0; q < 5; ++q) {
+          pv[cc][q] = 0.0;
+          if (c < ncols && b0 + 32 * q < nblocks) pv[cc][q] = __ldcg(part + (long long)c * nblocks + b0 + 32 * q);
         }
       }
 #pragma unroll
       for (int cc = 0; cc < kCols; ++cc) {
 #pragma unroll
-        for (int q = 0; q < 8; ++q) acc[cc] += pv[cc][q];
+        for (int q = 0; q < 5; ++q) acc[cc] += pv[cc][q];
       }
     }
-#pragma unroll
-    for (int cc = 0; cc < kCols; ++cc) {
-      const double v = warp_sum(acc[cc]);
-      if (lane == 0 && c0 + cc < ncols) out[c0 + cc] = v;
+#pragma unroll 1
+    for (int cc = 0; cc < kCols && c0 + cc * nw < ncols; ++cc) {
+      const double v = warp_sum(cc == 0 ? acc[0] : (cc == 1 ? acc[1] : acc[2]));
+      if (lane == 0) out[c0 + cc * nw] = v;
     }
   }
   __syncthreads();
 }
 
-// Block-reduce NV per-thread values and store them as this CTA's partials [col0, col0 + NV).
-template <int NV>
-__device__ void block_store_partials(const double (&v)[NV], double* part, int pw, int col0, double* sm, int blk) {
+// This CTA's sums of up to three values per thread into out[0..nv) of thread 0..nv-1's return value (one
+// copy, as above). sm: 3 doubles per warp.
+static __device__ __noinline__ double cta_sums(double v0, double v1, double v2, int nv, double* sm) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  double r[NV];
-#pragma unroll
-  for (int q = 0; q < NV; ++q) r[q] = warp_sum(v[q]);
-  __syncthreads();
-  if (lane == 0) {
-#pragma unroll
-    for (int q = 0; q < NV; ++q) sm[wid * NV + q] = r[q];
+#pragma unroll 1
+  for (int q = 0; q < nv; ++q) {
+    const double r = warp_sum(q == 0 ? v0 : (q == 1 ? v1 : v2));
+    if (lane == 0) sm[wid * 3 + q] = r;
   }
   __syncthreads();
-  if (threadIdx.x < NV) {
-    double acc = 0.0;
-    for (int wv = 0; wv < nw; ++wv) acc += sm[wv * NV + threadIdx.x];
-    part[(long long)blk * pw + col0 + threadIdx.x] = acc;
+  double acc = 0.0;
+  if ((int)threadIdx.x < nv)
+    for (int w = 0; w < nw; ++w) acc += sm[w * 3 + threadIdx.x];
+  return acc;
+}
+
+// A phase's sums over all CTAs of a solve. put stores this CTA's sum of a column, block_put reduces NV
+// values per thread first, all_sum waits for every CTA and leaves the totals of `cols` columns in
+// tot[] of every CTA. The partial sums (part: 2 x COLS x CTAs doubles) alternate between two buffers,
+// since a CTA may store those of the next phase while another one still reads these; a single CTA's
+// sums are the totals. sm: 3 doubles per warp of shared memory, tot: COLS.
+template <class Pol, int COLS>
+struct PhaseSums {
+  const Pol& pol;
+  GridSync* gs;
+  double* part;
+  double* sm;
+  double* tot;
+  unsigned int epoch;
+  int buf = 0;
+  __device__ __forceinline__ PhaseSums(const Pol& p, GridSync* g, double* pt, double* s, double* t)
+      : pol(p), gs(g), part(pt), sm(s), tot(t), epoch(p.first_epoch(g)) {}
+  __device__ __forceinline__ bool meet() { return pol.meet(gs, epoch); }
+  __device__ __forceinline__ void put(int col, double v) {
+    const int nblk = pol.nblocks();
+    if (nblk == 1) tot[col] = v;
+    else __stcg(part + ((long long)buf * COLS + col) * nblk + pol.block(), v);
   }
-  __syncthreads();
+  template <int NV>
+  __device__ __forceinline__ void block_put(const double (&v)[NV]) {
+    static_assert(NV <= 3, "staging of block_put");
+    const double acc = cta_sums(v[0], NV > 1 ? v[NV > 1] : 0.0, NV > 2 ? v[NV > 2 ? 2 : 0] : 0.0, NV, sm);
+    if (threadIdx.x < NV) put(threadIdx.x, acc);
+  }
+  __device__ __forceinline__ bool all_sum(int cols) {
+    if (!meet()) return false;
+    if (pol.nblocks() > 1) reduce_partials(part + (long long)buf * COLS * pol.nblocks(), pol.nblocks(), cols, tot);
+    buf ^= 1;
+    return true;
+  }
+};
+
+// Sums of N (a power of two) values per lane over the warp: lane l returns the sum of value
+// l / (32 / N). Halving the values at each of the first exchanges takes N - 1 + log2(32 / N) exchanges
+// instead of 5 N.
+template <int N>
+__device__ __forceinline__ double warp_sum_batch(double (&v)[N]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = N / 2, o = 16; h >= 1; h >>= 1, o >>= 1) {
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double keep = (lane & o) ? v[q + h] : v[q], give = (lane & o) ? v[q] : v[q + h];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+#pragma unroll
+  for (int o = 16 / N; o >= 1; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+// ---- the vector phases of a Lanczos step -----------------------------------------------------
+// (Inlined: a call would save and restore tens of registers of 512 threads through local memory, which
+// cost 4 to 15 us a phase at n = 2^20.)
+
+// P2: the three-term step w' = w - a3 V[j] - b3 V[j-1] (first pass only), then this warp's parts of the
+// reorthogonalisation coefficients h_k = V_k . w' (k <= j) and of w' . w' in red[warp][0 .. j + 1].
+// Removing the dominant components explicitly first keeps the single Gram-Schmidt pass stable. w' goes to
+// u (whose gathers are over), so that w can be read by several groups of threads.
+template <typename T>
+__device__ __forceinline__ void lanczos_dots(const T* V, long long ldv, const T* w, T* u, long long nvt, int j, int pass2,
+                                          double a3, double b3, double* red_all, int gtid, int nthreads) {
+  constexpr int VW = 16 / sizeof(T);
+  const int lane = tid_here() & 31;
+  double* red = red_all + (tid_here() >> 5) * kPartCols;
+  const T* Vj = V + (long long)j * ldv;
+  const T* Vm = V + (long long)(j > 0 ? j - 1 : 0) * ldv;
+  for (int c = lane; c <= j + 1; c += 32) red[c] = 0.0;
+  __syncwarp();
+  // threads to spare: group g of them takes the batches g, g + groups, ... of basis vectors (each forms
+  // w' itself), so that a small problem waits for one batch of loads instead of all of them in turn
+  constexpr int KB = 4;
+  const int batches = (j + KB) / KB;
+  const int nvw = ((int)nvt + 31) & ~31;
+  const int groups = max(1, min(batches, nthreads / nvw));
+  const int span = (nthreads / groups) & ~31;
+  const int grp = gtid / span, pos = gtid - grp * span;
+  if (grp >= groups) return;
+  for (int kb = grp * KB; kb <= j; kb += groups * KB) {
+    const T* Vk = V + (long long)kb * ldv;
+    double acc[KB], ww = 0.0;
+#pragma unroll
+    for (int q = 0; q < KB; ++q) acc[q] = 0.0;
+    for (int iv = pos; iv < (int)nvt; iv += span) {
+      const long long i0 = (long long)iv * VW;
+      // every load of the position before the first use or store, so that all are in flight
+      T wv[VW], vj[VW], vm[VW], vk[KB][VW];
+      ld16(w + i0, wv);
+      if (!pass2) {
+        ld16(Vj + i0, vj);
+        ld16(Vm + i0, vm);
+      }
+#pragma unroll
+      for (int q = 0; q < KB; ++q)
+        if (kb + q <= j) ld16(Vk + q * ldv + i0, vk[q]);
+      if (!pass2) {
+#pragma unroll
+        for (int r = 0; r < VW; ++r) {
+          double x = (double)wv[r] - a3 * (double)vj[r];
+          if (j > 0) x -= b3 * (double)vm[r];
+          wv[r] = (T)x;
+        }
+        if (kb == 0) st16(u + i0, wv);
+      }
+#pragma unroll
+      for (int r = 0; r < VW; ++r) {
+        const double wd = (double)wv[r];
+        if (kb == 0) ww += wd * wd;
+#pragma unroll
+        for (int q = 0; q < KB; ++q)
+          if (kb + q <= j) acc[q] += (double)vk[q][r] * wd;
+      }
+    }
+    const double d = warp_sum_batch(acc);
+    if ((lane & 7) == 0 && kb + (lane >> 3) <= j) red[kb + (lane >> 3)] = d;
+    if (kb == 0) {
+      ww = warp_sum(ww);
+      if (lane == 0) red[j + 1] = ww;
+    }
+  }
+}
+
+// P3: w = src - sum_k h_k V_k and u = sigma w; returns this thread's part of w . w. With threads to
+// spare, up to 8 lanes of a warp share a position and split its basis vectors between them.
+template <typename T>
+__device__ __forceinline__ double lanczos_update(const T* V, long long ldv, const T* src, const T* sigma, T* w, T* u,
+                                                 long long nvt, int j, const double* h, int gtid, int nthreads) {
+  constexpr int VW = 16 / sizeof(T), KB = 4;
+  double ww = 0.0;
+  int sl = 0;
+  while (sl < 3 && (nvt << (sl + 1)) <= nthreads) ++sl;
+  const int lane = tid_here() & 31, per = 32 >> sl, sub = lane >> (5 - sl), lanes = 1 << sl;
+  for (long long iv0 = (long long)(gtid >> 5) * per; iv0 < nvt; iv0 += nthreads >> sl) {
+    const long long iv = iv0 + (lane & (per - 1)), i0 = iv * VW;
+    const bool mine = iv < nvt;
+    T wv[VW];
+    double corr[VW];
+#pragma unroll
+    for (int r = 0; r < VW; ++r) corr[r] = 0.0;
+    if (mine) {
+      ld16(src + i0, wv);
+      for (int kb = sub; kb <= j; kb += KB * lanes) {
+        T vk[KB][VW];
+#pragma unroll
+        for (int q = 0; q < KB; ++q)
+          if (kb + q * lanes <= j) ld16(V + (long long)(kb + q * lanes) * ldv + i0, vk[q]);
+#pragma unroll
+        for (int q = 0; q < KB; ++q) {
+          if (kb + q * lanes <= j) {
+            const double hk = h[kb + q * lanes];
+#pragma unroll
+            for (int r = 0; r < VW; ++r) corr[r] += hk * (double)vk[q][r];
+          }
+        }
+      }
+    }
+#pragma unroll 1
+    for (int o = per; o < 32; o <<= 1) {
+#pragma unroll
+      for (int r = 0; r < VW; ++r) corr[r] += __shfl_xor_sync(0xffffffffu, corr[r], o);
+    }
+    if (mine && sub == 0) {
+      T sg[VW], uv[VW];
+      ld16(sigma + i0, sg);
+#pragma unroll
+      for (int r = 0; r < VW; ++r) {
+        wv[r] = (T)((double)wv[r] - corr[r]);
+        uv[r] = sg[r] * wv[r];
+        ww += (double)wv[r] * (double)wv[r];
+      }
+      st16(w + i0, wv);
+      st16(u + i0, uv);
+    }
+  }
+  return ww;
+}
+
+// The same two phases for problems that fill the GPU: every CTA owns a contiguous range of rows and
+// streams the vectors' tiles of it (kStreamTile bytes a vector, kStreamVecs vectors a group) into
+// shared memory with bulk asynchronous copies, kStreamBufs groups in flight. What bounds them is the
+// reading of the basis (from L2 and HBM); loads held in registers either keep too few bytes in flight
+// or take so many registers that the persistent kernel spills them through an L1 that the panels leave
+// 30 KB. At n = 2^20 (20 vectors) the dots move 3.3 TB/s and the update 3.8 TB/s with the FP32 to FP64
+// conversions (16 a cycle and SM) next in line; one step's dots and update went from 73 to 52.5 us,
+// Ritz test and barriers included.
+constexpr int kStreamTile = 16 * 1024;
+constexpr int kStreamVecs = 4;
+__host__ __device__ constexpr int stream_bufs(int elem) { return elem == 4 ? 3 : 2; }
+__host__ __device__ constexpr int stream_smem_bytes(int elem) { return stream_bufs(elem) * kStreamVecs * kStreamTile; }
+
+template <typename T>
+struct VecStream {
+  static constexpr int VW = 16 / sizeof(T);
+  static constexpr int kBufs = stream_bufs(sizeof(T));
+  static constexpr int kTileRows = kStreamTile / sizeof(T);
+  static constexpr int kChunks = kStreamTile / (16 * kThreads);   // 16-byte chunks of a tile per thread
+  char* smem;
+  unsigned long long* bars;   // kBufs mbarriers of one arrival
+  unsigned& par;              // their phase bits
+  int* err;
+  long long r0;               // first row, rows of the range and of a tile, number of tiles
+  int rows, sub, tiles;
+
+  // the CTA's range of n_pad rows (a multiple of VW)
+  __device__ __forceinline__ VecStream(char* sm, unsigned long long* b, unsigned& p, int* e, long long n_pad, int blk,
+                                       int nblk)
+      : smem(sm), bars(b), par(p), err(e) {
+    const long long per = ((n_pad + nblk - 1) / nblk + VW - 1) / VW * VW;
+    r0 = min(n_pad, per * blk);
+    rows = (int)(min(n_pad, r0 + per) - r0);
+    tiles = (rows + kTileRows - 1) / kTileRows;
+    sub = tiles ? ((rows + tiles - 1) / tiles + VW - 1) / VW * VW : 0;
+  }
+  __device__ __forceinline__ int tile_rows(int t) const { return min(sub, rows - t * sub); }
+  __device__ __forceinline__ long long tile_row0(int t) const { return r0 + (long long)t * sub; }
+
+  // Runs nv vectors (vec(v): the v-th one's base) over all tiles. begin(t) and end(t) bracket a tile;
+  // group(t, g, m, base) works on vectors 4 g .. 4 g + m - 1 of tile t, whose tiles lie kStreamTile
+  // apart from base. False, with SA_ERR_BARRIER_TIMEOUT in *err, if a copy does not complete in time.
+  template <class Vec, class Begin, class Group, class End>
+  __device__ __forceinline__ bool run(int nv, Vec&& vec, Begin&& begin, Group&& group, End&& end) {
+    const int ng = (nv + kStreamVecs - 1) / kStreamVecs, total = ng * tiles;
+    // copies of group k, by the first lanes of one warp (one vector each: in a single thread their issue
+    // would hold up its warp, and with it the group)
+    auto issue = [&](int k) {
+      const int q = threadIdx.x & 31;
+      const int t = k / ng, g = k - t * ng, b = k % kBufs;
+      const int m = min(kStreamVecs, nv - g * kStreamVecs);
+      const unsigned bytes = (unsigned)(tile_rows(t) * sizeof(T));
+      if (q == 0)
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&bars[b])), "r"(bytes * m)
+                     : "memory");
+      __syncwarp();
+      if (q < m) {
+        fence_proxy_async();
+        bulk_load(smem + (b * kStreamVecs + q) * kStreamTile, vec(g * kStreamVecs + q) + tile_row0(t), bytes, &bars[b]);
+      }
+    };
+    const int wid = threadIdx.x >> 5;
+    if (wid < kBufs && wid < total) issue(wid);
+    int k = 0;
+    for (int t = 0; t < tiles; ++t) {
+      begin(t);
+      for (int g = 0; g < ng; ++g, ++k) {
+        const int b = k % kBufs;
+        const unsigned par0 = par;
+        bool late = false;
+        for (unsigned long long spins = 0; !mbar_try_wait(&bars[b], (par0 >> b) & 1u);)
+          if (++spins > kPanelSpinLimit) {
+            late = true;
+            break;
+          }
+        late = __any_sync(0xffffffffu, late);
+        par ^= 1u << b;
+        if (!late) group(t, g, min(kStreamVecs, nv - g * kStreamVecs), smem + b * kStreamVecs * kStreamTile);
+        if (__syncthreads_or(late)) {
+          // as in the panel SpMV: record, wait (bounded) for the copies in flight, return together
+          if (threadIdx.x == 0) {
+            atomicExch(err, SA_ERR_BARRIER_TIMEOUT);
+            for (int q = k; q < k + kBufs && q < total; ++q) {
+              const int qb = q % kBufs;
+              for (unsigned long long spins = 0; !mbar_try_wait(&bars[qb], (par0 >> qb) & 1u);)
+                if (++spins > kPanelSpinLimit) break;
+            }
+          }
+          __syncthreads();
+          return false;
+        }
+        if (wid == k % kWarps && k + kBufs < total) issue(k + kBufs);
+      }
+      end(t);
+    }
+    return true;
+  }
+};
+
+// P2 streamed. The vectors in order: w, V[j], V[j-1], V[0], V[1], ..., V[j-2]; the first three give w',
+// which stays in registers for the tile.
+template <typename T>
+__device__ __forceinline__ bool stream_dots(VecStream<T>& S, const T* V, long long ldv, const T* w, T* u, int j, int pass2,
+                                            double a3, double b3, double* red_all) {
+  constexpr int VW = VecStream<T>::VW, NC = VecStream<T>::kChunks;
+  const int tid = tid_here(), lane = tid & 31;
+  double* red = red_all + (tid >> 5) * kPartCols;
+  for (int c = lane; c <= j + 1; c += 32) red[c] = 0.0;
+  __syncwarp();
+  auto index = [&](int v) { return v == 1 ? j : (v == 2 ? j - 1 : v - 3); };
+  double wd[NC][VW], ww = 0.0;
+  const bool ok = S.run(
+      j + 2, [&](int v) { return v == 0 ? w : V + (long long)index(v) * ldv; }, [](int) {},
+      [&](int t, int g, int m, const char* base) {
+        const T* x = (const T*)base;
+        const int cnt = S.tile_rows(t);
+        if (g == 0) {
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const int at = (c * kThreads + tid) * VW;
+            T wv[VW];
+#pragma unroll
+            for (int r = 0; r < VW; ++r) wv[r] = T(0);
+            if (at < cnt) {
+              lds16(x + at, wv);
+              if (!pass2) {
+                T vj[VW], vm[VW];
+                lds16(x + kStreamTile / sizeof(T) + at, vj);
+                if (j > 0) lds16(x + 2 * (kStreamTile / sizeof(T)) + at, vm);
+#pragma unroll
+                for (int r = 0; r < VW; ++r) {
+                  double y = (double)wv[r] - a3 * (double)vj[r];
+                  if (j > 0) y -= b3 * (double)vm[r];
+                  wv[r] = (T)y;
+                }
+                st16(u + S.tile_row0(t) + at, wv);
+              }
+            }
+#pragma unroll
+            for (int r = 0; r < VW; ++r) {
+              wd[c][r] = (double)wv[r];
+              ww += wd[c][r] * wd[c][r];
+            }
+          }
+        }
+        double acc[kStreamVecs];
+#pragma unroll
+        for (int q = 0; q < kStreamVecs; ++q) {
+          acc[q] = 0.0;
+          if (q < m && (g > 0 || q > 0)) {
+#pragma unroll
+            for (int c = 0; c < NC; ++c) {
+              const int at = (c * kThreads + tid) * VW;
+              if (at < cnt) {
+                T vk[VW];
+                lds16(x + q * (kStreamTile / sizeof(T)) + at, vk);
+#pragma unroll
+                for (int r = 0; r < VW; ++r) acc[q] += (double)vk[r] * wd[c][r];
+              }
+            }
+          }
+        }
+        const double d = warp_sum_batch(acc);
+        const int q = lane >> 3, v = g * kStreamVecs + q;
+        if ((lane & 7) == 0 && q < m && v > 0) red[index(v)] += d;
+      },
+      [](int) {});
+  ww = warp_sum(ww);
+  if (lane == 0) red[j + 1] = ww;
+  return ok;
+}
+
+// P3 streamed: the vectors in order src, sigma, V[0], ..., V[j]. Adds this thread's part of w . w to ww.
+template <typename T>
+__device__ __forceinline__ bool stream_update(VecStream<T>& S, const T* V, long long ldv, const T* src, const T* sigma,
+                                              T* w, T* u, int j, const double* h, double& ww) {
+  constexpr int VW = VecStream<T>::VW, NC = VecStream<T>::kChunks;
+  const int tid = tid_here();
+  T wv[NC][VW], sg[NC][VW];
+  double corr[NC][VW];
+  return S.run(
+      j + 3, [&](int v) { return v == 0 ? src : (v == 1 ? sigma : V + (long long)(v - 2) * ldv); },
+      [&](int) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c)
+#pragma unroll
+          for (int r = 0; r < VW; ++r) corr[c][r] = 0.0;
+      },
+      [&](int t, int g, int m, const char* base) {
+        const T* x = (const T*)base;
+        const int cnt = S.tile_rows(t);
+#pragma unroll
+        for (int q = 0; q < kStreamVecs; ++q) {
+          if (q >= m) break;
+          const double hk = (g > 0 || q > 1) ? h[g * kStreamVecs + q - 2] : 0.0;
+#pragma unroll
+          for (int c = 0; c < NC; ++c) {
+            const int at = (c * kThreads + tid) * VW;
+            if (at < cnt) {
+              T vk[VW];
+              lds16(x + q * (kStreamTile / sizeof(T)) + at, vk);
+              if (g == 0 && q < 2) {
+#pragma unroll
+                for (int r = 0; r < VW; ++r) (q == 0 ? wv : sg)[c][r] = vk[r];
+              } else {
+#pragma unroll
+                for (int r = 0; r < VW; ++r) corr[c][r] += hk * (double)vk[r];
+              }
+            }
+          }
+        }
+      },
+      [&](int t) {
+        const int cnt = S.tile_rows(t);
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          const int at = (c * kThreads + tid) * VW;
+          if (at < cnt) {
+            T uv[VW];
+#pragma unroll
+            for (int r = 0; r < VW; ++r) {
+              wv[c][r] = (T)((double)wv[c][r] - corr[c][r]);
+              uv[r] = sg[c][r] * wv[c][r];
+              ww += (double)wv[c][r] * (double)wv[c][r];
+            }
+            st16(w + S.tile_row0(t) + at, wv[c]);
+            st16(u + S.tile_row0(t) + at, uv);
+          }
+        }
+      });
+}
+
+// Restart: kept basis V[0..kk) <- V Q[:, 0..kk) and the new residual f = V Q[:, kk] beta + w sig (in w,
+// with u = sigma f), row by row in place (all m inputs of a row are read before its kk outputs are
+// written); returns this thread's part of f . f. q: m x (kk + 1) in shared memory. KK: kk when it is
+// known at compile time (the default), else 0.
+template <typename T, int KK>
+__device__ __forceinline__ double restart_basis(T* V, long long ldv, T* w, T* u, const T* sigma, long long n, int m, int kk_,
+                                             const double* q, double beta, double sig, long long gtid,
+                                             long long nthreads) {
+  constexpr int KM = KK > 0 ? KK : kRestartMax;
+  const int kk = KK > 0 ? KK : kk_;
+  double ff = 0.0;
+#pragma unroll 1
+  for (long long i = gtid; i < n; i += nthreads) {
+    double y[KM + 1];
+#pragma unroll
+    for (int c = 0; c <= KM; ++c) y[c] = 0.0;
+    const double wi = (double)__ldcg(w + i);
+#pragma unroll 1
+    for (int r0 = 0; r0 < m; r0 += 8) {
+      T vr[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) vr[r] = (r0 + r < m) ? __ldcg(V + (long long)(r0 + r) * ldv + i) : T(0);
+#pragma unroll
+      for (int r = 0; r < 8; ++r) {
+        if (r0 + r < m) {
+          const double* qr = q + (r0 + r) * (kk + 1);
+#pragma unroll
+          for (int c = 0; c <= KM; ++c)
+            if (KK > 0 || c <= kk) y[c] += (double)vr[r] * qr[c];
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < KM; ++c)
+      if (KK > 0 || c < kk) V[(long long)c * ldv + i] = (T)y[c];
+    double yk = y[KM];
+    if (KK == 0) {
+#pragma unroll
+      for (int c = 0; c <= KM; ++c)
+        if (c == kk) yk = y[c];
+    }
+    const T f = (T)(yk * beta + wi * sig);
+    w[i] = f;
+    u[i] = sigma[i] * f;
+    ff += (double)f * (double)f;
+  }
+  return ff;
 }
 
 template <typename T>
@@ -510,72 +1056,183 @@ __device__ __forceinline__ unsigned long long word_mix(long long widx, unsigned 
 
 // ---- the alpha-solve kernel ----------------------------------------------------------------
 
-// Shared scratch of the reductions: per-warp partials of block_store_partials (NW x 9) and the
-// reduced columns of the dot phase (up to 2 kNcvMax + kDotBatch + 8 partial columns).
-constexpr int kRedCols = 2 * kNcvMax + kDotBatch + 8;
+// Shared work space of a CTA: the SpMV's staging, the warps' dots, or the tridiagonal solvers' and the
+// restart's scratch (never two of them at a time).
+template <typename T, int NW>
+union AlphaWork {
+  SpmvSmem<T, NW> spmv;
+  double dots[NW * kPartCols];
+  double restart[kNcvMax * (kRestartMax + 1)];
+};
 
-// NW: warps per CTA at most (sizes the shared staging). kLayouts: the operator may use the column-panel
-// layout or the L2 column splits (the single-problem kernel); without it only the work list is compiled
-// (the batch kernel, whose register budget the other paths would spill).
-template <typename T, typename RP, class Pol, int NW = kWarps, bool kLayouts = true>
+template <typename T, int NW>
+__device__ __forceinline__ AlphaWork<T, NW>& alpha_work() {
+  __shared__ __align__(16) AlphaWork<T, NW> w;
+  return w;
+}
+
+// What a row does with its sum s = sum_j val_ij u_j: in a Lanczos step (P1) V[j] = w * inv_b and
+// w <- S V[j], adding V[j] . w to acc; in the final pass (last) |S y - theta y|^2 is added to it.
+template <typename T>
+struct RowStep {
+  const T* xin;   // w, or y in the final pass
+  const T* sigma;
+  T* vj;
+  T* w;
+  T rho, inv_b;
+  double theta;
+  bool last;
+  double acc;
+  __device__ __forceinline__ RowInputs<T> pre(long long r) const { return RowInputs<T>{__ldcg(xin + r), __ldcg(sigma + r)}; }
+  __device__ __forceinline__ void fin(long long r, T s, const RowInputs<T>& in) {
+    const T wr = in.x;
+    const T sw = rho * wr - in.s * s;
+    if (last) {
+      const double rr = (double)sw - theta * (double)wr;
+      acc += rr * rr;
+    } else {
+      const T vr = wr * inv_b;
+      const T wn = sw * inv_b;
+      vj[r] = vr;
+      w[r] = wn;
+      acc += (double)vr * (double)wn;
+    }
+  }
+};
+
+// The operator layouts.
+template <typename T>
+__device__ __forceinline__ bool panel_pass(const PanelArgs& P, const T* u, int blk, int nblk, unsigned long long* bars,
+                                        unsigned& par, int* err, RowStep<T>& out) {
+  extern __shared__ __align__(128) char panel_smem[];
+  RowStep<T> f = out;
+  unsigned pr = par;
+  const bool ok = panel_spmv<T>(P, u, blk, nblk, panel_smem, bars, pr, err, [&](long long r) { return f.pre(r); },
+                                [&](long long r, T s, const RowInputs<T>& in) { f.fin(r, s, in); });
+  par = pr;
+  out.acc = f.acc;
+  return ok;
+}
+
+// mode: bit 0 the first of the passes that make up a row's sum, bit 1 the last one (sums between the
+// passes in `part`).
+template <typename T, typename RP, int NW>
+__device__ __forceinline__ void items_pass(const SpmvArgs<T, RP>& S, const T* u, int gwarp, int nwarps, RowStep<T>& out,
+                                        T* part, int mode) {
+  RowStep<T> f = out;
+  const SpmvArgs<T, RP> L = S;
+  spmv_items<T, RP, false, NW>(L, u, gwarp, nwarps, alpha_work<T, NW>().spmv, [&](long long r, T s) {
+    const T sum = (mode & 1) ? s : __ldcg(part + r) + s;
+    if (mode & 2) f.fin(r, sum, f.pre(r));
+    else __stcg(part + r, sum);
+  });
+  out.acc = f.acc;
+}
+
+// What a kernel is compiled for (all in one would hold more registers than a thread has, and spill them
+// through the little L1 that the panels leave): the work list with register-held vector phases (small
+// problems and the batch kernel); the column panels with streamed vector phases; the work list or the
+// L2 column splits with streamed vector phases.
+enum AlphaMode : int { ALPHA_SMALL = 0, ALPHA_PANEL = 1, ALPHA_LARGE = 2 };
+
+// NW: warps per CTA at most (sizes the shared staging).
+template <typename T, typename RP, class Pol, int NW, int kMode>
 __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol& pol) {
   static_assert(2 * kTriPad + 7 * kNcvMax <= kNcvMax * (kRestartMax + 1), "restart scratch too small");
-  static_assert(NW * (kDotBatch + 1) <= kRedCols, "reduction scratch too small");
-  __shared__ double sm[kRedCols];
-  __shared__ double sh[kNcvMax];
-  __shared__ double s_theta, s_s2;
-  __shared__ SpmvSmem<T, NW> ssp;
-  __shared__ __align__(16) double sq[kNcvMax * (kRestartMax + 1)];
-  __shared__ unsigned long long pbars[kPanelBufs];
-  extern __shared__ __align__(128) char panel_smem[];
-  AlphaCtrl* C = A.ctrl;
+  AlphaWork<T, NW>& work = alpha_work<T, NW>();
+  __shared__ double sm[3 * NW];
+  __shared__ double tot[kPartCols];   // totals of the last phase's partial sums
+  __shared__ AlphaCtrl ctl;
+  __shared__ unsigned long long pbars[kPanelBufs], vbars[stream_bufs(sizeof(T))];
+  double* const sq = work.restart;
+  AlphaCtrl* const C = &ctl;     // this CTA's copy of the control block
+  AlphaCtrl* const G = A.ctrl;   // barrier, flags and signature of the whole grid; the copy that is published
   const long long n = A.n;
   const long long gtid = pol.tid();
   const long long nthreads = pol.nthr();
+  const int nblk = pol.nblocks(), blk = pol.block();
   const sa_alpha_params& P = A.p;
   const double rho = P.rho;
   const double bound = 10.0 * (P.rho + P.gershgorin);
   const int ncv = P.ncv;
+  constexpr int VW = 16 / sizeof(T);
+  const long long nvt = (n + VW - 1) / VW;   // positions of the vector phases
   unsigned ppar = 0;   // phase bits of the panel barriers
-  if (kLayouts && A.use_panel) panel_init(pbars);
-  // one operator application: fin(row, sum_j val_ij u_j) once per row; false on a timed-out wait
-  auto apply = [&](auto&& fin) -> bool {
-    if constexpr (kLayouts) {
-      if (A.use_panel)
-        return panel_spmv<T>(A.panel, A.u, pol.block(), pol.nblocks(), panel_smem, pbars, ppar, &C->gs.error, fin);
-    }
-    if constexpr (kLayouts) {
-      if (A.n_splits > 0) {
-        // pass s adds the row sums of split s; a barrier makes them visible to the next pass
-        for (int q = 0; q < A.n_splits; ++q) {
-          const bool first = q == 0, last = q + 1 == A.n_splits;
-          spmv_items<T, RP>(A.split[q], A.u, gtid >> 5, nthreads >> 5, ssp, [&](long long r, T acc) {
-            const T sum = first ? acc : __ldcg(A.split_part + r) + acc;
-            if (last) fin(r, sum);
-            else __stcg(A.split_part + r, sum);
-          });
-          if (!last && !pol.sync(&C->gs)) return false;
-        }
-        return true;
+  if (kMode == ALPHA_PANEL) panel_init(pbars, kPanelBufs);
+  unsigned vpar = 0;   // and of the vector streams'
+  if (kMode != ALPHA_SMALL) panel_init(vbars, stream_bufs(sizeof(T)));
+  PhaseSums<Pol, kPartCols> sums(pol, &G->gs, A.part, sm, tot);
+  // one operator application (this thread's sum goes to f.acc); false on a timed-out wait
+  auto apply = [&](RowStep<T>& f) -> bool {
+    if constexpr (kMode == ALPHA_PANEL) {
+      return panel_pass<T>(A.panel, A.u, blk, nblk, pbars, ppar, &G->gs.error, f);
+    } else {
+      // pass q adds the row sums of split q (the work list is one pass); a barrier makes them visible to
+      // the next pass
+      const int passes = kMode == ALPHA_LARGE && A.n_splits > 0 ? A.n_splits : 1;
+#pragma unroll 1
+      for (int q = 0; q < passes; ++q) {
+        const bool last = q + 1 == passes;
+        const SpmvArgs<T, RP>& S = kMode == ALPHA_LARGE && A.n_splits > 0 ? A.split[q] : A.S;
+        items_pass<T, RP, NW>(S, A.u, (int)(pol.tid() >> 5), (int)(nthreads >> 5), f, A.split_part,
+                              (q == 0 ? 1 : 0) | (last ? 2 : 0));
+        if (!last && !sums.meet()) return false;
       }
+      return true;
     }
-    spmv_items<T, RP>(A.S, A.u, gtid >> 5, nthreads >> 5, ssp, fin);
-    return true;
   };
 
   // phase timer: CTA 0 thread 0 charges the time since the previous barrier exit to a phase
-  unsigned long long t_mark = (pol.block() == 0 && threadIdx.x == 0) ? global_ns() : 0ull;
+  unsigned long long t_mark = (blk == 0 && threadIdx.x == 0) ? global_ns() : 0ull;
   auto mark = [&](int ph) {
-    if (pol.block() == 0 && threadIdx.x == 0) {
+    if (blk == 0 && threadIdx.x == 0) {
       const unsigned long long t = global_ns();
       C->tph[ph] += t - t_mark;
       t_mark = t;
     }
   };
+  // the control block as the host and the batched sweep read it (all but the barrier, the flag and the
+  // signature, which the grid shares)
+  auto publish = [&] {
+    if (blk != 0) return;
+    __syncthreads();
+    for (int i = threadIdx.x; i < kNcvMax; i += blockDim.x) {
+      G->a[i] = C->a[i];
+      G->b[i] = C->b[i];
+      G->h[i] = C->h[i];
+      G->s[i] = C->s[i];
+    }
+    if (threadIdx.x == 0) {
+      G->theta = C->theta;
+      G->inv_b = C->inv_b;
+      G->ww = C->ww;
+      G->scale = C->scale;
+      G->nrm_y = C->nrm_y;
+      G->rr = C->rr;
+      G->j = C->j;
+      G->action = C->action;
+      G->iters = C->iters;
+      G->restarts = C->restarts;
+      G->mode = C->mode;
+      G->pred_residual = C->pred_residual;
+      G->pred_accepted = C->pred_accepted;
+      G->status = C->status;
+      G->degree_scale = C->degree_scale;
+      G->align_dot = C->align_dot;
+      G->res_est = C->res_est;
+      G->bytes = C->bytes;
+      G->spmvs = C->spmvs;
+      for (int q = 0; q < 6; ++q) G->tph[q] = C->tph[q];
+    }
+  };
 
   // ---------------- P0: sigma, degree scale, start vector --------------------------------------
   int mode = P.start_mode;
-  if (pol.block() == 0 && threadIdx.x == 0) {
+  if (threadIdx.x == 0) {
+    if (blk == 0) {
+      G->nonfinite = 0;
+      G->sig = 0ull;
+    }
     C->mode = mode;
     C->test_pred = (mode == SA_START_DIAGONAL || mode == SA_START_SECANT || mode == SA_START_TANGENT) ? 1 : 0;
     C->pred_accepted = -1;
@@ -583,15 +1240,27 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
     C->iters = 0;
     C->restarts = 0;
     C->status = SA_OK;
-    C->nonfinite = 0;
-    C->sig = 0ull;
     C->secant_sign = 1;
     C->bytes = 0.0;
     C->spmvs = 0;
+    C->theta = C->res_est = C->nrm_y = C->rr = C->scale = C->align_dot = C->ww = 0.0;
+    C->j = 0;
+    C->pass2 = 0;
     for (int q = 0; q < 6; ++q) C->tph[q] = 0ull;
+  }
+  // the vector phases move whole 16-byte positions: the rows of the last one past n are zeros in
+  // every vector (they are inside each array's allocation) and stay zeros
+  {
+    const int past = (int)(nvt * VW - n);
+    for (long long i = gtid; i < (long long)past * (ncv + 3); i += nthreads) {
+      const int k = (int)(i / past);
+      T* const x = k < ncv ? A.V + (long long)k * A.ldv : (k == ncv ? A.w : (k == ncv + 1 ? A.u : A.sigma));
+      x[n + i % past] = T(0);
+    }
   }
   {
     double ds = 0.0;
+#pragma unroll 1
     for (long long i = gtid; i < n; i += nthreads) {
       const double ldi = (double)A.ld[i];
       const double ai = A.aoff ? P.alpha + A.aoff[i] : P.alpha;
@@ -601,36 +1270,35 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
       ds += exp2(logD);
     }
     double v[1] = {ds};
-    block_store_partials<1>(v, A.part, A.pw, 0, sm, pol.block());
+    sums.block_put(v);
   }
-  if (!pol.sync(&C->gs, [&] {
-        reduce_partials(A.part, A.pw, pol.nblocks(), 1, sh);
-        if (threadIdx.x == 0) {
-          C->degree_scale = sh[0];
-          C->bytes += (double)n * (8.0 + sizeof(T));
-        }
-      })) return;
+  if (!sums.all_sum(1)) return;
+  if (threadIdx.x == 0) {
+    C->degree_scale = tot[0];
+    C->bytes += (double)n * (8.0 + sizeof(T));
+  }
   mark(0);
 
   if (mode == SA_START_SECANT && A.has_prev) {
     double v[1] = {0.0};
+#pragma unroll 1
     for (long long i = gtid; i < n; i += nthreads) v[0] += (double)A.ylast[i] * (double)A.yprev[i];
-    block_store_partials<1>(v, A.part, A.pw, 0, sm, pol.block());
-    if (!pol.sync(&C->gs, [&] {
-          reduce_partials(A.part, A.pw, pol.nblocks(), 1, sh);
-          if (threadIdx.x == 0) {
-            C->secant_sign = (sh[0] < 0.0) ? -1 : 1;
-            C->bytes += 2.0 * (double)n * sizeof(T);
-          }
-        })) return;
+    sums.block_put(v);
+    if (!sums.all_sum(1)) return;
+    if (threadIdx.x == 0) {
+      C->secant_sign = (tot[0] < 0.0) ? -1 : 1;
+      C->bytes += 2.0 * (double)n * sizeof(T);
+    }
     mark(0);
   }
 
   while (true) {   // P0 loop (repeats for a predictor fallback or rejection)
-    mode = vload(&C->mode);
-    const int sgn = vload(&C->secant_sign);
+    __syncthreads();
+    mode = C->mode;
+    const int sgn = C->secant_sign;
     const unsigned long long key = splitmix64(P.seed ^ 0x57A27000ull) ^ splitmix64((unsigned long long)P.stream_id + 0x1234567ull);
     double v[3] = {0.0, 0.0, 0.0};   // ||v0||^2, ||s||^2 (secant), ||y||^2 (secant)
+#pragma unroll 1
     for (long long i = gtid; i < n; i += nthreads) {
       double x;
       if (mode == SA_START_RANDOM) {
@@ -659,430 +1327,307 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
       v[0] += (double)xt * (double)xt;
     }
     v[2] = v[0];
-    block_store_partials<3>(v, A.part, A.pw, 0, sm, pol.block());
-    if (!pol.sync(&C->gs, [&] {
-          reduce_partials(A.part, A.pw, pol.nblocks(), 3, sh);
-          if (threadIdx.x == 0) {
-            const int md = C->mode;
-            const double nrm = sqrt(sh[0]);
-            const double nin = (md == SA_START_RANDOM) ? 0.0 : ((md == SA_START_SECANT || md == SA_START_TANGENT) ? 2.0 : 1.0);
-            C->bytes += (double)n * sizeof(T) * (2.0 + nin) + (md == SA_START_DIAGONAL ? 8.0 * n : 0.0);
-            C->action = ACT_NEXT;
-            if (md == SA_START_DIAGONAL && nrm < kTinyNorm) {
-              C->mode = SA_START_RANDOM;           // utils/predictors.py:22-25
-              C->action = ACT_P0_AGAIN;
-            } else if (md == SA_START_SECANT &&
-                       (!A.has_prev || sqrt(sh[1]) < kTinyNorm || nrm < kTinyNorm)) {
-              C->mode = SA_START_PREV;             // utils/predictors.py:44-55
-              C->action = ACT_P0_AGAIN;
-            } else if (md == SA_START_TANGENT && (!A.has_last || !(nrm >= kTinyNorm) || !isfinite(nrm))) {
-              C->mode = SA_START_PREV;             // as the secant fallback
-              C->action = ACT_P0_AGAIN;
-            } else if (!(nrm > 0.0) || !isfinite(nrm)) {
-              C->status = SA_ERR_NONFINITE;
-              C->action = ACT_ERROR;
-            } else {
-              C->inv_b = 1.0 / nrm;
-              C->j = 0;
-              C->pass2 = 0;
-            }
-          }
-        })) return;
+    sums.block_put(v);
+    if (!sums.all_sum(3)) return;
+    if (threadIdx.x == 0) {
+      const int md = C->mode;
+      const double nrm = sqrt(tot[0]);
+      const double nin = (md == SA_START_RANDOM) ? 0.0 : ((md == SA_START_SECANT || md == SA_START_TANGENT) ? 2.0 : 1.0);
+      C->bytes += (double)n * sizeof(T) * (2.0 + nin) + (md == SA_START_DIAGONAL ? 8.0 * n : 0.0);
+      C->action = ACT_NEXT;
+      if (md == SA_START_DIAGONAL && nrm < kTinyNorm) {
+        C->mode = SA_START_RANDOM;           // utils/predictors.py:22-25
+        C->action = ACT_P0_AGAIN;
+      } else if (md == SA_START_SECANT &&
+                 (!A.has_prev || sqrt(tot[1]) < kTinyNorm || nrm < kTinyNorm)) {
+        C->mode = SA_START_PREV;             // utils/predictors.py:44-55
+        C->action = ACT_P0_AGAIN;
+      } else if (md == SA_START_TANGENT && (!A.has_last || !(nrm >= kTinyNorm) || !isfinite(nrm))) {
+        C->mode = SA_START_PREV;             // as the secant fallback
+        C->action = ACT_P0_AGAIN;
+      } else if (!(nrm > 0.0) || !isfinite(nrm)) {
+        C->status = SA_ERR_NONFINITE;
+        C->action = ACT_ERROR;
+      } else {
+        C->inv_b = 1.0 / nrm;
+        C->j = 0;
+        C->pass2 = 0;
+      }
+      C->ritz_ok = 0;
+    }
     mark(0);
-    const int act = vload(&C->action);
+    __syncthreads();
+    const int act = C->action;
     if (act == ACT_P0_AGAIN) continue;
-    if (act == ACT_ERROR) return;
+    if (act == ACT_ERROR) {
+      publish();
+      return;
+    }
 
     // ---------------- Lanczos steps ----------------------------------------------------------
     bool restart_p0 = false;
-    if (pol.block() == 0 && threadIdx.x == 0) C->ritz_ok = 0;
     while (true) {
-      const int j = vload(&C->j);
-      const int pass2 = vload(&C->pass2);
-      if (!pass2) {
-        // P1: V[j] = w * inv_b; w <- S V[j]; partial sums of a_j = V[j] . w
-        const T inv_b = (T)vload(&C->inv_b);
-        T* Vj = A.V + (long long)j * A.ldv;
-        const T trho = (T)rho;
-        double pa[1] = {0.0};
-        if (!apply([&](long long r, T acc) {
-              const T wr = __ldcg(A.w + r);
-              const T vr = wr * inv_b;
-              const T wn = (trho * wr - __ldcg(A.sigma + r) * acc) * inv_b;
-              Vj[r] = vr;
-              A.w[r] = wn;
-              pa[0] += (double)vr * (double)wn;
-            })) return;
-        block_store_partials<1>(pa, A.part, A.pw, 0, sm, pol.block());
-        if (!pol.sync(&C->gs, [&] {
-              reduce_partials(A.part, A.pw, pol.nblocks(), 1, sm);
-              if (threadIdx.x == 0) {
-                C->a[j] = sm[0];
-                C->bytes += A.spmv_bytes + (double)n * sizeof(T);
-                C->spmvs += 1;
-              }
-            })) return;
+      const int j = C->j;
+      const int pass2 = C->pass2;
+      const bool last = C->action == ACT_DONE;   // the final pass: the true residual of y (F2)
+      if (!pass2 && (!last || P.residual_check)) {
+        // P1: V[j] = w * inv_b; w <- S V[j]; partial sums of a_j = V[j] . w. (The final pass shares the
+        // operator's code: F2 |S y - theta y|^2.)
+        RowStep<T> f{last ? A.yout : A.w, A.sigma, A.V + (long long)j * A.ldv, A.w, (T)rho, (T)C->inv_b, C->theta, last, 0.0};
+        if (!apply(f)) return;
+        const double pa[1] = {f.acc};
+        sums.block_put(pa);
+        if (last) break;
+        if (!sums.all_sum(1)) return;
+        if (threadIdx.x == 0) {
+          C->a[j] = tot[0];
+          C->bytes += A.spmv_bytes + (double)n * sizeof(T);
+          C->spmvs += 1;
+        }
         mark(1);
-      }
-      // P2: three-term step w -= a_j V[j] + b_{j-1} V[j-1] (first pass only), then the
-      // reorthogonalisation coefficients h_k = V_k . w (k <= j) and ww = w . w. Removing the
-      // dominant components explicitly first keeps the single Gram-Schmidt pass stable.
-      {
-        const double a3 = pass2 ? 0.0 : vload(&C->a[j]);
-        const double b3 = (pass2 || j == 0) ? 0.0 : vload(&C->b[j - 1]);
-        const T* Vj = A.V + (long long)j * A.ldv;
-        const T* Vm = A.V + (long long)(j > 0 ? j - 1 : 0) * A.ldv;
-        constexpr int VW = 16 / sizeof(T);
-        const long long nvec = n / VW;
-        for (int kb = 0; kb <= j; kb += kDotBatch) {
-          double acc[kDotBatch + 1];
-#pragma unroll
-          for (int q = 0; q <= kDotBatch; ++q) acc[q] = 0.0;
-          const int nk = (j + 1 - kb < kDotBatch) ? (j + 1 - kb) : kDotBatch;
-          for (long long iv = gtid; iv < nvec; iv += nthreads) {
-            const long long i0 = iv * VW;
-            T wv[VW];
-            ld16(A.w + i0, wv);
-            double wd[VW];
-            if (kb == 0 && !pass2) {
-              T vj[VW], vm[VW];
-              ld16(Vj + i0, vj);
-              ld16(Vm + i0, vm);
-#pragma unroll
-              for (int r = 0; r < VW; ++r) {
-                double x = (double)wv[r] - a3 * (double)vj[r];
-                if (j > 0) x -= b3 * (double)vm[r];
-                wv[r] = (T)x;
-              }
-              st16(A.w + i0, wv);
-            }
-#pragma unroll
-            for (int r = 0; r < VW; ++r) wd[r] = (double)wv[r];
-#pragma unroll
-            for (int q = 0; q < kDotBatch; ++q) {
-              if (q < nk) {
-                T vk[VW];
-                ld16(A.V + (long long)(kb + q) * A.ldv + i0, vk);
-#pragma unroll
-                for (int r = 0; r < VW; ++r) acc[q] += (double)vk[r] * wd[r];
-              }
-            }
-            if (kb == 0) {
-#pragma unroll
-              for (int r = 0; r < VW; ++r) acc[kDotBatch] += wd[r] * wd[r];
-            }
-          }
-          for (long long i = nvec * VW + gtid; i < n; i += nthreads) {
-            double wi = (double)__ldcg(A.w + i);
-            if (kb == 0 && !pass2) {
-              wi -= a3 * (double)__ldcg(Vj + i);
-              if (j > 0) wi -= b3 * (double)__ldcg(Vm + i);
-              const T wt = (T)wi;
-              A.w[i] = wt;
-              wi = (double)wt;
-            }
-#pragma unroll
-            for (int q = 0; q < kDotBatch; ++q)
-              if (q < nk) acc[q] += (double)__ldcg(A.V + (long long)(kb + q) * A.ldv + i) * wi;
-            if (kb == 0) acc[kDotBatch] += wi * wi;
-          }
-          block_store_partials<kDotBatch + 1>(acc, A.part, A.pw, kb * 2, sm, pol.block());
-        }
-        if (!pol.sync(&C->gs, [&] {
-              // batch kb stored its 8 dots at cols [2kb, 2kb + 8) and ww (kb = 0) at col 8
-              const int nb = (j + kDotBatch) / kDotBatch;
-              reduce_partials(A.part, A.pw, pol.nblocks(), 2 * kDotBatch * (nb - 1) + kDotBatch + 1, sm);
-              if (threadIdx.x <= j) {
-                const int kb = (threadIdx.x / kDotBatch) * kDotBatch;
-                C->h[threadIdx.x] = sm[2 * kb + (threadIdx.x - kb)];
-              }
-              if (threadIdx.x == 0) {
-                C->ww = sm[kDotBatch];
-                C->a[j] += sm[2 * ((j / kDotBatch) * kDotBatch) + (j % kDotBatch)];
-                C->bytes += (double)n * sizeof(T) * (double)(j + 2 + (C->pass2 ? 0 : 3));
-              }
-            })) return;
-        mark(2);
-      }
-      // P3: w -= sum_k h_k V_k ; u = sigma w ; ww2
-      {
-        if (threadIdx.x <= j) sh[threadIdx.x] = vload(&C->h[threadIdx.x]);
         __syncthreads();
-        double v[1] = {0.0};
-        constexpr int VW = 16 / sizeof(T);
-        const long long nvec = n / VW;
-        // U positions per thread and iteration (iv, iv + nthreads), whose loads are in flight
-        // together, and KB3 basis vectors per batch (the same registers as one position and
-        // kDotBatch vectors); the batch kernel keeps one position within its register budget
-        constexpr int U = kLayouts ? 2 : 1;
-        constexpr int KB3 = kDotBatch / U;
-        for (long long iv = gtid; iv < nvec; iv += U * nthreads) {
-          const bool two = U == 2 && iv + nthreads < nvec;
-          const long long i0[2] = {iv * VW, (two ? iv + nthreads : iv) * VW};
-          // w and sigma are put in flight first; the basis is read kDotBatch vectors at a time
-          T wv[2][VW], sg[2][VW];
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            ld16(A.w + i0[u], wv[u]);
-            ld16(A.sigma + i0[u], sg[u]);
-          }
-          double corr[2][VW];
-#pragma unroll
-          for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int r = 0; r < VW; ++r) corr[u][r] = 0.0;
-          for (int kb = 0; kb <= j; kb += KB3) {
-            T vk[KB3][2][VW];
-#pragma unroll
-            for (int q = 0; q < KB3; ++q) {
-              if (kb + q <= j) {
-#pragma unroll
-                for (int u = 0; u < U; ++u) ld16(A.V + (long long)(kb + q) * A.ldv + i0[u], vk[q][u]);
-              }
-            }
-#pragma unroll
-            for (int q = 0; q < KB3; ++q) {
-              if (kb + q <= j) {
-#pragma unroll
-                for (int u = 0; u < U; ++u)
-#pragma unroll
-                  for (int r = 0; r < VW; ++r) corr[u][r] += sh[kb + q] * (double)vk[q][u][r];
-              }
-            }
-          }
-#pragma unroll
-          for (int u = 0; u < U; ++u) {
-            T uv[VW];
-#pragma unroll
-            for (int r = 0; r < VW; ++r) {
-              wv[u][r] = (T)((double)wv[u][r] - corr[u][r]);
-              uv[r] = sg[u][r] * wv[u][r];
-              if (u == 0 || two) v[0] += (double)wv[u][r] * (double)wv[u][r];
-            }
-            if (u == 0 || two) {
-              st16(A.w + i0[u], wv[u]);
-              st16(A.u + i0[u], uv);
-            }
-          }
-        }
-        for (long long i = nvec * VW + gtid; i < n; i += nthreads) {
-          const double corr = basis_combine(A.V, A.ldv, i, j, sh);
-          const T wi = (T)((double)__ldcg(A.w + i) - corr);
-          A.w[i] = wi;
-          A.u[i] = A.sigma[i] * wi;
-          v[0] += (double)wi * (double)wi;
-        }
-        block_store_partials<1>(v, A.part, A.pw, 0, sm, pol.block());
       }
-      if (!pol.sync(&C->gs, [&] {
-            reduce_partials(A.part, A.pw, pol.nblocks(), 1, sm);
-            const double ww2 = sm[0];
-            const double bj = sqrt(ww2);
-            const double aj = C->a[j];
-            if (threadIdx.x == 0) {
-              C->action = ACT_NEXT;
-              C->bytes += (double)n * sizeof(T) * (double)(j + 5);
-              if (!C->pass2) C->iters += 1;
-              if (!isfinite(aj) || !isfinite(bj) || fabs(aj) > bound || bj > bound) {
-                C->status = SA_ERR_BREAKDOWN;   // models/spectral_annealing.py:85-120
-                C->action = ACT_ERROR;
-              } else if (C->test_pred && j == 0) {
-                C->test_pred = 0;
-                C->pred_residual = bj;
-                C->pred_accepted = (bj > P.pred_tol) ? 0 : 1;
-                if (bj > P.pred_tol) {           // models/spectral_annealing.py:610-612
-                  C->mode = SA_START_PREV;
-                  C->iters = 0;
-                  C->action = ACT_REJECT;
-                }
-              }
-              if (C->action == ACT_NEXT && !C->pass2 && ww2 < 1e-4 * C->ww && bj > 1e-14 * bound) {
-                C->pass2 = 1;                    // second Gram-Schmidt pass
-                C->action = ACT_REPASS;
-              }
-              C->pass2 = (C->action == ACT_REPASS) ? 1 : 0;
-            }
-            __syncthreads();
-            const int act0 = C->action;
-            if (act0 == ACT_NEXT) {
-              const int m = j + 1;
-              double s2;
-              // previous step's Ritz value and residual estimate as the bracket to try first
-              double hlo = 0.0, hhi = -1.0;
-              if (m >= 2 && C->ritz_ok) {
-                const double th0 = C->theta, r0 = C->res_est;
-                const double pad = 1e-12 * fmax(1.0, fabs(th0));
-                hlo = th0 - 2.0 * r0 - pad;
-                hhi = th0 + pad;
-              }
-              const double th = smallest_eig_block(C->a, C->b, m, &s2, sq, hlo, hhi);
-              if (threadIdx.x == 0) {
-                s_theta = th;
-                s_s2 = s2;
-              }
-              __syncthreads();
-              if (threadIdx.x == 0) {
-                const double res = bj * sqrt(s_s2);
-                const bool invariant = bj <= 1e-14 * bound;
-                C->theta = s_theta;
-                C->res_est = invariant ? 0.0 : res;
-                C->ritz_ok = 1;
-                const bool conv = invariant || res <= P.tol;
-                if (conv || C->iters >= P.maxiter) {
-                  tridiag_eigvec(C->a, C->b, m, s_theta, C->s);
-                  C->status = conv ? SA_OK : SA_ERR_NOT_CONVERGED;
-                  C->b[j] = bj;
-                  C->action = ACT_DONE;
-                } else if (m >= ncv) {
-                  C->restarts += 1;
-                  C->action = ACT_RESTART;
-                } else {
-                  C->b[j] = bj;
-                  C->inv_b = 1.0 / bj;
-                  C->j = j + 1;
-                }
-              }
-              __syncthreads();
-              if (C->action == ACT_RESTART) {
-                const int keep = P.restart_keep > 0 ? P.restart_keep : kRestartDefault;
-                const int kk = max(1, min(min(keep, kRestartMax), ncv / 2));
-                implicit_restart(C, A.dense + kNcvMax * kNcvMax, m, kk, sq);
-              }
-            }
-          })) return;
+      if (last) break;
+      // P2: three-term step and reorthogonalisation coefficients
+      {
+        const double a3 = pass2 ? 0.0 : C->a[j], b3 = (pass2 || j == 0) ? 0.0 : C->b[j - 1];
+        if constexpr (kMode != ALPHA_SMALL) {
+          extern __shared__ __align__(128) char stream_smem[];
+          VecStream<T> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
+          if (!stream_dots<T>(S, A.V, A.ldv, A.w, A.u, j, pass2, a3, b3, work.dots)) return;
+        } else {
+          lanczos_dots<T>(A.V, A.ldv, A.w, A.u, nvt, j, pass2, a3, b3, work.dots, (int)pol.tid(), (int)nthreads);
+        }
+        __syncthreads();
+        if (threadIdx.x <= j + 1) {
+          double acc = 0.0;
+#pragma unroll 4
+          for (int w = 0; w < (int)(blockDim.x >> 5); ++w) acc += work.dots[w * kPartCols + threadIdx.x];
+          sums.put(threadIdx.x, acc);
+        }
+        if (!sums.all_sum(j + 2)) return;
+        if (threadIdx.x <= j) C->h[threadIdx.x] = tot[threadIdx.x];
+        if (threadIdx.x == 0) {
+          C->ww = tot[j + 1];
+          C->a[j] += tot[j];
+          C->bytes += (double)n * sizeof(T) * (double)(j + 2 + (pass2 ? 0 : 3));
+        }
+        mark(2);
+        __syncthreads();
+      }
+      // P3: w = w' - sum_k h_k V_k ; u = sigma w ; ww2
+      {
+        const T* src = pass2 ? A.w : A.u;
+        double v[1] = {0.0};
+        if constexpr (kMode != ALPHA_SMALL) {
+          extern __shared__ __align__(128) char stream_smem[];
+          VecStream<T> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
+          if (!stream_update<T>(S, A.V, A.ldv, src, A.sigma, A.w, A.u, j, C->h, v[0])) return;
+        } else {
+          v[0] = lanczos_update<T>(A.V, A.ldv, src, A.sigma, A.w, A.u, nvt, j, C->h, (int)pol.tid(), (int)nthreads);
+        }
+        sums.block_put(v);
+      }
+      if (!sums.all_sum(1)) return;
+      const double ww2 = tot[0];
+      const double bj = sqrt(ww2);
+      if (threadIdx.x == 0) {
+        const double aj = C->a[j];
+        C->action = ACT_NEXT;
+        C->bytes += (double)n * sizeof(T) * (double)(j + 5);
+        if (!C->pass2) C->iters += 1;
+        if (!isfinite(aj) || !isfinite(bj) || fabs(aj) > bound || bj > bound) {
+          C->status = SA_ERR_BREAKDOWN;   // models/spectral_annealing.py:85-120
+          C->action = ACT_ERROR;
+        } else if (C->test_pred && j == 0) {
+          C->test_pred = 0;
+          C->pred_residual = bj;
+          C->pred_accepted = (bj > P.pred_tol) ? 0 : 1;
+          if (bj > P.pred_tol) {           // models/spectral_annealing.py:610-612
+            C->mode = SA_START_PREV;
+            C->iters = 0;
+            C->action = ACT_REJECT;
+          }
+        }
+        if (C->action == ACT_NEXT && !C->pass2 && ww2 < 1e-4 * C->ww && bj > 1e-14 * bound) {
+          C->pass2 = 1;                    // second Gram-Schmidt pass
+          C->action = ACT_REPASS;
+        }
+        C->pass2 = (C->action == ACT_REPASS) ? 1 : 0;
+      }
+      __syncthreads();
+      if (C->action == ACT_NEXT) {
+        const int m = j + 1;
+        double s2;
+        // previous step's Ritz value and residual estimate as the bracket to try first
+        double hlo = 0.0, hhi = -1.0;
+        if (m >= 2 && C->ritz_ok) {
+          const double th0 = C->theta, r0 = C->res_est;
+          const double pad = 1e-12 * fmax(1.0, fabs(th0));
+          hlo = th0 - 2.0 * r0 - pad;
+          hhi = th0 + pad;
+        }
+        const double th = smallest_eig_block(C->a, C->b, m, &s2, hlo, hhi);
+        if (threadIdx.x == 0) {
+          const double res = bj * sqrt(s2);
+          const bool invariant = bj <= 1e-14 * bound;
+          C->theta = th;
+          C->res_est = invariant ? 0.0 : res;
+          C->ritz_ok = 1;
+          const bool conv = invariant || res <= P.tol;
+          if (conv || C->iters >= P.maxiter) {
+            C->status = conv ? SA_OK : SA_ERR_NOT_CONVERGED;
+            C->b[j] = bj;
+            C->action = ACT_DONE;
+          } else if (m >= ncv) {
+            C->restarts += 1;
+            C->action = ACT_RESTART;
+          } else {
+            C->b[j] = bj;
+            C->inv_b = 1.0 / bj;
+            C->j = j + 1;
+          }
+        }
+        __syncthreads();
+        if (C->action == ACT_DONE) {
+          tridiag_eigvec(C->a, C->b, m, th, C->s, sq);
+          __syncthreads();
+        }
+      }
+      const int act = C->action;
+      if (act == ACT_RESTART) {
+        // the first CTA runs the implicit restart; Q and the new tridiagonal reach the others in
+        // global memory
+        if (blk == 0) {
+          const int keep = P.restart_keep > 0 ? P.restart_keep : kRestartDefault;
+          const int kk = max(1, min(min(keep, kRestartMax), ncv / 2));
+          implicit_restart(C, A.dense + kNcvMax * kNcvMax, j + 1, kk, sq, (int)(sizeof(work) / sizeof(double)));
+          if (threadIdx.x < kk) {
+            G->a[threadIdx.x] = C->a[threadIdx.x];
+            G->b[threadIdx.x] = C->b[threadIdx.x];
+          }
+          if (threadIdx.x == 0) {
+            G->irl_beta = C->irl_beta;
+            G->irl_sigma = C->irl_sigma;
+            G->irl_k = C->irl_k;
+          }
+        }
+        if (!sums.meet()) return;
+        if (blk != 0) {
+          const int kk = vload(&G->irl_k);
+          if (threadIdx.x < kk) {
+            C->a[threadIdx.x] = vload(&G->a[threadIdx.x]);
+            C->b[threadIdx.x] = vload(&G->b[threadIdx.x]);
+          }
+          if (threadIdx.x == 0) {
+            C->irl_beta = vload(&G->irl_beta);
+            C->irl_sigma = vload(&G->irl_sigma);
+            C->irl_k = kk;
+          }
+          __syncthreads();
+        }
+      }
       mark(3);
-      const int act = vload(&C->action);
       if (act == ACT_NEXT) continue;
       if (act == ACT_REPASS) continue;
-      if (act == ACT_ERROR) return;
+      if (act == ACT_ERROR) {
+        publish();
+        return;
+      }
       if (act == ACT_REJECT) { restart_p0 = true; break; }
       if (act == ACT_RESTART) {
         // kept basis V[0..kk) <- V Q[:, 0..kk) and the new residual
         // f = V Q[:, kk] T+[kk][kk-1] + w Q[m-1][kk-1], row by row in place (all m inputs of a row
         // are read before its kk outputs are written)
         const int m = j + 1;
-        const int kk = vload(&C->irl_k);
-        const double beta_hat = vload(&C->irl_beta), sig_q = vload(&C->irl_sigma);
+        const int kk = C->irl_k;
+        const double beta_hat = C->irl_beta, sig_q = C->irl_sigma;
         const double* Qd = A.dense + kNcvMax * kNcvMax;
+#pragma unroll 1
         for (int idx = threadIdx.x; idx < m * (kk + 1); idx += blockDim.x) {
           const int r = idx / (kk + 1), c = idx % (kk + 1);
           sq[idx] = vload(Qd + r * m + c);
         }
         __syncthreads();
-        double v[1] = {0.0};
-        for (long long i = gtid; i < n; i += nthreads) {
-          double y[kRestartMax + 1];
-#pragma unroll
-          for (int c = 0; c <= kRestartMax; ++c) y[c] = 0.0;
-#pragma unroll 2
-          for (int r = 0; r < m; ++r) {
-            const double vr = (double)A.V[(long long)r * A.ldv + i];
-#pragma unroll
-            for (int c = 0; c <= kRestartMax; ++c)
-              if (c <= kk) y[c] += vr * sq[r * (kk + 1) + c];
+        const double v[1] = {kk == kRestartDefault
+                                 ? restart_basis<T, kRestartDefault>(A.V, A.ldv, A.w, A.u, A.sigma, n, m, kk, sq, beta_hat, sig_q, pol.tid(), nthreads)
+                                 : restart_basis<T, 0>(A.V, A.ldv, A.w, A.u, A.sigma, n, m, kk, sq, beta_hat, sig_q, pol.tid(), nthreads)};
+        sums.block_put(v);
+        if (!sums.all_sum(1)) return;
+        const double nf = sqrt(tot[0]);
+        const bool invariant = !(nf > 1e-14 * bound) || !isfinite(nf);
+        double th = 0.0;
+        if (invariant) th = smallest_eig_call(C->a, C->b, kk);
+        if (threadIdx.x == 0) {
+          C->pass2 = 0;
+          C->bytes += (double)n * sizeof(T) * (double)(m + kk + 3);
+          if (invariant) {
+            // the kept basis spans an invariant subspace: finish with its Ritz vector
+            C->theta = th;
+            C->j = kk - 1;
+            C->res_est = 0.0;
+            C->status = SA_OK;
+            C->action = ACT_DONE;
+          } else {
+            C->b[kk - 1] = nf;
+            C->inv_b = 1.0 / nf;
+            C->j = kk;
+            C->action = ACT_NEXT;
           }
-#pragma unroll
-          for (int c = 0; c < kRestartMax; ++c)
-            if (c < kk) A.V[(long long)c * A.ldv + i] = (T)y[c];
-          double yk = 0.0;
-#pragma unroll
-          for (int c = 0; c <= kRestartMax; ++c)
-            if (c == kk) yk = y[c];
-          const T f = (T)(yk * beta_hat + (double)A.w[i] * sig_q);
-          A.w[i] = f;
-          A.u[i] = A.sigma[i] * f;
-          v[0] += (double)f * (double)f;
         }
-        block_store_partials<1>(v, A.part, A.pw, 0, sm, pol.block());
-        if (!pol.sync(&C->gs, [&] {
-              reduce_partials(A.part, A.pw, pol.nblocks(), 1, sm);
-              const double nf = sqrt(sm[0]);
-              const bool invariant = !(nf > 1e-14 * bound) || !isfinite(nf);
-              double th = 0.0, s2 = 0.0;
-              if (invariant) th = smallest_eig_block(C->a, C->b, kk, &s2, sq);
-              if (threadIdx.x == 0) {
-                C->pass2 = 0;
-                C->bytes += (double)n * sizeof(T) * (double)(m + kk + 3);
-                if (invariant) {
-                  // the kept basis spans an invariant subspace: finish with its Ritz vector
-                  C->theta = th;
-                  tridiag_eigvec(C->a, C->b, kk, th, C->s);
-                  C->j = kk - 1;
-                  C->res_est = 0.0;
-                  C->status = SA_OK;
-                  C->action = ACT_DONE;
-                } else {
-                  C->b[kk - 1] = nf;
-                  C->inv_b = 1.0 / nf;
-                  C->j = kk;
-                  C->action = ACT_NEXT;
-                }
-              }
-            })) return;
         mark(4);
-        if (vload(&C->action) == ACT_DONE) break;
-        continue;
+        __syncthreads();
+        if (C->action == ACT_DONE) {
+          tridiag_eigvec(C->a, C->b, kk, th, C->s, sq);
+          __syncthreads();
+        } else {
+          continue;
+        }
       }
-      break;   // ACT_DONE
+      // ---------------- F1: Ritz vector y = V s, norm, alignment dot ------------------------------
+      const int jf = C->j;
+      const bool align = P.align && A.has_last;
+      {
+        double v[2] = {0.0, 0.0};
+        int bad = 0;
+#pragma unroll 1
+        for (long long i = pol.tid(); i < n; i += nthreads) {
+          const double y = basis_combine(A.V, A.ldv, i, jf, C->s);
+          const T yt = (T)y;
+          if (!isfinite((double)yt)) bad = 1;
+          A.yout[i] = yt;
+          A.u[i] = A.sigma[i] * yt;
+          v[0] += (double)yt * (double)yt;
+          if (align) v[1] += (double)yt * (double)A.ylast[i];
+        }
+        if (bad) atomicOr(&G->nonfinite, 1);
+        sums.block_put(v);
+      }
+      if (!sums.all_sum(2)) return;
+      if (threadIdx.x == 0) {
+        const double nrm = sqrt(tot[0]);
+        C->nrm_y = nrm;
+        C->align_dot = align ? tot[1] : 0.0;
+        C->bytes += (double)n * sizeof(T) * (double)(jf + 3 + (align ? 1 : 0));
+        const double sg = (align && tot[1] < 0.0) ? -1.0 : 1.0;
+        C->scale = (nrm > 0.0) ? sg / nrm : sg;
+      }
+      mark(5);
+      __syncthreads();
     }
     if (restart_p0) continue;
     break;
   }
 
-  // ---------------- F1: Ritz vector y = V s, norm, alignment dot ------------------------------
-  const int jf = vload(&C->j);
-  if (threadIdx.x <= jf) sh[threadIdx.x] = vload(&C->s[threadIdx.x]);
-  __syncthreads();
+  // ---------------- F2: rounding (the residual's sum was stored by the final operator pass) --------
+  const double scale = C->scale;
   {
-    double v[2] = {0.0, 0.0};
-    int bad = 0;
-    const bool align = P.align && A.has_last;
-    for (long long i = gtid; i < n; i += nthreads) {
-      const double y = basis_combine(A.V, A.ldv, i, jf, sh);
-      const T yt = (T)y;
-      if (!isfinite((double)yt)) bad = 1;
-      A.yout[i] = yt;
-      A.u[i] = A.sigma[i] * yt;
-      v[0] += (double)yt * (double)yt;
-      if (align) v[1] += (double)yt * (double)A.ylast[i];
-    }
-    if (bad) atomicOr(&C->nonfinite, 1);
-    block_store_partials<2>(v, A.part, A.pw, 0, sm, pol.block());
-  }
-  if (!pol.sync(&C->gs, [&] {
-        reduce_partials(A.part, A.pw, pol.nblocks(), 2, sh);
-        if (threadIdx.x == 0) {
-          const double nrm = sqrt(sh[0]);
-          const bool align = P.align && A.has_last;
-          C->nrm_y = nrm;
-          C->align_dot = align ? sh[1] : 0.0;
-          C->bytes += (double)n * sizeof(T) * (double)(jf + 3 + (align ? 1 : 0));
-          const double sg = (align && sh[1] < 0.0) ? -1.0 : 1.0;
-          C->scale = (nrm > 0.0) ? sg / nrm : sg;
-        }
-      })) return;
-  mark(5);
-
-  // ---------------- F2: true residual (one SpMV) and rounding -----------------------------------
-  const double theta = vload(&C->theta);
-  const double scale = vload(&C->scale);
-  {
-    double v[1] = {0.0};
-    if (P.residual_check) {
-      const T trho = (T)rho;
-      if (!apply([&](long long r, T acc) {
-            const T yt = __ldcg(A.yout + r);
-            const double yr = (double)yt;
-            const double sy = (double)(trho * yt - __ldcg(A.sigma + r) * acc);
-            const double rr = sy - theta * yr;
-            v[0] += rr * rr;
-          })) return;
-    }
     if (P.round) {
       const long long nr = (n + 31) & ~31ll;
       const T ts = (T)scale;
       unsigned long long hs = 0ull;
-      for (long long i = gtid; i < nr; i += nthreads) {
+#pragma unroll 1
+      for (long long i = pol.tid(); i < nr; i += nthreads) {
         bool bit = false;
         if (i < n) {
           const T x = (T)(A.yout[i] * ts) * (T)((double)A.sigma[i] * A.sqrt_c);
@@ -1094,26 +1639,25 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
           hs += word_mix(i >> 5, word);
         }
       }
-      if ((threadIdx.x & 31) == 0 && hs) atomicAdd(&C->sig, hs);
+      if ((threadIdx.x & 31) == 0 && hs) atomicAdd(&G->sig, hs);
     }
-    block_store_partials<1>(v, A.part, A.pw, 0, sm, pol.block());
   }
-  if (!pol.sync(&C->gs, [&] {
-        reduce_partials(A.part, A.pw, pol.nblocks(), 1, sh);
-        if (threadIdx.x == 0) {
-          C->rr = sh[0];
-          if (P.residual_check) { C->bytes += A.spmv_bytes; C->spmvs += 1; }
-          if (P.round) C->bytes += (double)n * sizeof(T) + (double)n / 8.0;
-          C->bytes += 2.0 * (double)n * sizeof(T);   // F3
-        }
-      })) return;
+  if (!sums.all_sum(P.residual_check ? 1 : 0)) return;
+  if (threadIdx.x == 0) {
+    C->rr = P.residual_check ? tot[0] : 0.0;
+    if (P.residual_check) { C->bytes += A.spmv_bytes; C->spmvs += 1; }
+    if (P.round) C->bytes += (double)n * sizeof(T) + (double)n / 8.0;
+    C->bytes += 2.0 * (double)n * sizeof(T);   // F3
+  }
   mark(5);
   // F3: y <- scale * y (aligned, unit norm)
   {
     const T ts = (T)scale;
-    for (long long i = gtid; i < n; i += nthreads) A.yout[i] = A.yout[i] * ts;
+#pragma unroll 1
+    for (long long i = pol.tid(); i < n; i += nthreads) A.yout[i] = A.yout[i] * ts;
   }
   mark(5);
+  publish();
 }
 
 }  // namespace sa

@@ -34,7 +34,7 @@ size_t ls_workspace_bytes(long long n, long long nnz, int k, int integer);
 
 constexpr int kBatchThreads = 128;
 constexpr int kBatchWarps = kBatchThreads / 32;
-constexpr int kBatchPartWidth = 2 * kNcvMax + kDotBatch + 8;
+constexpr int kBatchPartWidth = 2 * kPartCols;
 constexpr double kPlanStepFloor = 4.0e5;   // latency floor of a Lanczos step, in bytes-equivalent
 
 // One instance (matrix + prelude of its handle), shared by its seeds.
@@ -275,7 +275,6 @@ __device__ bool batch_problem(const BatchArgs& B, const BTeam& tm, int p, const 
         A.S.long_part = (T*)tm.long_part;
         A.S.scol = I.scol;
         A.S.wmag = (T)I.wmag;
-        A.use_panel = 0;
         A.n_splits = 0;
         A.n = n;
         A.ldv = I.ldv;
@@ -290,7 +289,6 @@ __device__ bool batch_problem(const BatchArgs& B, const BTeam& tm, int p, const 
         A.yout = (T*)tm.y[ld_volatile_i32(&S->iy_out)];
         A.v0 = nullptr;
         A.part = tm.part;
-        A.pw = kBatchPartWidth;
         A.ctrl = tm.actrl;
         A.bits = tm.bits;
         A.W = I.W;
@@ -322,7 +320,7 @@ __device__ bool batch_problem(const BatchArgs& B, const BTeam& tm, int p, const 
         A.dense = tm.dense;
       }
       __syncthreads();
-      alpha_body<T, RP, TeamPolicy, kBatchWarps, false>(A, pol);
+      alpha_body<T, RP, TeamPolicy, kBatchWarps, ALPHA_SMALL>(A, pol);
       if (ld_volatile_i32(&pol.gs->error)) return false;
       if (pol.block() == 0 && threadIdx.x == 0)
         for (int q = 0; q < 6; ++q) pr.sum->phase_ms[q] += (double)tm.actrl->tph[q] * 1e-6;

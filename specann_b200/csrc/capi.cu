@@ -45,7 +45,7 @@ struct Carve {
 };
 
 constexpr int kMaxBlocks = 1024;
-constexpr int kPartWidth = 2 * kNcvMax + kDotBatch + 8;
+constexpr int kPartWidth = 2 * (kNcvMax + 8);   // two buffers of partial sums (alpha_body.cuh: kPartCols)
 
 Carve carve(long long n, long long nnz, int prec, int ncv_max, int max_cand) {
   const size_t T = prec == 32 ? 4 : 8;
@@ -352,7 +352,6 @@ int sa_create(sa_handle** out, int64_t n, int64_t nnz, int32_t rowptr64, int32_t
   h->long_part = h->ws + c.long_part;
   h->cap_long_part = max_long_partials(nnz);
   h->blk_part = (double*)(h->ws + c.blk_part);
-  h->blk_part_width = kPartWidth;
   h->actrl = (AlphaCtrl*)(h->ws + c.actrl);
   h->red = (double*)(h->ws + c.red);
   h->cand = (uint32_t*)(h->ws + c.cand);

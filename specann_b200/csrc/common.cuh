@@ -38,7 +38,7 @@ struct GridSync {
   unsigned int count;
   unsigned int gen;
   int error;
-  int pad;
+  unsigned int arrivals;   // CTAs that have arrived at grid_arrive_wait since the block was zeroed
 };
 
 __device__ __forceinline__ unsigned int ld_volatile_u32(const unsigned int* p) {
@@ -103,6 +103,55 @@ __device__ __forceinline__ bool grid_barrier(GridSync* gs, Epilogue&& epi) {
 
 __device__ __forceinline__ bool grid_barrier(GridSync* gs) {
   return grid_barrier_n(gs, gridDim.x, [] {});
+}
+
+// Barrier of `expected` co-resident CTAs without an epilogue: every CTA adds one to a counter that is
+// never reset and waits until it reaches epoch * expected (epoch: this CTA's number of barriers, the
+// same in every thread). A CTA leaves as soon as the last one has arrived, one L2 round trip earlier
+// than from grid_barrier_n, whose last CTA works alone first and then releases the others. Waits are
+// bounded in the same way (after spin_limit polls the barrier records SA_ERR_BARRIER_TIMEOUT and
+// returns false, as it does when another CTA has recorded an error).
+__device__ __forceinline__ bool grid_arrive_wait(GridSync* gs, unsigned int expected, unsigned int& epoch,
+                                                 unsigned long long spin_limit = kSpinLimit) {
+  __shared__ int s_fail;
+  __syncthreads();
+  ++epoch;
+  if (threadIdx.x == 0) {
+    int fail = 0;
+    __threadfence();
+    atomicAdd(&gs->arrivals, 1u);
+    const unsigned int target = epoch * expected;
+    unsigned long long polls = 0;
+    while ((int)(ld_volatile_u32(&gs->arrivals) - target) < 0) {
+      if ((++polls & 63) != 0) continue;
+      if (ld_volatile_i32(&gs->error)) { fail = 1; break; }
+      if (polls > 4096) __nanosleep(64);
+      if (polls > spin_limit) {
+        atomicExch(&gs->error, SA_ERR_BARRIER_TIMEOUT);
+        fail = 1;
+        break;
+      }
+    }
+    __threadfence();
+    s_fail = fail;
+  }
+  __syncthreads();
+  return s_fail == 0;
+}
+
+// Barrier of all CTAs of this CTA's cluster (hardware; about 0.25 us), with the ordering of global
+// memory among them that a grid barrier gives.
+__device__ __forceinline__ void cluster_arrive_wait() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// threadIdx.x, read again where it is called: what a phase of a persistent kernel derives from it is
+// computed in the phase, instead of being hoisted out of the kernel's loop and held in registers (or
+// spilled) across all the other phases.
+__device__ __forceinline__ int tid_here() {
+  int t;
+  asm volatile("mov.u32 %0, %%tid.x;" : "=r"(t));
+  return t;
 }
 
 // Device clock in ns (phase timers of the persistent kernels).

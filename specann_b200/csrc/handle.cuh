@@ -153,7 +153,6 @@ struct sa_handle {
   long long cap_long_part = 0;
   long long n_long_part = 0;    // partial sums the bound matrix's multi-chunk rows use
   double* blk_part = nullptr;
-  int blk_part_width = 0;
   sa::AlphaCtrl* actrl = nullptr;
   double* dense = nullptr;      // implicit-restart scratch: dense T and Q (2 x kNcvMax^2 doubles)
   double* red = nullptr;        // small reduction scratch (set-up kernels)

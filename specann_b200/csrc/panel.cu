@@ -344,7 +344,8 @@ __global__ void __launch_bounds__(kThreads, 1) panel_spmv_kernel(PanelArgs P, co
   panel_init(bars);
   unsigned par = 0;
   panel_spmv<T>(P, u, blockIdx.x, gridDim.x, psm, bars, par, err,
-                [&](long long r, T acc) { y[r] = rho * x[r] - sigma[r] * acc; });
+                [&](long long r) { return RowInputs<T>{x[r], sigma[r]}; },
+                [&](long long r, T acc, const RowInputs<T>& in) { y[r] = rho * in.x - in.s * acc; });
 }
 
 }  // namespace

@@ -33,6 +33,7 @@ constexpr int kPanelRowBytes = 64 * 1024;   // row sums of one block
 // static shared memory); the dynamic shared memory of a panel kernel is the buffers + the row sums.
 __host__ __device__ constexpr int panel_buf_bytes(int elem) { return elem == 4 ? 64 * 1024 : 48 * 1024; }
 __host__ __device__ constexpr int panel_smem_bytes(int elem) { return kPanelBufs * panel_buf_bytes(elem) + kPanelRowBytes; }
+constexpr int kRowBatch = 4;                // rows per thread whose inputs are loaded together at the end
 constexpr unsigned long long kPanelSpinLimit = 1ull << 22;   // bounded wait for a panel copy
 
 struct PanelArgs {
@@ -65,13 +66,17 @@ __device__ __forceinline__ bool mbar_try_wait(unsigned long long* bar, unsigned 
 }
 
 // Stage `bytes` (a multiple of 16, both addresses 16-byte aligned) from global memory into shared
-// memory with completion on `bar` (one arrival carrying the byte count). One thread.
-__device__ __forceinline__ void panel_fill(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+// memory with completion on `bar` (panel_fill: with the one arrival carrying the byte count). One thread.
+__device__ __forceinline__ void bulk_load(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                    smem_u32(dst)),
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
+}
+
+__device__ __forceinline__ void panel_fill(void* dst, const void* src, unsigned bytes, unsigned long long* bar) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+  bulk_load(dst, src, bytes, bar);
 }
 
 // Orders this thread's earlier generic-proxy accesses (the reads of a panel buffer that is about to
@@ -80,9 +85,9 @@ __device__ __forceinline__ void panel_fill(void* dst, const void* src, unsigned 
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
 // Barrier set-up of a kernel that runs panel SpMVs (thread 0, then a CTA barrier).
-__device__ __forceinline__ void panel_init(unsigned long long* bars) {
+__device__ __forceinline__ void panel_init(unsigned long long* bars, int count = kPanelBufs) {
   if (threadIdx.x == 0) {
-    for (int q = 0; q < kPanelBufs; ++q) mbar_init(&bars[q], 1);
+    for (int q = 0; q < count; ++q) mbar_init(&bars[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -190,15 +195,24 @@ __device__ __forceinline__ void panel_batch(const unsigned (&r)[kPanelLane], con
   __syncwarp();
 }
 
-// One SpMV over the blocks of this CTA (b = blk, blk + nblk, ...): fin(row, sum) once per row with
-// sum = sum_j val_ij u_j. smem: panel_smem_bytes(sizeof(T)) dynamic bytes (panel buffers, then the row sums); bars:
+// A row's entries of the input vector and of the scaling.
+template <typename T>
+struct RowInputs {
+  T x, s;
+};
+
+// One SpMV over the blocks of this CTA (b = blk, blk + nblk, ...): fin(row, sum, pre(row)) once per row
+// with sum = sum_j val_ij u_j. pre(row) only loads: kRowBatch rows of it are in flight before their fin
+// stores anything (one after the other, the 14 to 28 rows of a thread at n = 2^20 would wait for L2 in
+// turn). smem: panel_smem_bytes(sizeof(T)) dynamic bytes (panel buffers, then the row sums); bars:
 // kPanelBufs mbarriers set up by panel_init; par: the barriers' phase bits (one bit per buffer,
 // kept by the caller across calls; every thread holds the same value). Returns false, with
 // SA_ERR_BARRIER_TIMEOUT in *err, if a panel copy does not complete in time.
-template <typename T, class Fin>
+template <typename T, class Pre, class Fin>
 __device__ __forceinline__ bool panel_spmv(const PanelArgs& P, const T* u, int blk, int nblk, char* smem,
-                                           unsigned long long* bars, unsigned& par, int* err, Fin&& fin) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+                                           unsigned long long* bars, unsigned& par, int* err, Pre&& pre, Fin&& fin) {
+  const int tid = tid_here();
+  const int lane = tid & 31, wid = tid >> 5;
   const unsigned long long pol = l2_policy_evict_first();
   T* ys = (T*)(smem + (size_t)kPanelBufs * panel_buf_bytes(sizeof(T)));
   const bool uniform = P.val == nullptr;
@@ -207,8 +221,8 @@ __device__ __forceinline__ bool panel_spmv(const PanelArgs& P, const T* u, int b
   const int np = P.n_panels;
   for (int b = blk; b < P.n_blocks; b += nblk) {
     const int r0 = __ldg(P.row0 + b), nr = __ldg(P.row0 + b + 1) - r0;
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) ys[i] = T(0);
-    if (threadIdx.x == 0) {
+    for (int i = tid; i < nr; i += blockDim.x) ys[i] = T(0);
+    if (tid == 0) {
       fence_proxy_async();
       for (int q = 0; q < kPanelBufs && q < np; ++q) panel_issue<T>(P, u, q, smem, bars);
     }
@@ -263,7 +277,7 @@ __device__ __forceinline__ bool panel_spmv(const PanelArgs& P, const T* u, int b
       if (__syncthreads_or(late)) {
         // Give up: record the timeout, then wait (bounded again) for the copies this CTA still has
         // in flight into its shared memory (panels p .. p + kPanelBufs - 1) before returning.
-        if (threadIdx.x == 0) {
+        if (tid == 0) {
           atomicExch(err, SA_ERR_BARRIER_TIMEOUT);
           for (int q = p; q < p + kPanelBufs && q < np; ++q) {
             const int qb = q % kPanelBufs;
@@ -274,12 +288,21 @@ __device__ __forceinline__ bool panel_spmv(const PanelArgs& P, const T* u, int b
         __syncthreads();
         return false;
       }
-      if (threadIdx.x == 0 && p + kPanelBufs < np) {
+      if (tid == 0 && p + kPanelBufs < np) {
         fence_proxy_async();
         panel_issue<T>(P, u, p + kPanelBufs, smem, bars);
       }
     }
-    for (int i = threadIdx.x; i < nr; i += blockDim.x) fin((long long)r0 + i, ys[i]);
+#pragma unroll 1
+    for (int i = tid; i < nr; i += kRowBatch * kThreads) {
+      decltype(pre(0ll)) x[kRowBatch];
+#pragma unroll
+      for (int q = 0; q < kRowBatch; ++q)
+        if (i + q * kThreads < nr) x[q] = pre((long long)r0 + i + q * kThreads);
+#pragma unroll
+      for (int q = 0; q < kRowBatch; ++q)
+        if (i + q * kThreads < nr) fin((long long)r0 + i + q * kThreads, ys[i + q * kThreads], x[q]);
+    }
     __syncthreads();
   }
   return true;

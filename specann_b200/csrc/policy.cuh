@@ -5,16 +5,28 @@
 
 namespace sa {
 
-// GridPolicy: one problem on the whole cooperative grid; phases are separated by grid_barrier on
-// the control block's GridSync (epilogue by the last CTA to arrive).
+// sync runs an epilogue on the last CTA to arrive before the others leave; meet only waits for all of
+// them (epoch: the caller's count of them, from first_epoch).
+//
+// GridPolicy: one problem on the whole grid. A cooperative grid separates phases on the control block's
+// GridSync; a grid that is one cluster (cluster = 1, only meet is used) by the cluster's barrier.
 struct GridPolicy {
-  __device__ __forceinline__ long long tid() const { return (long long)blockIdx.x * blockDim.x + threadIdx.x; }
+  int cluster = 0;
+  __device__ __forceinline__ long long tid() const { return (long long)blockIdx.x * blockDim.x + tid_here(); }
   __device__ __forceinline__ long long nthr() const { return (long long)gridDim.x * blockDim.x; }
   __device__ __forceinline__ int block() const { return blockIdx.x; }
   __device__ __forceinline__ int nblocks() const { return gridDim.x; }
   template <class E>
   __device__ __forceinline__ bool sync(GridSync* gs, E&& e) const { return grid_barrier(gs, e); }
   __device__ __forceinline__ bool sync(GridSync* gs) const { return grid_barrier(gs); }
+  __device__ __forceinline__ unsigned int first_epoch(GridSync*) const { return 0; }   // zeroed before the launch
+  __device__ __forceinline__ bool meet(GridSync* gs, unsigned int& epoch) const {
+    if (cluster) {
+      cluster_arrive_wait();
+      return true;
+    }
+    return grid_arrive_wait(gs, gridDim.x, epoch);
+  }
 };
 
 // TeamPolicy: one problem on the CTAs [b0, b0 + nb) of a cooperative grid (batched solves: every
@@ -24,7 +36,7 @@ struct GridPolicy {
 struct TeamPolicy {
   int b0, nb;
   GridSync* gs;
-  __device__ __forceinline__ long long tid() const { return (long long)(blockIdx.x - b0) * blockDim.x + threadIdx.x; }
+  __device__ __forceinline__ long long tid() const { return (long long)(blockIdx.x - b0) * blockDim.x + tid_here(); }
   __device__ __forceinline__ long long nthr() const { return (long long)nb * blockDim.x; }
   __device__ __forceinline__ int block() const { return (int)blockIdx.x - b0; }
   __device__ __forceinline__ int nblocks() const { return nb; }
@@ -39,6 +51,18 @@ struct TeamPolicy {
     return grid_barrier_n(gs, (unsigned int)nb, e);
   }
   __device__ __forceinline__ bool sync(GridSync* g) const { return sync(g, [] {}); }
+  // The counter runs on from solve to solve: between two barriers it stands in [E nb, (E + 1) nb) for
+  // every CTA that has left barrier E and not arrived at the next one.
+  __device__ __forceinline__ unsigned int first_epoch(GridSync*) const {
+    return nb == 1 ? 0u : ld_volatile_u32(&gs->arrivals) / (unsigned int)nb;
+  }
+  __device__ __forceinline__ bool meet(GridSync*, unsigned int& epoch) const {
+    if (nb == 1) {
+      __syncthreads();
+      return true;
+    }
+    return grid_arrive_wait(gs, (unsigned int)nb, epoch);
+  }
 };
 
 }  // namespace sa

@@ -162,8 +162,9 @@ __device__ __forceinline__ void load_tile(const SpmvArgs<T, RP>& S, const TileDe
 template <typename T, typename RP, bool kReadOnlyU = false, int NW = kWarps, class Fin>
 __device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u, long long gwarp,
                                            long long nwarps, SpmvSmem<T, NW>& sm, Fin&& fin) {
-  const int lane = threadIdx.x & 31;
-  const int wid = threadIdx.x >> 5;
+  const int tid = tid_here();
+  const int lane = tid & 31;
+  const int wid = tid >> 5;
   T* prod = sm.prod[wid];
   int* srp = sm.rp[wid];
   const unsigned long long pol_stream = l2_policy_evict_first();

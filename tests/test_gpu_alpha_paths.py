@@ -1,0 +1,67 @@
+"""The alpha solve at the edges of its paths: one cluster of 8 or 16 CTAs and the whole grid (by the
+tiles of the work list), vector phases in registers and streamed (by n), sizes that are no multiple of
+a 16-byte position, the column panels at small n, and basis and restart sizes other than the default.
+Each against SciPy's FP64 eigensolver on the exact operator, with a rounding that is bit-exact given
+the vector."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+import scipy.sparse.linalg as spla
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+from oracle import specann_oracle as O  # noqa: E402
+from specann_b200 import _lib, graphs  # noqa: E402
+from specann_b200.engine import Engine  # noqa: E402
+
+
+def check(J, precision, alpha, ncv=33, keep=0, layout="worklist", tol=1e-6):
+    J = sp.csr_matrix(J)
+    n = J.shape[0]
+    eng = Engine(n, J.nnz, precision=precision, ncv_max=ncv, max_candidates=2)
+    eng.upload_csr(J.indptr, J.indices, J.data.astype(np.float32 if precision == 32 else np.float64))
+    if layout == "panel":
+        eng.build_panels()
+    rec = eng.alpha_solve(alpha=alpha, alpha_prev=alpha, rho=1.001, gershgorin=1.0, tol=tol, pred_tol=1e-3,
+                          maxiter=4000, ncv=ncv, start_mode=_lib.SA_START_RANDOM, seed=7, stream_id=0, align=False,
+                          restart_keep=keep)
+    assert rec.status == _lib.SA_OK, rec.status
+    deg = np.asarray(abs(J).sum(axis=1)).ravel()
+    M, _ = O.scaled_operator_f64(J, deg, deg.max(), alpha)
+    y = eng.result_vector().double().cpu().numpy()
+    lam = 1.001 - rec.mu
+    # the solver stops at a residual estimate of tol; the FP32 operator adds its rounding
+    assert np.linalg.norm(M @ y - lam * y) <= (1e-5 if precision == 32 else 2 * tol)
+    ref = spla.eigsh(spla.aslinearoperator(M), k=1, which="LA", v0=y, tol=1e-10, return_eigenvectors=False)[0]
+    assert abs(lam - ref) <= (1e-6 if precision == 32 else 1e-8)
+    eng.keep_candidate(0)
+    assert np.array_equal(eng.candidate_spins(0).cpu().numpy(), np.where(y >= 0, 1, -1).astype(np.int8))
+    eng.close()
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+# 37: under a warp of positions; 1283 / 1290: about 128 tiles (8 or 16 CTAs); 2559 / 2566: about 256 (16 or the grid)
+@pytest.mark.parametrize("n", [37, 130, 1283, 1290, 2559, 2566])
+def test_cluster_and_grid_edges(n, precision):
+    check(graphs.barabasi_albert(n, 10, seed=n), precision, 0.5)
+
+
+@pytest.mark.parametrize("precision,n", [(32, 151549), (32, 151557), (64, 75775), (64, 75779)])
+def test_register_and_streamed_vector_phases(precision, n):
+    check(graphs.barabasi_albert(n, 4, seed=5), precision, 0.4)
+
+
+@pytest.mark.parametrize("precision", [32, 64])
+@pytest.mark.parametrize("n", [591, 4099])
+def test_streamed_phases_on_few_rows_per_cta(n, precision):
+    check(graphs.barabasi_albert(n, 20, seed=3), precision, 0.5, layout="panel")
+
+
+@pytest.mark.parametrize("ncv,keep", [(4, 0), (9, 3), (33, 16), (64, 8)])
+def test_basis_and_restart_sizes(ncv, keep):
+    # a leading gap small enough to restart several times
+    check(graphs.erdos_renyi(3000, 20 / 2999, seed=11), 64, 0.9, ncv=ncv, keep=keep, tol=1e-7)
