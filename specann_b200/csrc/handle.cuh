@@ -48,6 +48,15 @@ struct AlphaCtrl {
   int ritz_ok;              // theta / res_est hold the previous step's Ritz value and residual estimate
 };
 
+// Counters of one local-search pass (three sets in turn: a pass counts in one, the next pass's is already
+// zero, and the last pass's may still be read).
+struct LsPass {
+  unsigned int wq;          // wanting nodes of ordinary rows (from the front of the queue)
+  unsigned int lq;          // wanting nodes of long rows (from its back)
+  unsigned long long wl;    // work-list entries
+  int counts[128];          // flips per candidate
+};
+
 // Control block of the local-search kernel.
 struct LsCtrl {
   GridSync gs;
@@ -64,6 +73,7 @@ struct LsCtrl {
   unsigned int active[4];   // candidates that have not yet had a pass without a flip
   long long counts[128];    // flips per candidate in the current pass
   unsigned long long tph[4];  // ns by phase (set-up, decide, scatter, final)
+  LsPass pass[3];
 };
 
 struct Layout {

@@ -1,10 +1,14 @@
 // Host launch of the batched local search (cooperative grid; device code in ls_body.cuh).
+#include <algorithm>
+
 #include "ls_body.cuh"
 
 namespace sa {
 
+constexpr int kLsCtas = 2;   // CTAs per SM: the phases wait for memory, not for the SM
+
 template <typename VT, typename RP, typename GT>
-__global__ void __launch_bounds__(kThreads) ls_kernel(LsArgs<VT, RP, GT> A) {
+__global__ void __launch_bounds__(kThreads, kLsCtas) ls_kernel(LsArgs<VT, RP, GT> A) {
   ls_body<VT, RP, GT>(A, GridPolicy{});
 }
 
@@ -55,7 +59,11 @@ static int launch_ls(sa_handle* h, const sa_ls_params* p, char* ws, int kp, int 
   if (A.m_final < 1) A.m_final = 1;
   if (cudaMemsetAsync(A.ctrl, 0, sizeof(GridSync), h->stream) != cudaSuccess) return SA_ERR_CUDA;
   void* args[] = {&A};
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)ls_kernel<VT, RP, GT>, dim3(h->blocks),
+  int per_sm = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)ls_kernel<VT, RP, GT>, kThreads, 0) != cudaSuccess ||
+      per_sm < 1)
+    return SA_ERR_CUDA;
+  cudaError_t e = cudaLaunchCooperativeKernel((const void*)ls_kernel<VT, RP, GT>, dim3(h->sm_count * std::min(per_sm, kLsCtas)),
                                               dim3(kThreads), args, 0, h->stream);
   count_launches(1);
   return e == cudaSuccess ? SA_OK : SA_ERR_CUDA;

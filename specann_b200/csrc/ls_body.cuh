@@ -5,19 +5,25 @@
 //   priority (default): a wanting node flips unless a wanting neighbour has a lower rank in the
 //     pass's permutation, so the flips form an independent set and every flip lowers the energy
 //     by its gain (phases D1: wanting masks and ranks, D2: blocking check, U);
-//   snapshot: every wanting node flips (phases D, U).
+//   snapshot: every wanting node flips (phases D1, U).
 // Layout (node-major, so one read of a CSR row serves every candidate):
 //   sb[i * kw + t]     bit c of word t: spin of candidate 32 t + c at node i is +1
 //   h[i * kp + c]      local field of node i in candidate c (int32 for integer couplings, which
 //                      makes every gain and energy exact; double otherwise)
 //   flipm[i * kw + t]  candidates flipping at node i in the current pass
-// A pass: (D) every selected node decides for every candidate from the pass-start state, flips
-// its own spin bits and appends (node, chunk) entries to a work list; (U) one warp per entry
-// scatters the field changes 2 J_ij s_i(new) to the neighbours of the chunk for the flipped
-// candidates (integer atomics: exact and order-independent). Arrays that other CTAs change during
-// the kernel (h, sb, flipm, the work list) are read with ld.global.cg: the per-SM L1 is not
-// coherent with their writes. The last CTA at each barrier runs
-// the stopping rules of flip_refinement / gpu_final_sweep (models/spectral_annealing.py:983-1112).
+// A pass: (D1) every selected node decides for every candidate from the pass-start state; wanting nodes
+// go to a queue (snapshot: flip); (D2) one warp per queued node (one CTA for a long row) finds the flips
+// that no neighbour blocks, flips the node's spin bits and appends (node, chunk) entries to a work
+// list; (U) one warp per entry scatters the field changes 2 J_ij s_i(new) to the neighbours of the chunk
+// for the flipped candidates (integer atomics: exact and order-independent). Arrays that other CTAs
+// change during the kernel (h, sb, flipm, the lists) are read with ld.global.cg: the per-SM L1 is not
+// coherent with their writes. After a pass every CTA reads the flip counts and applies the stopping
+// rules of flip_refinement / gpu_final_sweep (models/spectral_annealing.py:983-1112) itself.
+//
+// What bounds it: chains of dependent loads (queue -> row -> neighbours -> their masks) over a few
+// thousand nodes, so the phases keep many loads in flight: batches of 8 field loads in D1, two row
+// entries per lane in D2, the entries of a chunk over the lanes in U, and two CTAs per SM. Search of 128
+// candidates on BA(2^16, m = 20): 16.4 -> 7.5 ms; of 40 on BA(200003, m = 15), integer weights: 15.5 -> 7.1 ms.
 #pragma once
 #include <cmath>
 #include <cstring>
@@ -135,17 +141,76 @@ __device__ void energy_phase(const LsArgs<VT, RP, GT>& A, EAcc<GT>* out, EAcc<GT
   __syncthreads();
 }
 
+// The kw words of a node's mask (p: its first one), zeros above.
+__device__ __forceinline__ void ld_words(const uint32_t* p, int kw, uint32_t (&w)[4]) {
+  w[0] = w[1] = w[2] = w[3] = 0u;
+  if (kw == 4) {
+    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p));
+    w[0] = v.x; w[1] = v.y; w[2] = v.z; w[3] = v.w;
+  } else if (kw == 2) {
+    const uint2 v = __ldcg(reinterpret_cast<const uint2*>(p));
+    w[0] = v.x; w[1] = v.y;
+  } else {
+    w[0] = __ldcg(p);
+    if (kw == 3) { w[1] = __ldcg(p + 1); w[2] = __ldcg(p + 2); }
+  }
+}
+
+// Local fields of all candidates (cp = 32: lane c has candidate 32 t + c) for entries [e0, e1) of a row,
+// in entry order: the warp reads 32 entries at a time, then each entry's spin words, four in flight.
+template <typename VT, typename RP, typename GT>
+__device__ __forceinline__ void row_fields(const LsArgs<VT, RP, GT>& A, long long e0, long long e1, GT (&acc)[4]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int t = 0; t < 4; ++t) acc[t] = GT(0);
+  for (long long e = e0; e < e1; e += 32) {
+    const int cnt = (int)((e1 - e < 32) ? e1 - e : 32);
+    int j = 0;
+    GT v = GT(0);
+    if (lane < cnt) {
+      j = __ldg(A.col + e + lane);
+      v = coupling_as<GT>(__ldg(A.val + e + lane));
+    }
+    for (int g = 0; g < cnt; g += 4) {
+      uint32_t w[4][4];
+      GT vv[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const int src = (g + q < cnt) ? g + q : 0;
+        const int jj = __shfl_sync(0xffffffffu, j, src);
+        vv[q] = __shfl_sync(0xffffffffu, v, src);
+        if (g + q < cnt) ld_words(A.sb + (long long)jj * A.kw, A.kw, w[q]);
+      }
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (g + q < cnt) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t) acc[t] += ((w[q][t] >> lane) & 1u) ? vv[q] : -vv[q];
+        }
+      }
+    }
+  }
+}
+
+constexpr int kLsLongRow = 512;   // entries above which a wanting node's row is checked by a whole CTA
+constexpr int kLsSpread = 8;      // flips of a node up to which U spreads its entries over the lanes
+
 template <typename VT, typename RP, typename GT, class Pol>
 __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& pol) {
   __shared__ EAcc<GT> s_acc[128];           // per-CTA energy sums
-  __shared__ long long s_cnt[128];
+  __shared__ int s_cnt[128];                // this CTA's flips of the pass
+  __shared__ unsigned int s_active[4];      // candidates that have not yet had a pass without a flip
+  __shared__ unsigned int s_block[4];       // blocking masks of a long row
+  __shared__ unsigned long long s_total;
   LsCtrl* C = A.ctrl;
   const int lane = threadIdx.x & 31;
   const long long gtid = pol.tid();
   const long long nthreads = pol.nthr();
   const long long gwarp = gtid >> 5, nwarps = nthreads >> 5;
   const long long n = A.n;
-  const int cp = A.cp, ne = 32 / cp, slot = lane / cp, c = lane % cp;
+  const int cp = A.cp, ne = 32 / cp, slot = lane / cp, c = lane % cp, kw = A.kw;
+  unsigned int epoch = pol.first_epoch(&C->gs);
+  auto meet = [&]() -> bool { return pol.meet(&C->gs, epoch); };
   // phase timer: the first CTA's thread 0 charges the time since its previous mark to a phase
   const bool timer = pol.block() == 0 && threadIdx.x == 0;
   unsigned long long t_mark = timer ? global_ns() : 0ull;
@@ -158,19 +223,16 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
   };
 
   // ---- L0: candidate-major packed spins -> node-major bits; zero the fields -----------------
-  if (pol.block() == 0 && threadIdx.x == 0) {
-    C->it = 0; C->round = 0; C->sub = 0; C->final_passes = 0; C->total_flips = 0; C->wl_count = 0;
-    C->wq_count = 0;
-    for (int q = 0; q < 4; ++q) C->active[q] = 0u;
-    for (int q = 0; q < A.k; ++q) C->active[q >> 5] |= 1u << (q & 31);
-    for (int q = 0; q < 128; ++q) C->counts[q] = 0;
-    for (int q = 0; q < 4; ++q) C->tph[q] = 0ull;
-    const bool main_loop = A.p.max_iterations > 0;
-    const bool final_sweep = A.p.num_rounds > 0 && A.p.final_sweep_iters > 0;
-    C->phase = main_loop ? 0 : (final_sweep ? 1 : 2);
-    C->stream = main_loop ? 0 : kFinalStreamBase;
-    C->m = main_loop ? A.m_main : A.m_final;
+  if (pol.block() == 0) {
+    if (threadIdx.x == 0)
+      for (int q = 0; q < 4; ++q) C->tph[q] = 0ull;
+    for (int q = threadIdx.x; q < 3 * (int)(sizeof(LsPass) / 4); q += blockDim.x) ((unsigned int*)C->pass)[q] = 0u;
   }
+  if (threadIdx.x < 4) {
+    const int b = A.k - 32 * (int)threadIdx.x;
+    s_active[threadIdx.x] = b >= 32 ? 0xffffffffu : (b > 0 ? (1u << b) - 1u : 0u);
+  }
+  if (threadIdx.x == 0) s_total = 0ull;
   for (long long i = gtid; i < n; i += nthreads) {
     for (int t = 0; t < A.kw; ++t) {
       uint32_t word = 0u;
@@ -181,55 +243,63 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
       }
       A.sb[i * A.kw + t] = word;
     }
-    for (int q = 0; q < A.kp; ++q) A.h[i * A.kp + q] = GT(0);
   }
+  for (long long q = gtid; q < n * A.kp; q += nthreads) A.h[q] = GT(0);
   for (long long q = gtid; q < A.kp; q += nthreads) { A.ebefore[q] = 0; A.eafter[q] = 0; }
-  if (!pol.sync(&C->gs)) return;
+  if (!meet()) return;
 
   // ---- L1: local fields h = J s for all candidates (work-list balanced) ---------------------
   for (long long itm = gwarp; itm < A.n_items; itm += nwarps) {
     const long long e0 = __ldg(&A.items[itm].e0);
     const int irow = __ldg(&A.items[itm].row);
     const int meta = __ldg(&A.items[itm].meta);
-    if (irow >= 0) {
-      const long long r1 = irow + item_nrows(meta);
-      for (long long r = irow; r < r1; ++r) {
-        const long long rs = rp_load(A.rowptr, r), re = rp_load(A.rowptr, r + 1);
-        for (int t = 0; t < A.kw; ++t) {
-          const GT f = row_field(A, rs, re, t);
-          if (slot == 0 && 32 * t + c < A.kp) A.h[r * A.kp + 32 * t + c] = f;
-        }
-      }
-    } else {
-      const long long row = -((long long)irow + 1);
-      const long long cb = e0;
-      const long long ce = e0 + item_len(meta);
-      for (int t = 0; t < A.kw; ++t) {
-        const GT f = row_field(A, cb, ce, t);
-        if (slot == 0 && 32 * t + c < A.kp) atomicAdd(&A.h[row * A.kp + 32 * t + c], f);
+    const long long row0 = irow >= 0 ? irow : -((long long)irow + 1);
+    const long long row1 = irow >= 0 ? irow + item_nrows(meta) : row0 + 1;
+    for (long long r = row0; r < row1; ++r) {
+      const long long rs = irow >= 0 ? rp_load(A.rowptr, r) : e0;
+      const long long re = irow >= 0 ? rp_load(A.rowptr, r + 1) : e0 + item_len(meta);
+      GT f[4];
+      if (cp == 32) row_fields(A, rs, re, f);
+      else f[0] = row_field(A, rs, re, 0);
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        if (t >= kw || slot != 0 || 32 * t + c >= A.kp) continue;
+        if (irow >= 0) A.h[r * A.kp + 32 * t + c] = f[t];
+        else atomicAdd(&A.h[r * A.kp + 32 * t + c], f[t]);
       }
     }
   }
-  if (!pol.sync(&C->gs)) return;
+  if (!meet()) return;
   energy_phase(A, A.ebefore, s_acc, gwarp, nwarps);
-  if (!pol.sync(&C->gs)) return;
+  if (!meet()) return;
   mark(0);
 
   // ---- passes ------------------------------------------------------------------------------
-  while (ld_volatile_i32(&C->phase) != 2) {
-    const long long m = *((volatile long long*)&C->m);
-    const long long stream = *((volatile long long*)&C->stream);
+  const bool has_final = A.p.num_rounds > 0 && A.p.final_sweep_iters > 0;
+  int phase = A.p.max_iterations > 0 ? 0 : (has_final ? 1 : 2);   // 0 main loop, 1 final sweep, 2 done
+  int it = 0, round = 0, sub = 0, final_passes = 0, set = 0;
+  // D1 tiles: TN nodes, whose `steps` (node group, candidate word) loads a warp takes 8 at a time
+  const int TN = cp < 32 || kw == 1 ? 32 : (kw == 2 ? 16 : 8);
+  const int steps = (TN / ne) * kw, inv_kw = (65536 + kw - 1) / kw;
+  const unsigned int cmask = cp == 32 ? 0xffffffffu : (1u << cp) - 1u;
+  while (phase != 2) {
+    LsPass* const cur = &C->pass[set];
+    const long long m = phase == 0 ? A.m_main : A.m_final;
     const bool all_sel = m >= n;
-    const SelKeys keys = make_sel_keys(A.p.seed, stream, n);
+    const SelKeys keys = make_sel_keys(A.p.seed, phase == 0 ? (long long)it : kFinalStreamBase + round, n);
     for (int q = threadIdx.x; q < 128; q += blockDim.x) s_cnt[q] = 0;
     __syncthreads();
+    auto push_chunks = [&](long long i, long long deg) {
+      const long long nch = deg > kChunk ? (deg + kChunk - 1) / kChunk : 1;
+      const long long pos = (long long)atomicAdd(&cur->wl, (unsigned long long)nch);
+      for (long long q = 0; q < nch && pos + q < A.wl_cap; ++q) A.wl[pos + q] = (i << 22) | q;
+    };
     // D1: every selected node decides for every candidate from the pass-start state. Snapshot
     // passes flip the wanting pairs here; priority passes record the wanting masks and ranks.
-    int cnt[4] = {0, 0, 0, 0};
-    for (long long tile = gwarp * 32; tile < n; tile += nwarps * 32) {
+    for (long long tile = gwarp * TN; tile < n; tile += nwarps * TN) {
       bool selb = false;
       int rk = 0x7fffffff;
-      if (tile + lane < n) {
+      if (lane < TN && tile + lane < n) {
         if (all_sel && !A.priority) {
           selb = true;
         } else {
@@ -240,112 +310,186 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
         if (A.priority) A.prio[tile + lane] = selb ? rk : 0x7fffffff;
       }
       const uint32_t selmask = __ballot_sync(0xffffffffu, selb);
-      for (int sub = 0; sub < 32; sub += ne) {
-        const long long i = tile + sub + slot;
-        const bool valid = i < n && ((selmask >> (sub + slot)) & 1u);
-        uint32_t fl[4] = {0u, 0u, 0u, 0u};
-        for (int t = 0; t < A.kw; ++t) {
-          bool f = false;
-          uint32_t word = 0u;
-          if (valid) {
-            word = __ldcg(A.sb + i * A.kw + t);
-            const GT hv = __ldcg(A.h + i * A.kp + 32 * t + c);
-            const bool sp = (word >> c) & 1u;
-            f = (32 * t + c < A.k) && (sp ? (hv < GT(0)) : (hv > GT(0)));
-          }
-          const uint32_t bal = __ballot_sync(0xffffffffu, f);
-          const uint32_t bits = (cp == 32) ? bal : ((bal >> (slot * cp)) & ((1u << cp) - 1u));
-          fl[t] = bits;
-          if (!A.priority) {
-            cnt[t] += f ? 1 : 0;
-            if (c == 0 && bits) A.sb[i * A.kw + t] = word ^ bits;
+      uint32_t want = 0u;   // nodes of the tile that want some candidate
+      for (int f0 = 0; f0 < steps; f0 += 8) {
+        uint32_t word[8];
+        GT hv[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int s = ((f0 + q) * inv_kw) >> 16, t = f0 + q - s * kw, node = s * ne + slot;
+          const long long i = tile + node;
+          word[q] = 0u;
+          hv[q] = GT(0);
+          if (f0 + q < steps && ((selmask >> node) & 1u)) {
+            word[q] = __ldcg(A.sb + i * kw + t);
+            hv[q] = __ldcg(A.h + i * A.kp + 32 * t + c);
           }
         }
-        if (c == 0 && i < n) {
-          uint32_t any = 0u;
-          for (int t = 0; t < A.kw; ++t) any |= fl[t];
-          if (A.priority) {
-            for (int t = 0; t < A.kw; ++t) A.wm[i * A.kw + t] = fl[t];
-            if (any) {
-              const long long pos = (long long)atomicAdd((unsigned long long*)&C->wq_count, 1ull);
-              A.wq[pos] = (int)i;
-            }
-          } else if (any) {
-            for (int t = 0; t < A.kw; ++t) A.flipm[i * A.kw + t] = fl[t];
-            const long long deg = rp_load(A.rowptr, i + 1) - rp_load(A.rowptr, i);
-            const long long nch = deg > kChunk ? (deg + kChunk - 1) / kChunk : 1;
-            const long long pos = (long long)atomicAdd((unsigned long long*)&C->wl_count, (unsigned long long)nch);
-            for (long long q = 0; q < nch && pos + q < A.wl_cap; ++q) A.wl[pos + q] = (i << 22) | q;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          if (f0 + q >= steps) break;
+          const int s = ((f0 + q) * inv_kw) >> 16, t = f0 + q - s * kw;
+          const long long i = tile + s * ne + slot;
+          // (a node that is not selected has a zero field here)
+          const bool f = (32 * t + c < A.k) && (((word[q] >> c) & 1u) ? (hv[q] < GT(0)) : (hv[q] > GT(0)));
+          const uint32_t bal = __ballot_sync(0xffffffffu, f);
+          const uint32_t bits = cp == 32 ? bal : ((bal >> (slot * cp)) & cmask);
+          if (c == 0 && i < n) {
+            (A.priority ? A.wm : A.flipm)[i * kw + t] = bits;
+            if (!A.priority && bits) A.sb[i * kw + t] = word[q] ^ bits;
           }
+          if (!A.priority && f) atomicAdd(&s_cnt[32 * t + c], 1);
+          if (bal) {
+            if (cp == 32) want |= 1u << s;
+            else
+              for (int sl = 0; sl < ne; ++sl)
+                if ((bal >> (sl * cp)) & cmask) want |= 1u << (s * ne + sl);
+          }
+        }
+      }
+      if (want) {
+        const bool mine = (want >> lane) & 1u;
+        const long long i = tile + lane;
+        const long long deg = mine ? rp_load(A.rowptr, i + 1) - rp_load(A.rowptr, i) : 0;
+        if (!A.priority) {
+          if (mine) push_chunks(i, deg);
+        } else {
+          // one reservation per tile and queue
+          const uint32_t big = __ballot_sync(0xffffffffu, deg > kLsLongRow), small = want & ~big;
+          unsigned int at = 0u, at_big = 0u;
+          if (lane == 0) {
+            if (small) at = atomicAdd(&cur->wq, (unsigned int)__popc(small));
+            if (big) at_big = atomicAdd(&cur->lq, (unsigned int)__popc(big));
+          }
+          at = __shfl_sync(0xffffffffu, at, 0);
+          at_big = __shfl_sync(0xffffffffu, at_big, 0);
+          const uint32_t below = (1u << lane) - 1u;
+          if ((small >> lane) & 1u) A.wq[at + __popc(small & below)] = (int)i;
+          if ((big >> lane) & 1u) A.wq[n - 1 - (long long)(at_big + __popc(big & below))] = (int)i;
         }
       }
     }
-    if (!A.priority) {
-      for (int t = 0; t < A.kw; ++t) {
-        int v = cnt[t];
-        for (int o = cp; o < 32; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if (slot == 0 && v) atomicAdd((unsigned long long*)&s_cnt[32 * t + c], (unsigned long long)v);
-      }
-    } else {
-      if (!pol.sync(&C->gs)) return;
-      // D2: a wanting node flips the candidates for which no wanting neighbour has a lower rank
-      // (one warp per wanting node; the blocking masks are OR-reduced over the row)
-      const long long nwq = *((volatile long long*)&C->wq_count);
-      int cnt2[4] = {0, 0, 0, 0};
-      for (long long e = gwarp; e < nwq; e += nwarps) {
-        const long long i = (long long)__ldcg(A.wq + e);
+    if (A.priority) {
+      if (!meet()) return;
+      // every CTA is past the reading of the last pass's counters: the set of the pass after next
+      if (pol.block() == 0)
+        for (int q = threadIdx.x; q < (int)(sizeof(LsPass) / 4); q += blockDim.x)
+          ((unsigned int*)&C->pass[set == 0 ? 2 : set - 1])[q] = 0u;
+      // D2: a wanting node flips the candidates for which no wanting neighbour has a lower rank (the
+      // blocking masks are OR-reduced over the row). Long rows: one CTA each.
+      auto commit = [&](long long i, const uint32_t (&W)[4], long long deg) {
+        for (int t = 0; t < kw; ++t) {
+          A.flipm[i * kw + t] = W[t];
+          if (W[t]) A.sb[i * kw + t] = __ldcg(A.sb + i * kw + t) ^ W[t];
+        }
+        push_chunks(i, deg);
+      };
+      const long long nlq = (long long)ld_volatile_u32(&cur->lq), nwq = (long long)ld_volatile_u32(&cur->wq);
+      for (long long e = pol.block(); e < nlq; e += pol.nblocks()) {
+        const long long i = (long long)__ldcg(A.wq + n - 1 - e);
         const int pi = __ldcg(A.prio + i);
-        uint32_t W[4] = {0u, 0u, 0u, 0u}, B[4] = {0u, 0u, 0u, 0u};
-        for (int t = 0; t < A.kw; ++t) W[t] = __ldcg(A.wm + i * A.kw + t);
         const long long rs = rp_load(A.rowptr, i), re = rp_load(A.rowptr, i + 1);
-        for (long long p = rs + lane; p < re; p += 32) {
+        uint32_t B[4] = {0u, 0u, 0u, 0u}, W[4];
+        if (threadIdx.x < 4) s_block[threadIdx.x] = 0u;
+        __syncthreads();
+        for (long long p = rs + threadIdx.x; p < re; p += blockDim.x) {
           const int j = __ldg(A.col + p);
-          if (__ldcg(A.prio + j) < pi)
-            for (int t = 0; t < A.kw; ++t) B[t] |= __ldcg(A.wm + (long long)j * A.kw + t);
+          if (__ldcg(A.prio + j) < pi) {
+            uint32_t w[4];
+            ld_words(A.wm + (long long)j * kw, kw, w);
+#pragma unroll
+            for (int t = 0; t < 4; ++t) B[t] |= w[t];
+          }
+        }
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          const uint32_t b = __reduce_or_sync(0xffffffffu, B[t]);
+          if (lane == 0 && b) atomicOr(&s_block[t], b);
+        }
+        __syncthreads();
+        ld_words(A.wm + i * kw, kw, W);
+        uint32_t any = 0u;
+#pragma unroll
+        for (int t = 0; t < 4; ++t) any |= (W[t] &= ~s_block[t]);
+        if (threadIdx.x < 32) {
+#pragma unroll
+          for (int t = 0; t < 4; ++t)
+            if ((W[t] >> lane) & 1u) atomicAdd(&s_cnt[32 * t + lane], 1);
+          if (lane == 0 && any) commit(i, W, re - rs);
+        }
+        __syncthreads();
+      }
+      int cnt[4] = {0, 0, 0, 0};
+      long long i = gwarp < nwq ? (long long)__ldcg(A.wq + gwarp) : 0;
+      for (long long e = gwarp; e < nwq; e += nwarps) {
+        const long long next = e + nwarps < nwq ? (long long)__ldcg(A.wq + e + nwarps) : 0;
+        const int pi = __ldcg(A.prio + i);
+        const long long rs = rp_load(A.rowptr, i), re = rp_load(A.rowptr, i + 1);
+        uint32_t W[4], B[4] = {0u, 0u, 0u, 0u};
+        ld_words(A.wm + i * kw, kw, W);
+        for (long long p = rs + lane; p < re; p += 64) {
+          const bool two = p + 32 < re;
+          const int j0 = __ldg(A.col + p), j1 = two ? __ldg(A.col + p + 32) : 0;
+          const int p0 = __ldcg(A.prio + j0), p1 = two ? __ldcg(A.prio + j1) : 0x7fffffff;
+          uint32_t w0[4] = {0u, 0u, 0u, 0u}, w1[4] = {0u, 0u, 0u, 0u};
+          if (p0 < pi) ld_words(A.wm + (long long)j0 * kw, kw, w0);
+          if (p1 < pi) ld_words(A.wm + (long long)j1 * kw, kw, w1);
+#pragma unroll
+          for (int t = 0; t < 4; ++t) B[t] |= w0[t] | w1[t];
         }
         uint32_t any = 0u;
-        for (int t = 0; t < A.kw; ++t) {
-          B[t] = __reduce_or_sync(0xffffffffu, B[t]);
-          W[t] &= ~B[t];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) {
+          if (t < kw) W[t] &= ~__reduce_or_sync(0xffffffffu, B[t]);
           any |= W[t];
-          cnt2[t] += (W[t] >> lane) & 1u;
+          cnt[t] += (W[t] >> lane) & 1u;
         }
-        if (lane == 0 && any) {
-          for (int t = 0; t < A.kw; ++t) {
-            A.flipm[i * A.kw + t] = W[t];
-            if (W[t]) A.sb[i * A.kw + t] = __ldcg(A.sb + i * A.kw + t) ^ W[t];
-          }
-          const long long deg = re - rs;
-          const long long nch = deg > kChunk ? (deg + kChunk - 1) / kChunk : 1;
-          const long long pos = (long long)atomicAdd((unsigned long long*)&C->wl_count, (unsigned long long)nch);
-          for (long long q = 0; q < nch && pos + q < A.wl_cap; ++q) A.wl[pos + q] = (i << 22) | q;
-        }
+        if (lane == 0 && any) commit(i, W, re - rs);
+        i = next;
       }
-      for (int t = 0; t < A.kw; ++t)
-        if (cnt2[t]) atomicAdd((unsigned long long*)&s_cnt[32 * t + lane], (unsigned long long)cnt2[t]);
+#pragma unroll
+      for (int t = 0; t < 4; ++t)
+        if (cnt[t]) atomicAdd(&s_cnt[32 * t + lane], cnt[t]);
     }
     __syncthreads();
     for (int q = threadIdx.x; q < A.k; q += blockDim.x)
-      if (s_cnt[q]) atomicAdd((unsigned long long*)&C->counts[q], (unsigned long long)s_cnt[q]);
-    if (!pol.sync(&C->gs)) return;
+      if (s_cnt[q]) atomicAdd(&cur->counts[q], s_cnt[q]);
+    if (!meet()) return;
     mark(1);
 
-    // U: scatter field changes of the flipped (node, candidate) pairs
-    const long long nwl = min(*((volatile long long*)&C->wl_count), A.wl_cap);
+    // U: scatter field changes of the flipped (node, candidate) pairs. Few flips: the chunk's entries
+    // over the lanes, flip after flip; many: candidates over the lanes, entry after entry, where the
+    // updates of an entry share sectors (from about 8 of the 128-byte line's 32 on).
+    const long long nwl = min((long long)*((volatile unsigned long long*)&cur->wl), A.wl_cap);
     for (long long e = gwarp; e < nwl; e += nwarps) {
       const long long ent = __ldcg(A.wl + e);
       const long long i = ent >> 22;
       const long long q = ent & ((1ll << 22) - 1);
       const long long rs = rp_load(A.rowptr, i), re = rp_load(A.rowptr, i + 1);
+      uint32_t F[4], S[4];
+      ld_words(A.flipm + i * kw, kw, F);
+      ld_words(A.sb + i * kw, kw, S);
       const long long cb = rs + q * kChunk;
       const long long ce = (cb + kChunk < re) ? cb + kChunk : re;
-      for (int t = 0; t < A.kw; ++t) {
-        const uint32_t F = __ldcg(A.flipm + i * A.kw + t);
-        if (!F) continue;
-        const uint32_t S = __ldcg(A.sb + i * A.kw + t);
-        const bool mine = (F >> c) & 1u;
-        const bool up = (S >> c) & 1u;
-        if (!mine) continue;
+      if (__popc(F[0]) + __popc(F[1]) + __popc(F[2]) + __popc(F[3]) <= kLsSpread) {
+        for (long long p = cb + lane; p < ce; p += 32) {
+          GT* hj = A.h + (long long)__ldg(A.col + p) * A.kp;
+          const GT v2 = GT(2) * coupling_as<GT>(__ldg(A.val + p));
+#pragma unroll
+          for (int t = 0; t < 4; ++t) {
+            for (uint32_t b = F[t]; b; b &= b - 1u) {
+              const int cc = __ffs(b) - 1;
+              atomicAdd(hj + 32 * t + cc, ((S[t] >> cc) & 1u) ? v2 : -v2);
+            }
+          }
+        }
+        continue;
+      }
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        if (!((F[t] >> c) & 1u)) continue;
+        const bool up = (S[t] >> c) & 1u;
+#pragma unroll 4
         for (long long p = cb + slot; p < ce; p += ne) {
           const int j = __ldg(A.col + p);
           const GT v = coupling_as<GT>(__ldg(A.val + p));
@@ -353,43 +497,44 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
         }
       }
     }
-    if (!pol.sync(&C->gs, [&] {
-          if (threadIdx.x == 0) {
-            long long tot = 0;
-            bool any = false;
-            for (int q = 0; q < A.k; ++q) {
-              const long long cq = C->counts[q];
-              tot += cq;
-              any |= cq > 0;
-              if (C->phase == 0 && cq == 0) C->active[q >> 5] &= ~(1u << (q & 31));
-              C->counts[q] = 0;
-            }
-            C->total_flips += tot;
-            C->wl_count = 0;
-            C->wq_count = 0;
-            if (C->phase == 0) {
-              C->it += 1;
-              const bool any_active = (C->active[0] | C->active[1] | C->active[2] | C->active[3]) != 0u;
-              if (!any_active || C->it >= A.p.max_iterations) {
-                const bool final_sweep = A.p.num_rounds > 0 && A.p.final_sweep_iters > 0;
-                C->phase = final_sweep ? 1 : 2;
-                C->round = 0;
-                C->sub = 0;
-              }
-            } else {
-              C->sub += 1;
-              C->final_passes += 1;
-              if (!any || C->sub >= A.p.final_sweep_iters) {
-                C->round += 1;
-                C->sub = 0;
-                if (C->round >= A.p.num_rounds) C->phase = 2;
-              }
-            }
-            if (C->phase == 0) { C->stream = C->it; C->m = A.m_main; }
-            else if (C->phase == 1) { C->stream = kFinalStreamBase + C->round; C->m = A.m_final; }
-          }
-        })) return;
+    if (!meet()) return;
+    // the stopping rules, in every CTA
+    const int cq = (int)threadIdx.x < A.k ? __ldcg(&cur->counts[threadIdx.x]) : 0;
+    if (threadIdx.x < 128) {
+      const unsigned int flipped = __ballot_sync(0xffffffffu, cq > 0);
+      if (lane == 0 && phase == 0) s_active[threadIdx.x >> 5] &= flipped;
+      if (timer || pol.block() == 0) {
+        const int tot = __reduce_add_sync(0xffffffffu, cq);
+        if (lane == 0) atomicAdd(&s_total, (unsigned long long)tot);
+      }
+    }
+    const bool any = __syncthreads_or(cq > 0);
+    if (!A.priority && pol.block() == 0)   // (a snapshot pass has no barrier between D1 and here)
+      for (int q = threadIdx.x; q < (int)(sizeof(LsPass) / 4); q += blockDim.x)
+        ((unsigned int*)&C->pass[set == 0 ? 2 : set - 1])[q] = 0u;
+    set = set == 2 ? 0 : set + 1;
+    if (phase == 0) {
+      it += 1;
+      if (!(s_active[0] | s_active[1] | s_active[2] | s_active[3]) || it >= A.p.max_iterations) {
+        phase = has_final ? 1 : 2;
+        round = 0;
+        sub = 0;
+      }
+    } else {
+      sub += 1;
+      final_passes += 1;
+      if (!any || sub >= A.p.final_sweep_iters) {
+        round += 1;
+        sub = 0;
+        if (round >= A.p.num_rounds) phase = 2;
+      }
+    }
     mark(2);
+  }
+  if (timer) {
+    C->it = it;
+    C->final_passes = final_passes;
+    C->total_flips = (long long)s_total;
   }
 
   // ---- energies after, refined candidates back to candidate-major ---------------------------
