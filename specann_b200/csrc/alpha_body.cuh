@@ -15,6 +15,7 @@
 #pragma once
 #include <cmath>
 #include <cstdio>
+#include <type_traits>
 
 #include "common.cuh"
 #include "handle.cuh"
@@ -66,6 +67,7 @@ struct AlphaArgs {
   SpmvArgs<T, RP> split[kMaxSplits];   // L2 column splits of the operator (n_splits > 0): one
   int n_splits;                        // work-list pass per split, partial row sums in split_part
   T* split_part;
+  int long_rows;         // rows of several chunks in the work list (RowStep::fixed is in use)
   int cluster;           // the grid is one cluster (GridPolicy)
 };
 
@@ -608,10 +610,10 @@ struct PhaseSums {
     else __stcg(part + ((long long)buf * COLS + col) * nblk + pol.block(), v);
   }
   template <int NV>
-  __device__ __forceinline__ void block_put(const double (&v)[NV]) {
+  __device__ __forceinline__ void block_put(const double (&v)[NV], int cols = NV) {
     static_assert(NV <= 3, "staging of block_put");
-    const double acc = cta_sums(v[0], NV > 1 ? v[NV > 1] : 0.0, NV > 2 ? v[NV > 2 ? 2 : 0] : 0.0, NV, sm);
-    if (threadIdx.x < NV) put(threadIdx.x, acc);
+    const double acc = cta_sums(v[0], NV > 1 ? v[NV > 1] : 0.0, NV > 2 ? v[NV > 2 ? 2 : 0] : 0.0, cols, sm);
+    if ((int)threadIdx.x < cols) put(threadIdx.x, acc);
   }
   __device__ __forceinline__ bool all_sum(int cols) {
     if (!meet()) return false;
@@ -1083,7 +1085,12 @@ struct RowStep {
   double theta;
   bool last;
   double acc;
+  // Parts of V[j] . w from rows that any warp may finish, as multiples of 1 / scale: their sum is exact, so
+  // a_j, and with it every later step, does not depend on which warp it was.
+  double scale;
+  long long fixed;
   __device__ __forceinline__ RowInputs<T> pre(long long r) const { return RowInputs<T>{__ldcg(xin + r), __ldcg(sigma + r)}; }
+  template <bool kAny = false>
   __device__ __forceinline__ void fin(long long r, T s, const RowInputs<T>& in) {
     const T wr = in.x;
     const T sw = rho * wr - in.s * s;
@@ -1095,7 +1102,9 @@ struct RowStep {
       const T wn = sw * inv_b;
       vj[r] = vr;
       w[r] = wn;
-      acc += (double)vr * (double)wn;
+      const double part = (double)vr * (double)wn;
+      if (kAny) fixed += __double2ll_rn(part * scale);
+      else acc += part;
     }
   }
 };
@@ -1121,11 +1130,15 @@ __device__ __forceinline__ void items_pass(const SpmvArgs<T, RP>& S, const T* u,
                                         T* part, int mode) {
   RowStep<T> f = out;
   const SpmvArgs<T, RP> L = S;
-  spmv_items<T, RP, false, NW>(L, u, gwarp, nwarps, alpha_work<T, NW>().spmv, [&](long long r, T s) {
+  auto row = [&](auto any, long long r, T s) {
     const T sum = (mode & 1) ? s : __ldcg(part + r) + s;
-    if (mode & 2) f.fin(r, sum, f.pre(r));
+    if (mode & 2) f.template fin<decltype(any)::value>(r, sum, f.pre(r));
     else __stcg(part + r, sum);
-  });
+  };
+  spmv_items<T, RP, false, NW>(L, u, gwarp, nwarps, alpha_work<T, NW>().spmv,
+                               [&](long long r, T s) { row(std::false_type{}, r, s); },
+                               [&](long long r, T s) { row(std::true_type{}, r, s); });
+  out.fixed = f.fixed;
   out.acc = f.acc;
 }
 
@@ -1154,6 +1167,8 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
   const sa_alpha_params& P = A.p;
   const double rho = P.rho;
   const double bound = 10.0 * (P.rho + P.gershgorin);
+  // |a_j| is at most 2 rho < bound: 2^61 / bound or more keeps the sums of RowStep::fixed below 2^62
+  const double fix_scale = scalbn(1.0, 60 - ilogb(fmax(bound, 1.0)));
   const int ncv = P.ncv;
   constexpr int VW = 16 / sizeof(T);
   const long long nvt = (n + VW - 1) / VW;   // positions of the vector phases
@@ -1373,14 +1388,16 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
       if (!pass2 && (!last || P.residual_check)) {
         // P1: V[j] = w * inv_b; w <- S V[j]; partial sums of a_j = V[j] . w. (The final pass shares the
         // operator's code: F2 |S y - theta y|^2.)
-        RowStep<T> f{last ? A.yout : A.w, A.sigma, A.V + (long long)j * A.ldv, A.w, (T)rho, (T)C->inv_b, C->theta, last, 0.0};
+        RowStep<T> f{last ? A.yout : A.w, A.sigma, A.V + (long long)j * A.ldv, A.w, (T)rho, (T)C->inv_b, C->theta, last, 0.0, fix_scale, 0ll};
         if (!apply(f)) return;
-        const double pa[1] = {f.acc};
-        sums.block_put(pa);
+        // the fixed-point part in two columns, whose sums are exact integers in any order
+        const int cols = !last && kMode != ALPHA_PANEL && A.long_rows ? 3 : 1;
+        const double pa[3] = {f.acc, (double)(f.fixed >> 32), (double)(f.fixed & 0xffffffffll)};
+        sums.block_put(pa, cols);
         if (last) break;
-        if (!sums.all_sum(1)) return;
+        if (!sums.all_sum(cols)) return;
         if (threadIdx.x == 0) {
-          C->a[j] = tot[0];
+          C->a[j] = cols == 1 ? tot[0] : tot[0] + (tot[1] * 0x1p32 + tot[2]) / fix_scale;
           C->bytes += A.spmv_bytes + (double)n * sizeof(T);
           C->spmvs += 1;
         }

@@ -97,6 +97,7 @@ int launch_alpha(sa_handle* h, const sa_alpha_params* p) {
         cudaSuccess)
       return SA_ERR_CUDA;
   }
+  A.long_rows = mode == ALPHA_LARGE || h->n_mc > 0;   // (the splits have row chunks of their own)
   A.n_splits = 0;
   A.split_part = nullptr;
   if (mode == ALPHA_LARGE && h->split_on) {

@@ -275,6 +275,7 @@ __device__ bool batch_problem(const BatchArgs& B, const BTeam& tm, int p, const 
         A.S.long_part = (T*)tm.long_part;
         A.S.scol = I.scol;
         A.S.wmag = (T)I.wmag;
+        A.long_rows = 1;
         A.n_splits = 0;
         A.n = n;
         A.ldv = I.ldv;

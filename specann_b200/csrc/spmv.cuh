@@ -158,10 +158,12 @@ __device__ __forceinline__ void load_tile(const SpmvArgs<T, RP>& S, const TileDe
   }
 }
 
-// fin(row, sum) is called exactly once per row with sum = sum_j val_ij * u_j (T arithmetic).
-template <typename T, typename RP, bool kReadOnlyU = false, int NW = kWarps, class Fin>
+// fin(row, sum) is called exactly once per row with sum = sum_j val_ij * u_j (T arithmetic), by a warp
+// that follows from the work list alone; for a row of several chunks it is fin_any instead, called by
+// the warp that happens to finish last.
+template <typename T, typename RP, bool kReadOnlyU = false, int NW = kWarps, class Fin, class FinAny>
 __device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u, long long gwarp,
-                                           long long nwarps, SpmvSmem<T, NW>& sm, Fin&& fin) {
+                                           long long nwarps, SpmvSmem<T, NW>& sm, Fin&& fin, FinAny&& fin_any) {
   const int tid = tid_here();
   const int lane = tid & 31;
   const int wid = tid >> 5;
@@ -227,7 +229,7 @@ __device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u,
             T tot = T(0);
             for (int c = 0; c < nch; ++c) tot += *((volatile T*)(S.long_part + base + c));
             S.mc_count[z] = 0;
-            fin(row, tot);
+            fin_any(row, tot);
           }
         }
       }
@@ -242,6 +244,12 @@ __device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u,
     }
     it += nwarps;
   }
+}
+
+template <typename T, typename RP, bool kReadOnlyU = false, int NW = kWarps, class Fin>
+__device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u, long long gwarp,
+                                           long long nwarps, SpmvSmem<T, NW>& sm, Fin&& fin) {
+  spmv_items<T, RP, kReadOnlyU, NW>(S, u, gwarp, nwarps, sm, fin, fin);
 }
 
 }  // namespace sa

@@ -40,6 +40,11 @@ def check(J, precision, alpha, ncv=33, keep=0, layout="worklist", tol=1e-6):
     assert abs(lam - ref) <= (1e-6 if precision == 32 else 1e-8)
     eng.keep_candidate(0)
     assert np.array_equal(eng.candidate_spins(0).cpu().numpy(), np.where(y >= 0, 1, -1).astype(np.int8))
+    again = eng.alpha_solve(alpha=alpha, alpha_prev=alpha, rho=1.001, gershgorin=1.0, tol=tol, pred_tol=1e-3,
+                            maxiter=4000, ncv=ncv, start_mode=_lib.SA_START_RANDOM, seed=7, stream_id=0, align=False,
+                            restart_keep=keep)
+    assert again.mu == rec.mu and again.iterations == rec.iterations   # no dependence on timing
+    assert torch.equal(eng.result_vector().double().cpu(), torch.from_numpy(y))
     eng.close()
 
 
