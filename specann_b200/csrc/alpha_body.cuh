@@ -1145,8 +1145,10 @@ __device__ __forceinline__ void items_pass(const SpmvArgs<T, RP>& S, const T* u,
 // What a kernel is compiled for (all in one would hold more registers than a thread has, and spill them
 // through the little L1 that the panels leave): the work list with register-held vector phases (small
 // problems and the batch kernel); the column panels with streamed vector phases; the work list or the
-// L2 column splits with streamed vector phases.
-enum AlphaMode : int { ALPHA_SMALL = 0, ALPHA_PANEL = 1, ALPHA_LARGE = 2 };
+// L2 column splits with streamed vector phases; the column panels with register-held ones.
+enum AlphaMode : int { ALPHA_SMALL = 0, ALPHA_PANEL = 1, ALPHA_LARGE = 2, ALPHA_PANEL_SMALL = 3 };
+__host__ __device__ constexpr bool alpha_panels(int mode) { return mode == ALPHA_PANEL || mode == ALPHA_PANEL_SMALL; }
+__host__ __device__ constexpr bool alpha_streams(int mode) { return mode == ALPHA_PANEL || mode == ALPHA_LARGE; }
 
 // NW: warps per CTA at most (sizes the shared staging).
 template <typename T, typename RP, class Pol, int NW, int kMode>
@@ -1173,13 +1175,13 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
   constexpr int VW = 16 / sizeof(T);
   const long long nvt = (n + VW - 1) / VW;   // positions of the vector phases
   unsigned ppar = 0;   // phase bits of the panel barriers
-  if (kMode == ALPHA_PANEL) panel_init(pbars, kPanelBufs);
+  if (alpha_panels(kMode)) panel_init(pbars, kPanelBufs);
   unsigned vpar = 0;   // and of the vector streams'
-  if (kMode != ALPHA_SMALL) panel_init(vbars, stream_bufs(sizeof(T)));
+  if (alpha_streams(kMode)) panel_init(vbars, stream_bufs(sizeof(T)));
   PhaseSums<Pol, kPartCols> sums(pol, &G->gs, A.part, sm, tot);
   // one operator application (this thread's sum goes to f.acc); false on a timed-out wait
   auto apply = [&](RowStep<T>& f) -> bool {
-    if constexpr (kMode == ALPHA_PANEL) {
+    if constexpr (alpha_panels(kMode)) {
       return panel_pass<T>(A.panel, A.u, blk, nblk, pbars, ppar, &G->gs.error, f);
     } else {
       // pass q adds the row sums of split q (the work list is one pass); a barrier makes them visible to
@@ -1391,7 +1393,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
         RowStep<T> f{last ? A.yout : A.w, A.sigma, A.V + (long long)j * A.ldv, A.w, (T)rho, (T)C->inv_b, C->theta, last, 0.0, fix_scale, 0ll};
         if (!apply(f)) return;
         // the fixed-point part in two columns, whose sums are exact integers in any order
-        const int cols = !last && kMode != ALPHA_PANEL && A.long_rows ? 3 : 1;
+        const int cols = !last && !alpha_panels(kMode) && A.long_rows ? 3 : 1;
         const double pa[3] = {f.acc, (double)(f.fixed >> 32), (double)(f.fixed & 0xffffffffll)};
         sums.block_put(pa, cols);
         if (last) break;
@@ -1408,7 +1410,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
       // P2: three-term step and reorthogonalisation coefficients
       {
         const double a3 = pass2 ? 0.0 : C->a[j], b3 = (pass2 || j == 0) ? 0.0 : C->b[j - 1];
-        if constexpr (kMode != ALPHA_SMALL) {
+        if constexpr (alpha_streams(kMode)) {
           extern __shared__ __align__(128) char stream_smem[];
           VecStream<T> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
           if (!stream_dots<T>(S, A.V, A.ldv, A.w, A.u, j, pass2, a3, b3, work.dots)) return;
@@ -1436,7 +1438,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
       {
         const T* src = pass2 ? A.w : A.u;
         double v[1] = {0.0};
-        if constexpr (kMode != ALPHA_SMALL) {
+        if constexpr (alpha_streams(kMode)) {
           extern __shared__ __align__(128) char stream_smem[];
           VecStream<T> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
           if (!stream_update<T>(S, A.V, A.ldv, src, A.sigma, A.w, A.u, j, C->h, v[0])) return;

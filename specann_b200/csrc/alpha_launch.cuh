@@ -22,6 +22,7 @@ __global__ void __launch_bounds__(kThreads, 1) alpha_kernel(const __grid_constan
 template <typename T, typename RP>
 const void* alpha_kernel_of(int mode) {
   if (mode == ALPHA_PANEL) return (const void*)alpha_kernel<T, RP, ALPHA_PANEL>;
+  if (mode == ALPHA_PANEL_SMALL) return (const void*)alpha_kernel<T, RP, ALPHA_PANEL_SMALL>;
   if (mode == ALPHA_LARGE) return (const void*)alpha_kernel<T, RP, ALPHA_LARGE>;
   return (const void*)alpha_kernel<T, RP, ALPHA_SMALL>;
 }
@@ -29,11 +30,12 @@ const void* alpha_kernel_of(int mode) {
 // Vector phases streamed through shared memory when a thread has more than half a 16-byte position of
 // the vectors, held in registers below. One step's dots and update at n = 2^16 in FP64 (43 % of a
 // position): 16.9 us in registers, 24 us streamed; at n = 2^20 in FP32 (346 %): 71 us in registers
-// (85 us where they spill), 52.5 us streamed.
+// (85 us where they spill), 52.5 us streamed; with panels at n = 2^16 in FP32 (22 %): 18.4 against 26.3 us.
 inline int alpha_mode(const sa_handle* h) {
-  if (h->panel_on) return ALPHA_PANEL;
   const long long positions = h->n * (h->prec == 32 ? 4 : 8) / 16;
-  return h->split_on || 2 * positions > (long long)h->blocks * kThreads ? ALPHA_LARGE : ALPHA_SMALL;
+  const bool large = 2 * positions > (long long)h->blocks * kThreads;
+  if (h->panel_on) return large ? ALPHA_PANEL : ALPHA_PANEL_SMALL;
+  return h->split_on || large ? ALPHA_LARGE : ALPHA_SMALL;
 }
 
 // CTAs of the one cluster that a problem runs on, 0 for the whole (cooperative) grid. A cluster's hardware
@@ -88,9 +90,9 @@ int launch_alpha(sa_handle* h, const sa_alpha_params* p) {
   A.spmv_bytes = (double)h->nnz * (4.0 + sizeof(T)) + (double)(h->n + 1) * sizeof(RP) + 3.0 * (double)h->n * sizeof(T);
   const int mode = alpha_mode(h);
   const void* kernel = alpha_kernel_of<T, RP>(mode);
-  A.panel = mode == ALPHA_PANEL ? panel_args(h) : PanelArgs{};
-  const int dyn = std::max(mode == ALPHA_PANEL ? panel_smem_bytes((int)sizeof(T)) : 0,
-                           mode != ALPHA_SMALL ? stream_smem_bytes((int)sizeof(T)) : 0);
+  A.panel = alpha_panels(mode) ? panel_args(h) : PanelArgs{};
+  const int dyn = std::max(alpha_panels(mode) ? panel_smem_bytes((int)sizeof(T)) : 0,
+                           alpha_streams(mode) ? stream_smem_bytes((int)sizeof(T)) : 0);
   if (dyn > 0) {
     // set on every launch: the attribute belongs to the current device
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) !=

@@ -134,10 +134,12 @@ class Engine:
         return int(nb.value), int(blocks.value)
 
     def panels_pay(self) -> bool:
-        """The column-panel SpMV is chosen in FP32 when rows average at least 16 entries and every
-        SM holds one row block (in FP64 the persistent kernels spill with its shared-memory budget
-        and the alpha solve measured slower: 15.6 against 11.5 ms on BA(2^18, 20))."""
-        if self.precision != 32 or self.n < 4096 or self.nnz < 16 * self.n:
+        """The column-panel SpMV is chosen when every SM holds one row block and, in FP32, rows average at
+        least 16 entries (n >= 4096); in FP64, where a panel holds half the columns, rows average at least
+        32 (n >= 65536). A Lanczos step in FP64, work list against panels: BA(2^16, 20) 46.5 against
+        42.9 us, BA(2^18, 20) 120 against 98 us, BA(150000, 10) 57.0 against 62.5 us."""
+        n_min, row_min = (4096, 16) if self.precision == 32 else (65536, 32)
+        if self.n < n_min or self.nnz < row_min * self.n:
             return False
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         try:

@@ -163,8 +163,8 @@ class SpectralAnnealing:
         self.tangent_tol = float(kwargs.pop("tangent_tol", 1e-2))
         # Ritz vectors kept by an implicit restart of the Lanczos basis (0: the kernel's default, 8)
         self.restart_keep = int(kwargs.pop("restart_keep", 0))
-        # operator layout: "auto" (column panels when rows average >= 16 entries and the row
-        # blocks fit the SMs; L2 column splits when the gathered vector is larger than 48 MB; else
+        # operator layout: "auto" (column panels when rows average >= 16 entries, in FP64 >= 32, and the
+        # row blocks fit the SMs; L2 column splits when the gathered vector is larger than 48 MB; else
         # the work list), "panel", "split" or "worklist"
         self.spmv = str(kwargs.pop("spmv", "auto"))
         if self.spmv not in ("auto", "panel", "split", "worklist"):

@@ -1,0 +1,53 @@
+"""The batched local search at the edges of its passes: candidate counts around the word and tile widths,
+rows around the length from which a whole CTA checks them, both pass semantics; spins, energies and
+pass counts exact against the oracle."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+if not torch.cuda.is_available():
+    pytest.skip("no CUDA device", allow_module_level=True)
+
+from oracle import specann_oracle as O  # noqa: E402
+from specann_b200 import graphs  # noqa: E402
+from specann_b200.engine import Engine  # noqa: E402
+
+
+def with_hubs(n, degrees, seed):
+    """A +-1 Barabasi-Albert graph whose first nodes are joined to more nodes, up to the given degrees."""
+    J = graphs.barabasi_albert(n, 6, seed=seed, couplings="pm1").tolil()
+    rng = np.random.default_rng(seed)
+    for hub, deg in enumerate(degrees):
+        have = set(J.rows[hub]) | {hub}
+        free = np.array([v for v in range(n) if v not in have])
+        for v in rng.permutation(free)[: max(0, deg - len(J.rows[hub]))]:
+            J[hub, v] = J[v, hub] = float(rng.choice([-1, 1]))
+    return sp.csr_matrix(J)
+
+
+@pytest.fixture(scope="module")
+def hubs():
+    # 512 / 513: the longest row of a warp and the shortest of a CTA; 1400: several chunks
+    return with_hubs(1501, (512, 513, 1400), seed=4)
+
+
+@pytest.mark.parametrize("semantics", ["priority", "snapshot"])
+@pytest.mark.parametrize("k", [1, 8, 9, 16, 17, 33, 70, 128])
+def test_search_matches_oracle(hubs, k, semantics):
+    n = hubs.shape[0]
+    S = np.where(np.random.default_rng(k).random((k, n)) < 0.5, 1, -1).astype(np.int8)
+    eng = Engine(n, hubs.nnz, precision=32, ncv_max=4, max_candidates=k)
+    eng.upload_csr(hubs.indptr, hubs.indices, hubs.data.astype(np.float32))
+    for c in range(k):
+        eng.set_candidate(c, S[c])
+    iters, rounds = (1000, 25) if semantics == "priority" else (12, 3)   # snapshot passes may oscillate
+    eb, ea, res = eng.local_search(k, max_iterations=iters, num_rounds=rounds, seed=5, semantics=semantics)
+    ref = O.local_search(hubs, S, seed=5, max_iterations=iters, num_rounds=rounds, semantics=semantics)
+    got = np.stack([eng.candidate_spins(c, refined=True).cpu().numpy() for c in range(k)])
+    assert np.array_equal(got, ref.spins)
+    assert np.array_equal(ea, np.asarray(ref.energies_after, dtype=np.float64))
+    assert res.iterations == ref.iterations
+    eng.close()
