@@ -825,7 +825,7 @@ struct VecStream {
                      : "memory");
       __syncwarp();
       if (q < m) {
-        fence_proxy_async();
+        if (k < kBufs) fence_proxy_async();   // (before the first copies; a refill only follows reads)
         bulk_load(smem + (b * kStreamVecs + q) * kStreamTile, vec(g * kStreamVecs + q) + tile_row0(t), bytes, &bars[b]);
       }
     };
