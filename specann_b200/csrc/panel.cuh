@@ -140,8 +140,22 @@ template <typename T>
 __device__ __forceinline__ void panel_load_vals(const T* val, long long e, long long ce, int lane,
                                                 T (&v)[kPanelLane], unsigned long long pol) {
   const long long k = e + (long long)kPanelLane * lane;
+  if (k < ce) {
+    // 16-byte loads as for the words (a lane's slots start on 32 or 64 bytes). One load a value was
+    // bound by the load unit: the FP32 operator took 38.6 instead of 29.2 us at BA(150,001) and 194
+    // instead of 133 us at BA(2^20), both with values in +-1..100.
+    constexpr int VW = 16 / sizeof(T);
 #pragma unroll
-  for (int j = 0; j < kPanelLane; ++j) v[j] = (k < ce) ? ld_stream(val + k + j, pol) : T(0);
+    for (int j = 0; j < kPanelLane; j += VW) {
+      const uint4 x = ld_stream_v4(reinterpret_cast<const unsigned*>(val + k + j), pol);
+      const T* c = reinterpret_cast<const T*>(&x);
+#pragma unroll
+      for (int q = 0; q < VW; ++q) v[j + q] = c[q];
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < kPanelLane; ++j) v[j] = T(0);
+  }
 }
 
 // Products of one batch added into the block's row sums ys. The entries are in row order, so
@@ -294,7 +308,7 @@ __device__ __forceinline__ bool panel_spmv(const PanelArgs& P, const T* u, int b
       }
       // (no proxy fence: the buffer was only read through the generic proxy, and those reads are done. A
       // fence per panel waits for everything the thread has outstanding: the operator at n = 2^20 took 127
-      // instead of 120 us, in FP64 at n = 160,001 59 instead of 47.5 us.)
+      // instead of 120 us, the FP64 SpMV steps of the gradient's eigenpair at n = 2^18 69 instead of 67 us.)
       if (tid == 0 && p + kPanelBufs < np) {
         panel_issue<T>(P, u, p + kPanelBufs, smem, bars);
       }
