@@ -1486,7 +1486,20 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
           hlo = th0 - 2.0 * r0 - pad;
           hhi = th0 + pad;
         }
-        const double th = smallest_eig_block(C->a, C->b, m, &s2, hlo, hhi);
+        double th = 0.0;
+        const bool shared_test = Pol::kShareRitz && nblk > 1;
+        if (!shared_test || blk == 0) th = smallest_eig_block(C->a, C->b, m, &s2, hlo, hhi);
+        if (shared_test) {
+          if (blk == 0 && threadIdx.x == 0) {
+            G->theta = th;
+            G->scale = s2;
+          }
+          if (!sums.meet()) return;
+          if (blk != 0) {
+            th = vload(&G->theta);
+            s2 = vload(&G->scale);
+          }
+        }
         if (threadIdx.x == 0) {
           const double res = bj * sqrt(s2);
           const bool invariant = bj <= 1e-14 * bound;

@@ -49,6 +49,7 @@ struct BInstance {
   long long n, nnz, W, ldv;
   double c, dmin, dmax, half_log2_c, sqrt_c;
   int integer_J, rp64;
+  int long_rows;     // rows of several chunks in items (their step has two more sums to reduce)
   const int* scol;   // packed signed columns (one coupling magnitude wmag) or null
   double wmag;
 };
@@ -132,7 +133,7 @@ __device__ __forceinline__ void ls_geometry_dev(int k, int* kp, int* kw, int* cp
 
 // The local search (or only the energies) of the problem's k candidates on the team.
 template <typename T, typename RP, typename GT>
-__device__ bool batch_ls(const BatchArgs& B, const BTeam& tm, const BProblem& pr, const BInstance& I, int k,
+__device__ __noinline__ bool batch_ls(const BatchArgs& B, const BTeam& tm, const BProblem& pr, const BInstance& I, int k,
                          const TeamPolicy& pol) {
   __shared__ LsArgs<T, RP, GT> L;
   const sa_batch_config& cfg = *B.cfg;
@@ -275,7 +276,7 @@ __device__ bool batch_problem(const BatchArgs& B, const BTeam& tm, int p, const 
         A.S.long_part = (T*)tm.long_part;
         A.S.scol = I.scol;
         A.S.wmag = (T)I.wmag;
-        A.long_rows = 1;
+        A.long_rows = I.long_rows;
         A.n_splits = 0;
         A.n = n;
         A.ldv = I.ldv;
@@ -776,6 +777,7 @@ int sa_batch_create(sa_batch** out, int32_t n_inst, sa_handle* const* inst, int3
     I.items = h->items;
     I.n_items = h->n_items;
     I.mc_base = h->mc_base;
+    I.long_rows = h->n_mc > 0;
     I.ld = h->ld;
     I.n = h->n;
     I.nnz = h->nnz;
