@@ -12,18 +12,21 @@
 //                      makes every gain and energy exact; double otherwise)
 //   flipm[i * kw + t]  candidates flipping at node i in the current pass
 // A pass: (D1) every selected node decides for every candidate from the pass-start state; wanting nodes
-// go to a queue (snapshot: flip); (D2) one warp per queued node (one CTA for a long row) finds the flips
-// that no neighbour blocks, flips the node's spin bits and appends (node, chunk) entries to a work
-// list; (U) one warp per entry scatters the field changes 2 J_ij s_i(new) to the neighbours of the chunk
-// for the flipped candidates (integer atomics: exact and order-independent). Arrays that other CTAs
-// change during the kernel (h, sb, flipm, the lists) are read with ld.global.cg: the per-SM L1 is not
-// coherent with their writes. After a pass every CTA reads the flip counts and applies the stopping
-// rules of flip_refinement / gpu_final_sweep (models/spectral_annealing.py:983-1112) itself.
+// go to a queue (snapshot: flip). In priority passes only nodes of which a field or a spin has changed
+// since their wanting mask was computed (U marks them in prio) read their fields; for the others the
+// mask still holds. (D2) one warp per queued node (one CTA for a long row) finds the flips that no
+// neighbour blocks, flips the node's spin bits and appends (node, chunk) entries to a work list; (U) one
+// warp per entry scatters the field changes 2 J_ij s_i(new) to the neighbours of the chunk for the
+// flipped candidates (integer atomics: exact and order-independent). Arrays that other CTAs change
+// during the kernel (h, sb, flipm, the lists) are read with ld.global.cg: the per-SM L1 is not coherent
+// with their writes. After a pass every CTA reads the flip counts and applies the stopping rules of
+// flip_refinement / gpu_final_sweep (models/spectral_annealing.py:983-1112) itself.
 //
 // What bounds it: chains of dependent loads (queue -> row -> neighbours -> their masks) over a few
 // thousand nodes, so the phases keep many loads in flight: batches of 8 field loads in D1, two row
 // entries per lane in D2, the entries of a chunk over the lanes in U, and two CTAs per SM. Search of 128
-// candidates on BA(2^16, m = 20): 16.4 -> 7.5 ms; of 40 on BA(200003, m = 15), integer weights: 15.5 -> 7.1 ms.
+// candidates on BA(2^16, m = 20): 16.4 -> 7.5 ms, and 5.9 ms with the masks of unchanged nodes kept; of 40
+// on BA(200003, m = 15), integer weights: 15.5 -> 7.1 -> 5.2 ms.
 #pragma once
 #include <cmath>
 #include <cstring>
@@ -193,6 +196,10 @@ __device__ __forceinline__ void row_fields(const LsArgs<VT, RP, GT>& A, long lon
 }
 
 constexpr int kLsLongRow = 512;   // entries above which a wanting node's row is checked by a whole CTA
+// Values of prio beside the ranks: a selected node's rank is below both "not selected" values.
+constexpr int kLsChanged = -1;            // set by U: a field or a spin of the node changed in the last pass
+constexpr int kLsSkipped = 0x7fffffff;    // not selected; its wanting mask is the current one
+constexpr int kLsSkippedOld = 0x7ffffffe; // not selected, and changed since its mask was computed
 constexpr int kLsSpread = 8;      // flips of a node up to which U spreads its entries over the lanes
 
 template <typename VT, typename RP, typename GT, class Pol>
@@ -243,6 +250,7 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
       }
       A.sb[i * A.kw + t] = word;
     }
+    if (A.priority) A.prio[i] = kLsChanged;
   }
   for (long long q = gtid; q < n * A.kp; q += nthreads) A.h[q] = GT(0);
   for (long long q = gtid; q < A.kp; q += nthreads) { A.ebefore[q] = 0; A.eafter[q] = 0; }
@@ -297,9 +305,13 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
     // D1: every selected node decides for every candidate from the pass-start state. Snapshot
     // passes flip the wanting pairs here; priority passes record the wanting masks and ranks.
     for (long long tile = gwarp * TN; tile < n; tile += nwarps * TN) {
-      bool selb = false;
-      int rk = 0x7fffffff;
+      bool selb = false, old = false;   // old: the node's wanting mask has to be computed again
       if (lane < TN && tile + lane < n) {
+        int rk = 0;
+        if (A.priority) {
+          const int was = __ldcg(A.prio + tile + lane);
+          old = was == kLsChanged || was == kLsSkippedOld;
+        }
         if (all_sel && !A.priority) {
           selb = true;
         } else {
@@ -307,11 +319,18 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
           selb = r < m;
           rk = (int)r;
         }
-        if (A.priority) A.prio[tile + lane] = selb ? rk : 0x7fffffff;
+        if (A.priority) A.prio[tile + lane] = selb ? rk : (old ? kLsSkippedOld : kLsSkipped);
       }
-      const uint32_t selmask = __ballot_sync(0xffffffffu, selb);
+      const uint32_t selmask = __ballot_sync(0xffffffffu, selb && (old || !A.priority));
       uint32_t want = 0u;   // nodes of the tile that want some candidate
+      if (A.priority) {
+        uint32_t w[4] = {0u, 0u, 0u, 0u};
+        if (selb && !old) ld_words(A.wm + (tile + lane) * kw, kw, w);
+        want = __ballot_sync(0xffffffffu, (w[0] | w[1] | w[2] | w[3]) != 0u);
+      }
       for (int f0 = 0; f0 < steps; f0 += 8) {
+        const int s0 = (f0 * inv_kw) >> 16, s1 = ((min(f0 + 8, steps) - 1) * inv_kw) >> 16;
+        if (!(selmask & ((2u << (s1 * ne + ne - 1)) - 1u) & ~((1u << (s0 * ne)) - 1u))) continue;
         uint32_t word[8];
         GT hv[8];
 #pragma unroll
@@ -328,13 +347,13 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
 #pragma unroll
         for (int q = 0; q < 8; ++q) {
           if (f0 + q >= steps) break;
-          const int s = ((f0 + q) * inv_kw) >> 16, t = f0 + q - s * kw;
-          const long long i = tile + s * ne + slot;
-          // (a node that is not selected has a zero field here)
+          const int s = ((f0 + q) * inv_kw) >> 16, t = f0 + q - s * kw, node = s * ne + slot;
+          const long long i = tile + node;
+          // (a node that is not read has a zero field here)
           const bool f = (32 * t + c < A.k) && (((word[q] >> c) & 1u) ? (hv[q] < GT(0)) : (hv[q] > GT(0)));
           const uint32_t bal = __ballot_sync(0xffffffffu, f);
           const uint32_t bits = cp == 32 ? bal : ((bal >> (slot * cp)) & cmask);
-          if (c == 0 && i < n) {
+          if (c == 0 && ((selmask >> node) & 1u)) {
             (A.priority ? A.wm : A.flipm)[i * kw + t] = bits;
             if (!A.priority && bits) A.sb[i * kw + t] = word[q] ^ bits;
           }
@@ -430,7 +449,7 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
         for (long long p = rs + lane; p < re; p += 64) {
           const bool two = p + 32 < re;
           const int j0 = __ldg(A.col + p), j1 = two ? __ldg(A.col + p + 32) : 0;
-          const int p0 = __ldcg(A.prio + j0), p1 = two ? __ldcg(A.prio + j1) : 0x7fffffff;
+          const int p0 = __ldcg(A.prio + j0), p1 = two ? __ldcg(A.prio + j1) : kLsSkipped;
           uint32_t w0[4] = {0u, 0u, 0u, 0u}, w1[4] = {0u, 0u, 0u, 0u};
           if (p0 < pi) ld_words(A.wm + (long long)j0 * kw, kw, w0);
           if (p1 < pi) ld_words(A.wm + (long long)j1 * kw, kw, w1);
@@ -471,9 +490,12 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
       ld_words(A.sb + i * kw, kw, S);
       const long long cb = rs + q * kChunk;
       const long long ce = (cb + kChunk < re) ? cb + kChunk : re;
+      if (A.priority && q == 0 && lane == 0) A.prio[i] = kLsChanged;
       if (__popc(F[0]) + __popc(F[1]) + __popc(F[2]) + __popc(F[3]) <= kLsSpread) {
         for (long long p = cb + lane; p < ce; p += 32) {
-          GT* hj = A.h + (long long)__ldg(A.col + p) * A.kp;
+          const int j = __ldg(A.col + p);
+          GT* hj = A.h + (long long)j * A.kp;
+          if (A.priority) A.prio[j] = kLsChanged;
           const GT v2 = GT(2) * coupling_as<GT>(__ldg(A.val + p));
 #pragma unroll
           for (int t = 0; t < 4; ++t) {
@@ -485,6 +507,8 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
         }
         continue;
       }
+      if (A.priority)
+        for (long long p = cb + lane; p < ce; p += 32) A.prio[__ldg(A.col + p)] = kLsChanged;
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         if (!((F[t] >> c) & 1u)) continue;

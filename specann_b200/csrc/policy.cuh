@@ -35,8 +35,8 @@ struct GridPolicy {
 // on the team's own GridSync (the control block's is not used); a team of one CTA uses
 // __syncthreads, with the epilogue run by the whole CTA.
 struct TeamPolicy {
-  // The team's first CTA runs the Ritz test for all: two CTAs share an SM's FP64 units here, and the
-  // redundant tests of two teams cost more than the barrier that hands the result over (a sweep of
+  // The team's first CTA runs the Ritz test for all: four CTAs share an SM's FP64 units here, and the
+  // redundant tests cost more than the barrier that hands the result over (a sweep of
   // twelve problems, n to 16,346: 104 ms with a test in every CTA, 100 ms with one a team).
   static constexpr bool kShareRitz = true;
   int b0, nb;

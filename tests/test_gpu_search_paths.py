@@ -51,3 +51,23 @@ def test_search_matches_oracle(hubs, k, semantics):
     assert np.array_equal(ea, np.asarray(ref.energies_after, dtype=np.float64))
     assert res.iterations == ref.iterations
     eng.close()
+
+
+# nodes that a pass leaves out keep their changes for a later one: small subsets, and a final sweep over
+# a part of the nodes
+@pytest.mark.parametrize("k, sub, final", [(3, 0.3, 1.0), (40, 0.3, 0.6), (70, 0.05, 0.5), (128, 0.6, 0.9)])
+def test_search_with_small_subsets(hubs, k, sub, final):
+    n = hubs.shape[0]
+    S = np.where(np.random.default_rng(k).random((k, n)) < 0.5, 1, -1).astype(np.int8)
+    eng = Engine(n, hubs.nnz, precision=32, ncv_max=4, max_candidates=k)
+    eng.upload_csr(hubs.indptr, hubs.indices, hubs.data.astype(np.float32))
+    for c in range(k):
+        eng.set_candidate(c, S[c])
+    kw = dict(seed=9, max_iterations=60, subset_fraction=sub, final_sweep_fraction=final, num_rounds=4)
+    eb, ea, res = eng.local_search(k, **kw)
+    ref = O.local_search(hubs, S, **kw)
+    got = np.stack([eng.candidate_spins(c, refined=True).cpu().numpy() for c in range(k)])
+    assert np.array_equal(got, ref.spins)
+    assert np.array_equal(ea, np.asarray(ref.energies_after, dtype=np.float64))
+    assert res.iterations == ref.iterations
+    eng.close()
