@@ -137,14 +137,17 @@ class Engine:
         """The column-panel SpMV is chosen when every SM holds one row block and, in FP32, rows average at
         least 16 entries (n >= 4096); in FP64, where a panel holds half the columns, rows average at least
         32 (n >= 65536). A Lanczos step in FP64, work list against panels: BA(2^16, 20) 46.5 against
-        42.9 us, BA(2^18, 20) 120 against 98 us, BA(150000, 10) 57.0 against 62.5 us."""
+        42.9 us, BA(2^18, 20) 120 against 98 us, BA(150000, 10) 57.0 against 62.5 us. A layout that takes
+        more than half of the free memory is left out in FP64, so that what fits without it still runs."""
         n_min, row_min = (4096, 16) if self.precision == 32 else (65536, 32)
         if self.n < n_min or self.nnz < row_min * self.n:
             return False
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
         try:
-            blocks = self.panel_plan()[1]
+            ws, blocks = self.panel_plan()
         except _lib.SpecAnnError:      # more panels than the layout supports
+            return False
+        if self.precision == 64 and 2 * ws > torch.cuda.mem_get_info(self.device)[0]:
             return False
         return blocks <= sms
 
