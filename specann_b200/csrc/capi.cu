@@ -145,6 +145,7 @@ __global__ void logdeg_kernel(const double* deg, long long n, double c, double* 
 template <typename T>
 __global__ void scale_kernel(const double* ld, long long n, double alpha, double half_log2_c, const T* x,
                              T* sigma, T* u) {
+  allow_dependent();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const double logD = (alpha == 0.0) ? 0.0 : alpha * (double)ld[i];
     const double logDc = fmax(logD, -39.86313713864835);
@@ -160,6 +161,7 @@ __global__ void __launch_bounds__(kThreads, 2) spmv_kernel(SpmvArgs<T, RP> S, in
   __shared__ SpmvSmem<T> ssp;
   const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nthreads = (long long)gridDim.x * blockDim.x;
+  wait_for_previous();
   spmv_items<T, RP, true>(S, u, gtid >> 5, nthreads >> 5, ssp, [&](long long r, T acc) {
     y[r] = rho * x[r] - sigma[r] * acc;
   });
@@ -577,12 +579,12 @@ int sa_spmv_scaled(sa_handle* h, double alpha, double rho, const void* x, void* 
     if (h->rp64) {
       S64 = SpmvArgs<float, long long>{(const long long*)h->rowptr, h->col, (const float*)h->val, h->items, h->n_items, h->mc_base, h->mc_count, (float*)h->long_part};
       set_policy(S64, h);
-      spmv_kernel<float, long long><<<gs, kThreads, 0, h->stream>>>(S64, h->group, (const float*)h->u, (const float*)x, (const float*)h->sigma, (float)rho, (float*)y);
+      SA_CUDA(launch_behind(spmv_kernel<float, long long>, gs, kThreads, 0, h->stream, S64, h->group, (const float*)h->u, (const float*)x, (const float*)h->sigma, (float)rho, (float*)y));
       count_launches(1);
     } else {
       S32 = SpmvArgs<float, int>{(const int*)h->rowptr, h->col, (const float*)h->val, h->items, h->n_items, h->mc_base, h->mc_count, (float*)h->long_part};
       set_policy(S32, h);
-      spmv_kernel<float, int><<<gs, kThreads, 0, h->stream>>>(S32, h->group, (const float*)h->u, (const float*)x, (const float*)h->sigma, (float)rho, (float*)y);
+      SA_CUDA(launch_behind(spmv_kernel<float, int>, gs, kThreads, 0, h->stream, S32, h->group, (const float*)h->u, (const float*)x, (const float*)h->sigma, (float)rho, (float*)y));
       count_launches(1);
     }
   } else {
@@ -591,12 +593,12 @@ int sa_spmv_scaled(sa_handle* h, double alpha, double rho, const void* x, void* 
     if (h->rp64) {
       SpmvArgs<double, long long> S{(const long long*)h->rowptr, h->col, (const double*)h->val, h->items, h->n_items, h->mc_base, h->mc_count, (double*)h->long_part};
       set_policy(S, h);
-      spmv_kernel<double, long long><<<gs, kThreads, 0, h->stream>>>(S, h->group, (const double*)h->u, (const double*)x, (const double*)h->sigma, rho, (double*)y);
+      SA_CUDA(launch_behind(spmv_kernel<double, long long>, gs, kThreads, 0, h->stream, S, h->group, (const double*)h->u, (const double*)x, (const double*)h->sigma, rho, (double*)y));
       count_launches(1);
     } else {
       SpmvArgs<double, int> S{(const int*)h->rowptr, h->col, (const double*)h->val, h->items, h->n_items, h->mc_base, h->mc_count, (double*)h->long_part};
       set_policy(S, h);
-      spmv_kernel<double, int><<<gs, kThreads, 0, h->stream>>>(S, h->group, (const double*)h->u, (const double*)x, (const double*)h->sigma, rho, (double*)y);
+      SA_CUDA(launch_behind(spmv_kernel<double, int>, gs, kThreads, 0, h->stream, S, h->group, (const double*)h->u, (const double*)x, (const double*)h->sigma, rho, (double*)y));
       count_launches(1);
     }
   }

@@ -265,4 +265,28 @@ __device__ __forceinline__ double block_sum(double v, double* scratch) {
 __device__ __forceinline__ long long rp_load(const int* rp, long long i) { return (long long)__ldg(rp + i); }
 __device__ __forceinline__ long long rp_load(const long long* rp, long long i) { return __ldg(rp + i); }
 
+// ---- a kernel launched behind the one that prepares its input ----------------------------------
+// The standalone operator is two kernels, the scaling of x and the SpMV. The SpMV's launch (its CTAs with
+// their shared memory) runs while the scaling still works; its threads wait here before they read
+// anything that the scaling writes. Without the launch attribute both calls do nothing. Operator at
+// n = 2^20 125.2 -> 119.9 us, at n = 150,001 with values in +-1..100 28.7 -> 26.7 us.
+__device__ __forceinline__ void allow_dependent() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_behind(void (*kernel)(KArgs...), int grid, int threads, int smem, cudaStream_t stream,
+                                 Args... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = stream;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...);
+}
+
 }  // namespace sa

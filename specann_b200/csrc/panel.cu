@@ -343,6 +343,7 @@ __global__ void __launch_bounds__(kThreads, 1) panel_spmv_kernel(PanelArgs P, co
   __shared__ unsigned long long bars[kPanelBufs];
   panel_init(bars);
   unsigned par = 0;
+  wait_for_previous();
   panel_spmv<T>(P, u, blockIdx.x, gridDim.x, psm, bars, par, err,
                 [&](long long r) { return RowInputs<T>{x[r], sigma[r]}; },
                 [&](long long r, T acc, const RowInputs<T>& in) { y[r] = rho * in.x - in.s * acc; });
@@ -387,13 +388,13 @@ int panel_spmv_launch(sa_handle* h, const void* u, const void* x, const void* si
   if (h->prec == 32) {
     auto k = panel_spmv_kernel<float, int>;
     PN_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem_bytes(4)));
-    k<<<grid, kThreads, panel_smem_bytes(4), h->stream>>>(P, (const float*)u, (const float*)x, (const float*)sigma,
-                                                          (float)rho, (float*)y, err);
+    PN_CUDA(launch_behind(k, grid, kThreads, panel_smem_bytes(4), h->stream, P, (const float*)u, (const float*)x, (const float*)sigma,
+                                                          (float)rho, (float*)y, err));
   } else {
     auto k = panel_spmv_kernel<double, int>;
     PN_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, panel_smem_bytes(8)));
-    k<<<grid, kThreads, panel_smem_bytes(8), h->stream>>>(P, (const double*)u, (const double*)x, (const double*)sigma,
-                                                          rho, (double*)y, err);
+    PN_CUDA(launch_behind(k, grid, kThreads, panel_smem_bytes(8), h->stream, P, (const double*)u, (const double*)x, (const double*)sigma,
+                                                          rho, (double*)y, err));
   }
   count_launches(1);
   PN_CUDA(cudaGetLastError());

@@ -70,3 +70,55 @@ def test_streamed_phases_on_few_rows_per_cta(n, precision):
 def test_basis_and_restart_sizes(ncv, keep):
     # a leading gap small enough to restart several times
     check(graphs.erdos_renyi(3000, 20 / 2999, seed=11), 64, 0.9, ncv=ncv, keep=keep, tol=1e-7)
+
+
+@pytest.mark.parametrize("n,m,precision,pays", [(65535, 20, 64, False), (65536, 20, 64, True), (65536, 10, 64, False),
+                                                (65536, 10, 32, True)])
+def test_panel_rule(n, m, precision, pays, monkeypatch):
+    J = graphs.barabasi_albert(n, m, seed=2)
+    eng = Engine(n, J.nnz, precision=precision, ncv_max=4, max_candidates=1)
+    eng.upload_csr(J.indptr, J.indices, J.data.astype(np.float32 if precision == 32 else np.float64))
+    assert eng.panels_pay() == pays
+    # FP64: a layout of more than half of the free memory is left out
+    monkeypatch.setattr(torch.cuda, "mem_get_info", lambda device=None: (2 * eng.panel_plan()[0] - 1, 1 << 37))
+    assert eng.panels_pay() == (pays and precision == 32)
+    eng.close()
+
+
+@pytest.mark.parametrize("layout", ["worklist", "panel"])
+@pytest.mark.parametrize("precision", [32, 64])
+def test_operator_calls_in_a_row_and_captured(layout, precision):
+    # each call's scaling writes the buffers that the call before still reads: nothing may overlap there
+    J = graphs.barabasi_albert(70003, 20, seed=6, couplings="pm1")
+    n, dt = J.shape[0], torch.float32 if precision == 32 else torch.float64
+    eng = Engine(n, J.nnz, precision=precision, ncv_max=4, max_candidates=1, stream=torch.cuda.Stream())
+    eng.upload_csr(J.indptr, J.indices, J.data.astype(np.float32 if precision == 32 else np.float64))
+    if layout == "panel":
+        eng.build_panels()
+    g = torch.Generator(device="cuda").manual_seed(3)
+    X = torch.randn(12, n, device="cuda", generator=g, dtype=dt)
+    alphas = np.linspace(0.0, 1.0, 12)
+    torch.cuda.synchronize()
+    alone = torch.empty_like(X)
+    for q in range(12):
+        eng.spmv(alphas[q], 1.001, X[q], alone[q])
+        torch.cuda.synchronize()
+    row = torch.zeros_like(X)
+    torch.cuda.synchronize()
+    for q in range(12):
+        eng.spmv(alphas[q], 1.001, X[q], row[q])
+    torch.cuda.synchronize()
+    assert torch.equal(row, alone)
+    captured = torch.zeros_like(X)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=eng.stream):
+        for q in range(12):
+            eng.spmv(alphas[q], 1.001, X[q], captured[q])
+    for _ in range(2):
+        captured.zero_()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(captured, alone)
+    assert eng.operator_status() == 0
+    eng.close()
