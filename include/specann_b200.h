@@ -462,6 +462,33 @@ int sa_spmv_scaled_noalloc(int64_t n, int64_t nnz, const int32_t* rowptr, const 
 int sa_barrier_selftest(int32_t blocks, int32_t expected, uint64_t spin_limit, void* scratch, size_t scratch_bytes,
                         int32_t* status, int32_t* passed_blocks, int32_t* epilogues, void* stream);
 
+/* Diagnostics of the streamed vector phases of the alpha solve (no reference counterpart): with `blocks`
+ * CTAs (1 .. the SM count), each over its share of the n rows, and `buffers` (1 .. 3) groups of tiles in
+ * flight,
+ *   u = w - a3 V[j] - b3 V[j-1] (the last term for j > 0 only);
+ *   dots[block * (j + 2) + k] = the block's part of V[k] . u for k <= j, and of u . u for k = j + 1;
+ *   w = u - sum_k h[k] V[k], then u = sigma w.
+ * V: j + 1 vectors, ldv >= n elements apart; V, w, u and sigma in the working precision on the device,
+ * 16-byte aligned and readable (zeros) to the next multiple of 16 bytes, as are rows of V; h (j + 1
+ * values) and dots are device doubles. withhold != 0: no wait for a copy can end, so that the first one
+ * runs out after spin_limit polls (1 .. 2^22). words: a device buffer of 1 + blocks integers.
+ * Synchronises `stream`. *status: SA_OK or SA_ERR_BARRIER_TIMEOUT; *passed_blocks: CTAs whose phases
+ * both returned success. */
+typedef struct {
+  int32_t precision, buffers, blocks, j;
+  int64_t n, ldv;
+  const void* V;
+  void *w, *u;
+  const void* sigma;
+  const double* h;
+  double* dots;
+  double a3, b3;
+  uint64_t spin_limit;
+  int32_t withhold, reserved;
+} sa_stream_test;
+int sa_stream_selftest(const sa_stream_test* p, int32_t* words, int32_t* status, int32_t* passed_blocks,
+                       void* stream);
+
 /* Version string of the library. */
 const char* sa_version(void);
 

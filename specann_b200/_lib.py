@@ -119,6 +119,13 @@ class BatchSummary(C.Structure):
                 ("energy_before", C.c_double * 128), ("energy_after", C.c_double * 128)]
 
 
+class StreamTest(C.Structure):
+    _fields_ = [("precision", C.c_int32), ("buffers", C.c_int32), ("blocks", C.c_int32), ("j", C.c_int32),
+                ("n", C.c_int64), ("ldv", C.c_int64), ("V", C.c_void_p), ("w", C.c_void_p), ("u", C.c_void_p),
+                ("sigma", C.c_void_p), ("h", C.c_void_p), ("dots", C.c_void_p), ("a3", C.c_double),
+                ("b3", C.c_double), ("spin_limit", C.c_uint64), ("withhold", C.c_int32), ("reserved", C.c_int32)]
+
+
 _I32P = C.POINTER(C.c_int32)
 
 SIGNATURES = {
@@ -136,6 +143,7 @@ SIGNATURES = {
     "sa_spmv_scaled": (C.c_int, [C.c_void_p, C.c_double, C.c_double, C.c_void_p, C.c_void_p]),
     "sa_set_spmv_policy": (C.c_int, [C.c_void_p, C.c_int32]),
     "sa_operator_status": (C.c_int, [C.c_void_p, _I32P]),
+    "sa_stream_selftest": (C.c_int, [C.POINTER(StreamTest), C.c_void_p, _I32P, _I32P, C.c_void_p]),
     "sa_barrier_selftest": (C.c_int, [C.c_int32, C.c_int32, C.c_uint64, C.c_void_p, C.c_size_t, _I32P, _I32P,
                                       _I32P, C.c_void_p]),
     "sa_panel_workspace_size": (C.c_int, [C.c_void_p, C.POINTER(C.c_size_t), C.POINTER(C.c_int32)]),

@@ -20,7 +20,7 @@ CSRC = PKG / "csrc"
 CUDA_LIB = "libspecann_b200.so"
 GRAPH_LIB = "libspecann_graphs.so"
 CU_SOURCES = ["capi.cu", "alpha.cu", "alpha_f32.cu", "alpha_f64.cu", "ls.cu", "batch.cu", "adjoint.cu", "noalloc.cu", "panel.cu", "split.cu", "coo.cu",
-              "guard.cu"]
+              "guard.cu", "selftest.cu"]
 HEADERS = ["common.cuh", "handle.cuh", "spmv.cuh", "policy.cuh", "alpha_body.cuh", "alpha_launch.cuh", "ls_body.cuh", "panel.cuh"]
 
 

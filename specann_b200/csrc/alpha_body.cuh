@@ -515,15 +515,6 @@ __device__ __forceinline__ void ld16(const T* p, T* out) {
   for (int r = 0; r < (int)(16 / sizeof(T)); ++r) out[r] = c[r];
 }
 
-// (from shared memory)
-template <typename T>
-__device__ __forceinline__ void lds16(const T* p, T* out) {
-  const typename Vec16<T>::type v = *reinterpret_cast<const typename Vec16<T>::type*>(p);
-  const T* c = reinterpret_cast<const T*>(&v);
-#pragma unroll
-  for (int r = 0; r < (int)(16 / sizeof(T)); ++r) out[r] = c[r];
-}
-
 template <typename T>
 __device__ __forceinline__ void st16(T* p, const T* in) {
   typename Vec16<T>::type v;
@@ -781,16 +772,16 @@ constexpr int kStreamVecs = 4;
 __host__ __device__ constexpr int stream_bufs(int elem) { return elem == 4 ? 3 : 2; }
 __host__ __device__ constexpr int stream_smem_bytes(int elem) { return stream_bufs(elem) * kStreamVecs * kStreamTile; }
 
-template <typename T>
+template <typename T, int kBufs>
 struct VecStream {
   static constexpr int VW = 16 / sizeof(T);
-  static constexpr int kBufs = stream_bufs(sizeof(T));
   static constexpr int kTileRows = kStreamTile / sizeof(T);
   static constexpr int kChunks = kStreamTile / (16 * kThreads);   // 16-byte chunks of a tile per thread
   char* smem;
   unsigned long long* bars;   // kBufs mbarriers of one arrival
   unsigned& par;              // their phase bits
   int* err;
+  unsigned long long spin_limit = kPanelSpinLimit;
   long long r0;               // first row, rows of the range and of a tile, number of tiles
   int rows, sub, tiles;
 
@@ -839,7 +830,7 @@ struct VecStream {
         const unsigned par0 = par;
         bool late = false;
         for (unsigned long long spins = 0; !mbar_try_wait(&bars[b], (par0 >> b) & 1u);)
-          if (++spins > kPanelSpinLimit) {
+          if (++spins > spin_limit) {
             late = true;
             break;
           }
@@ -853,7 +844,7 @@ struct VecStream {
             for (int q = k; q < k + kBufs && q < total; ++q) {
               const int qb = q % kBufs;
               for (unsigned long long spins = 0; !mbar_try_wait(&bars[qb], (par0 >> qb) & 1u);)
-                if (++spins > kPanelSpinLimit) break;
+                if (++spins > spin_limit) break;
             }
           }
           __syncthreads();
@@ -869,10 +860,10 @@ struct VecStream {
 
 // P2 streamed. The vectors in order: w, V[j], V[j-1], V[0], V[1], ..., V[j-2]; the first three give w',
 // which stays in registers for the tile.
-template <typename T>
-__device__ __forceinline__ bool stream_dots(VecStream<T>& S, const T* V, long long ldv, const T* w, T* u, int j, int pass2,
+template <typename T, int kBufs>
+__device__ __forceinline__ bool stream_dots(VecStream<T, kBufs>& S, const T* V, long long ldv, const T* w, T* u, int j, int pass2,
                                             double a3, double b3, double* red_all) {
-  constexpr int VW = VecStream<T>::VW, NC = VecStream<T>::kChunks;
+  constexpr int VW = VecStream<T, kBufs>::VW, NC = VecStream<T, kBufs>::kChunks;
   const int tid = tid_here(), lane = tid & 31;
   double* red = red_all + (tid >> 5) * kPartCols;
   for (int c = lane; c <= j + 1; c += 32) red[c] = 0.0;
@@ -892,11 +883,11 @@ __device__ __forceinline__ bool stream_dots(VecStream<T>& S, const T* V, long lo
 #pragma unroll
             for (int r = 0; r < VW; ++r) wv[r] = T(0);
             if (at < cnt) {
-              lds16(x + at, wv);
+              ld_filled16(x + at, wv);
               if (!pass2) {
                 T vj[VW], vm[VW];
-                lds16(x + kStreamTile / sizeof(T) + at, vj);
-                if (j > 0) lds16(x + 2 * (kStreamTile / sizeof(T)) + at, vm);
+                ld_filled16(x + kStreamTile / sizeof(T) + at, vj);
+                if (j > 0) ld_filled16(x + 2 * (kStreamTile / sizeof(T)) + at, vm);
 #pragma unroll
                 for (int r = 0; r < VW; ++r) {
                   double y = (double)wv[r] - a3 * (double)vj[r];
@@ -923,7 +914,7 @@ __device__ __forceinline__ bool stream_dots(VecStream<T>& S, const T* V, long lo
               const int at = (c * kThreads + tid) * VW;
               if (at < cnt) {
                 T vk[VW];
-                lds16(x + q * (kStreamTile / sizeof(T)) + at, vk);
+                ld_filled16(x + q * (kStreamTile / sizeof(T)) + at, vk);
 #pragma unroll
                 for (int r = 0; r < VW; ++r) acc[q] += (double)vk[r] * wd[c][r];
               }
@@ -941,10 +932,10 @@ __device__ __forceinline__ bool stream_dots(VecStream<T>& S, const T* V, long lo
 }
 
 // P3 streamed: the vectors in order src, sigma, V[0], ..., V[j]. Adds this thread's part of w . w to ww.
-template <typename T>
-__device__ __forceinline__ bool stream_update(VecStream<T>& S, const T* V, long long ldv, const T* src, const T* sigma,
+template <typename T, int kBufs>
+__device__ __forceinline__ bool stream_update(VecStream<T, kBufs>& S, const T* V, long long ldv, const T* src, const T* sigma,
                                               T* w, T* u, int j, const double* h, double& ww) {
-  constexpr int VW = VecStream<T>::VW, NC = VecStream<T>::kChunks;
+  constexpr int VW = VecStream<T, kBufs>::VW, NC = VecStream<T, kBufs>::kChunks;
   const int tid = tid_here();
   T wv[NC][VW], sg[NC][VW];
   double corr[NC][VW];
@@ -968,7 +959,7 @@ __device__ __forceinline__ bool stream_update(VecStream<T>& S, const T* V, long 
             const int at = (c * kThreads + tid) * VW;
             if (at < cnt) {
               T vk[VW];
-              lds16(x + q * (kStreamTile / sizeof(T)) + at, vk);
+              ld_filled16(x + q * (kStreamTile / sizeof(T)) + at, vk);
               if (g == 0 && q < 2) {
 #pragma unroll
                 for (int r = 0; r < VW; ++r) (q == 0 ? wv : sg)[c][r] = vk[r];
@@ -1412,8 +1403,8 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
         const double a3 = pass2 ? 0.0 : C->a[j], b3 = (pass2 || j == 0) ? 0.0 : C->b[j - 1];
         if constexpr (alpha_streams(kMode)) {
           extern __shared__ __align__(128) char stream_smem[];
-          VecStream<T> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
-          if (!stream_dots<T>(S, A.V, A.ldv, A.w, A.u, j, pass2, a3, b3, work.dots)) return;
+          VecStream<T, stream_bufs(sizeof(T))> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
+          if (!stream_dots(S, A.V, A.ldv, A.w, A.u, j, pass2, a3, b3, work.dots)) return;
         } else {
           lanczos_dots<T>(A.V, A.ldv, A.w, A.u, nvt, j, pass2, a3, b3, work.dots, (int)pol.tid(), (int)nthreads);
         }
@@ -1440,8 +1431,8 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
         double v[1] = {0.0};
         if constexpr (alpha_streams(kMode)) {
           extern __shared__ __align__(128) char stream_smem[];
-          VecStream<T> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
-          if (!stream_update<T>(S, A.V, A.ldv, src, A.sigma, A.w, A.u, j, C->h, v[0])) return;
+          VecStream<T, stream_bufs(sizeof(T))> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
+          if (!stream_update(S, A.V, A.ldv, src, A.sigma, A.w, A.u, j, C->h, v[0])) return;
         } else {
           v[0] = lanczos_update<T>(A.V, A.ldv, src, A.sigma, A.w, A.u, nvt, j, C->h, (int)pol.tid(), (int)nthreads);
         }
