@@ -767,10 +767,17 @@ __device__ __forceinline__ double lanczos_update(const T* V, long long ldv, cons
 // 30 KB. At n = 2^20 (20 vectors) the dots move 3.3 TB/s and the update 3.8 TB/s with the FP32 to FP64
 // conversions (16 a cycle and SM) next in line; one step's dots and update went from 73 to 52.5 us,
 // Ritz test and barriers included.
+// Buffers: three where the panels take as much shared memory anyway (FP32). Without panels two, since the
+// gathers of the work list and of the splits live on what is left to L1: with three (28 KB of L1) a step's
+// SpMV on BA(2^22, 10) took 900 us, with two (92 KB) 617 us, the vector phases 132 and 135 us; on BA(2^20, 4)
+// 105 and 70 us, and 48 and 46 us. Tiles of 8 KB with two buffers (156 KB of L1): SpMV 567 and 68 us, vector
+// phases 167 and 56 us.
 constexpr int kStreamTile = 16 * 1024;
 constexpr int kStreamVecs = 4;
-__host__ __device__ constexpr int stream_bufs(int elem) { return elem == 4 ? 3 : 2; }
-__host__ __device__ constexpr int stream_smem_bytes(int elem) { return stream_bufs(elem) * kStreamVecs * kStreamTile; }
+__host__ __device__ constexpr int stream_bufs(int elem, bool panels) { return panels && elem == 4 ? 3 : 2; }
+__host__ __device__ constexpr int stream_smem_bytes(int elem, bool panels) {
+  return stream_bufs(elem, panels) * kStreamVecs * kStreamTile;
+}
 
 template <typename T, int kBufs>
 struct VecStream {
@@ -1149,7 +1156,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
   __shared__ double sm[3 * NW];
   __shared__ double tot[kPartCols];   // totals of the last phase's partial sums
   __shared__ AlphaCtrl ctl;
-  __shared__ unsigned long long pbars[kPanelBufs], vbars[stream_bufs(sizeof(T))];
+  __shared__ unsigned long long pbars[kPanelBufs], vbars[stream_bufs(sizeof(T), alpha_panels(kMode))];
   double* const sq = work.restart;
   AlphaCtrl* const C = &ctl;     // this CTA's copy of the control block
   AlphaCtrl* const G = A.ctrl;   // barrier, flags and signature of the whole grid; the copy that is published
@@ -1168,7 +1175,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
   unsigned ppar = 0;   // phase bits of the panel barriers
   if (alpha_panels(kMode)) panel_init(pbars, kPanelBufs);
   unsigned vpar = 0;   // and of the vector streams'
-  if (alpha_streams(kMode)) panel_init(vbars, stream_bufs(sizeof(T)));
+  if (alpha_streams(kMode)) panel_init(vbars, stream_bufs(sizeof(T), alpha_panels(kMode)));
   PhaseSums<Pol, kPartCols> sums(pol, &G->gs, A.part, sm, tot);
   // one operator application (this thread's sum goes to f.acc); false on a timed-out wait
   auto apply = [&](RowStep<T>& f) -> bool {
@@ -1403,7 +1410,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
         const double a3 = pass2 ? 0.0 : C->a[j], b3 = (pass2 || j == 0) ? 0.0 : C->b[j - 1];
         if constexpr (alpha_streams(kMode)) {
           extern __shared__ __align__(128) char stream_smem[];
-          VecStream<T, stream_bufs(sizeof(T))> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
+          VecStream<T, stream_bufs(sizeof(T), alpha_panels(kMode))> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
           if (!stream_dots(S, A.V, A.ldv, A.w, A.u, j, pass2, a3, b3, work.dots)) return;
         } else {
           lanczos_dots<T>(A.V, A.ldv, A.w, A.u, nvt, j, pass2, a3, b3, work.dots, (int)pol.tid(), (int)nthreads);
@@ -1431,7 +1438,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
         double v[1] = {0.0};
         if constexpr (alpha_streams(kMode)) {
           extern __shared__ __align__(128) char stream_smem[];
-          VecStream<T, stream_bufs(sizeof(T))> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
+          VecStream<T, stream_bufs(sizeof(T), alpha_panels(kMode))> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
           if (!stream_update(S, A.V, A.ldv, src, A.sigma, A.w, A.u, j, C->h, v[0])) return;
         } else {
           v[0] = lanczos_update<T>(A.V, A.ldv, src, A.sigma, A.w, A.u, nvt, j, C->h, (int)pol.tid(), (int)nthreads);

@@ -92,7 +92,7 @@ int launch_alpha(sa_handle* h, const sa_alpha_params* p) {
   const void* kernel = alpha_kernel_of<T, RP>(mode);
   A.panel = alpha_panels(mode) ? panel_args(h) : PanelArgs{};
   const int dyn = std::max(alpha_panels(mode) ? panel_smem_bytes((int)sizeof(T)) : 0,
-                           alpha_streams(mode) ? stream_smem_bytes((int)sizeof(T)) : 0);
+                           alpha_streams(mode) ? stream_smem_bytes((int)sizeof(T), alpha_panels(mode)) : 0);
   if (dyn > 0) {
     // set on every launch: the attribute belongs to the current device
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn) !=

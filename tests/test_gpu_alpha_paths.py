@@ -122,3 +122,32 @@ def test_operator_calls_in_a_row_and_captured(layout, precision):
         assert torch.equal(captured, alone)
     assert eng.operator_status() == 0
     eng.close()
+
+
+def test_work_list_spmv_keeps_its_l1():
+    # the vector phases' shared memory comes out of the L1 that the gathers need: a step's SpMV against the
+    # standalone operator on the same work list (1.3 times as long; 1.9 times with only 28 KB of L1)
+    J = graphs.barabasi_albert(1 << 20, 4, seed=42, dtype=np.float32)
+    eng = Engine(J.shape[0], J.nnz, precision=32, ncv_max=33, max_candidates=1)
+    eng.upload_csr(J.indptr, J.indices, J.data)
+
+    def step():
+        rec = eng.alpha_solve(alpha=0.6, alpha_prev=0.6, rho=1.001, gershgorin=1.0, tol=1e-30, pred_tol=1e-3, maxiter=30,
+                              ncv=33, start_mode=_lib.SA_START_RANDOM, seed=7, stream_id=0, align=False)
+        return rec.phase_ms[1] / rec.iterations
+
+    x = torch.randn(J.shape[0], device="cuda")
+    y = torch.empty_like(x)
+
+    def operator(reps=10):
+        e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        e0.record()
+        for _ in range(reps):
+            eng.spmv(0.6, 1.001, x, y)
+        e1.record()
+        torch.cuda.synchronize()
+        return e0.elapsed_time(e1) / reps
+
+    step(), operator()
+    assert min(step() for _ in range(5)) < 1.6 * min(operator() for _ in range(5))
+    eng.close()
