@@ -452,15 +452,27 @@ int sa_spmv_scaled_noalloc(int64_t n, int64_t nnz, const int32_t* rowptr, const 
                            const float* val, double alpha, double rho, const float* x, float* y,
                            void* stream);
 
-/* Diagnostics of the bounded grid barrier that separates the phases of the persistent kernels (no
- * reference counterpart): one launch of `blocks` CTAs (1 .. the SM count) that meet at one barrier of
- * `expected` arrivals, each waiting at most spin_limit sleeps of ~64 ns (1 .. 2^25). scratch: a
+/* Diagnostics of the bounded grid barrier with an epilogue (the guarded search, the decisions of a batch
+ * team; no reference counterpart): one launch of `blocks` CTAs (1 .. the SM count) that meet at one barrier of
+ * `expected` arrivals, each waiting at most spin_limit polls of a sleep of ~64 ns (1 .. 2^25). scratch: a
  * caller-owned device buffer of at least 16 + 4 * blocks bytes, 16-byte aligned. Synchronises
  * `stream`. *status: the barrier's error word (SA_OK, or SA_ERR_BARRIER_TIMEOUT when a wait ran out,
  * e.g. with expected > blocks); *passed_blocks: CTAs whose barrier returned success; *epilogues:
  * CTAs that ran the last-arrival epilogue (1 on success, 0 when nobody arrives last). */
 int sa_barrier_selftest(int32_t blocks, int32_t expected, uint64_t spin_limit, void* scratch, size_t scratch_bytes,
                         int32_t* status, int32_t* passed_blocks, int32_t* epilogues, void* stream);
+
+/* The same for the barrier without an epilogue, at which the CTAs of an alpha solve, an adjoint, a local
+ * search or a batch team meet: one launch of `blocks` CTAs (1 .. the SM count) as a team of `expected`
+ * (>= blocks) goes through solves x meets barriers (1 .. 1000 each), with the team's counter at its
+ * value after first_epoch barriers. Waits end after spin_limit polls (1 .. 2^25, rounded up to a
+ * multiple of 64). scratch: a caller-owned device buffer of at least 32 + 4 * blocks bytes, 16-byte
+ * aligned. Synchronises `stream`. *status: SA_OK, or SA_ERR_BARRIER_TIMEOUT when a wait ran out (with
+ * expected > blocks); *passed_blocks: CTAs whose barriers all returned success; *early_blocks: CTAs that
+ * left a barrier before every CTA had come to it (0). */
+int sa_meet_selftest(int32_t blocks, int32_t expected, int32_t solves, int32_t meets, uint32_t first_epoch,
+                     uint64_t spin_limit, void* scratch, size_t scratch_bytes, int32_t* status,
+                     int32_t* passed_blocks, int32_t* early_blocks, void* stream);
 
 /* Diagnostics of the streamed vector phases of the alpha solve (no reference counterpart): with `blocks`
  * CTAs (1 .. the SM count), each over its share of the n rows, and `buffers` (1 .. 3) groups of tiles in

@@ -143,6 +143,8 @@ SIGNATURES = {
     "sa_spmv_scaled": (C.c_int, [C.c_void_p, C.c_double, C.c_double, C.c_void_p, C.c_void_p]),
     "sa_set_spmv_policy": (C.c_int, [C.c_void_p, C.c_int32]),
     "sa_operator_status": (C.c_int, [C.c_void_p, _I32P]),
+    "sa_meet_selftest": (C.c_int, [C.c_int32, C.c_int32, C.c_int32, C.c_int32, C.c_uint32, C.c_uint64, C.c_void_p,
+                                   C.c_size_t, _I32P, _I32P, _I32P, C.c_void_p]),
     "sa_stream_selftest": (C.c_int, [C.POINTER(StreamTest), C.c_void_p, _I32P, _I32P, C.c_void_p]),
     "sa_barrier_selftest": (C.c_int, [C.c_int32, C.c_int32, C.c_uint64, C.c_void_p, C.c_size_t, _I32P, _I32P,
                                       _I32P, C.c_void_p]),

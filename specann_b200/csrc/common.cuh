@@ -16,7 +16,9 @@ constexpr int kSegRows = 64;              // rows per short segment at most
 constexpr int kTileIt = kSegMax / 32;     // entries per lane of a tile
 constexpr int kNcvMax = 64;               // largest Lanczos basis
 constexpr int kDotBatch = 8;              // basis vectors per register batch in the dot phase
-constexpr unsigned long long kSpinLimit = 1ull << 25;   // ~2 s of 64 ns sleeps
+// Polls after which a barrier wait gives up. A poll is a round trip to L2 and, in grid_barrier_n, a sleep of
+// about 64 ns as well: some tens of seconds, well above what one CTA can make the others wait.
+constexpr unsigned long long kSpinLimit = 1ull << 25;
 constexpr int kMaxSplits = 8;             // column splits of an operator larger than L2 (split.cu)
 
 // One tile of the SpMV work list: at most kSegMax stored entries starting at e0.
@@ -50,7 +52,7 @@ __device__ __forceinline__ int ld_volatile_i32(const int* p) {
 
 // Barrier of `expected` co-resident CTAs (a cooperative grid, or a team of CTAs inside one),
 // with an epilogue run by the last CTA to arrive (the whole CTA runs it, after every other CTA's
-// writes are visible) before the others are released. Waits are bounded: after spin_limit sleeps
+// writes are visible) before the others are released. Waits are bounded: after spin_limit polls
 // the barrier records SA_ERR_BARRIER_TIMEOUT in gs->error and returns false, and a waiting CTA
 // also stops as soon as another CTA has recorded an error; the caller must then return. The
 // decision is taken by thread 0 and shared through shared memory, so the whole CTA returns the

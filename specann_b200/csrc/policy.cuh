@@ -61,12 +61,13 @@ struct TeamPolicy {
   __device__ __forceinline__ unsigned int first_epoch(GridSync*) const {
     return nb == 1 ? 0u : ld_volatile_u32(&gs->arrivals) / (unsigned int)nb;
   }
-  __device__ __forceinline__ bool meet(GridSync*, unsigned int& epoch) const {
+  __device__ __forceinline__ bool meet(GridSync*, unsigned int& epoch,
+                                       unsigned long long spin_limit = kSpinLimit) const {
     if (nb == 1) {
       __syncthreads();
       return true;
     }
-    return grid_arrive_wait(gs, (unsigned int)nb, epoch);
+    return grid_arrive_wait(gs, (unsigned int)nb, epoch, spin_limit);
   }
 };
 

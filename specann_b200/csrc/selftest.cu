@@ -1,5 +1,6 @@
-// Diagnostics of the streamed vector phases (sa_stream_selftest): one CTA each over its range of rows,
-// without the rest of a Lanczos step.
+// Diagnostics of parts of the persistent kernels by themselves: the barrier between their phases
+// (sa_meet_selftest), and the streamed vector phases (sa_stream_selftest), one CTA each over its range
+// of rows, without the rest of a Lanczos step.
 #include <algorithm>
 
 #include "alpha_body.cuh"
@@ -7,6 +8,27 @@
 namespace sa {
 
 namespace {
+
+// A team's solves of `meets` barriers each. tick counts the CTAs that came to a barrier, words[b] says
+// whether CTA b passed them all (bit 0) and whether it left one before every CTA had come (bit 1).
+__global__ void meet_selftest_kernel(GridSync* gs, unsigned int* tick, int nb, int solves, int meets,
+                                     unsigned long long spin_limit, int* words) {
+  const TeamPolicy pol{0, nb, gs};
+  bool ok = true, early = false;
+  unsigned int before = 0;   // CTAs that have to come before this barrier ends
+  for (int s = 0; s < solves && ok; ++s) {
+    unsigned int epoch = pol.first_epoch(gs);
+    for (int m = 0; m < meets && ok; ++m) {
+      if (threadIdx.x == 0) atomicAdd(tick, 1u);
+      before += (unsigned int)gridDim.x;
+      ok = pol.meet(gs, epoch, spin_limit);
+      if (ok && ld_volatile_u32(tick) < before) early = true;
+    }
+    __syncthreads();
+  }
+  const int any = __syncthreads_or(early);
+  if (threadIdx.x == 0) words[blockIdx.x] = (ok ? 1 : 0) | (any ? 2 : 0);
+}
 
 template <typename T, int kBufs>
 __global__ void __launch_bounds__(kThreads, 1) stream_selftest_kernel(const __grid_constant__ sa_stream_test P,
@@ -70,6 +92,44 @@ int run_stream_selftest(const sa_stream_test& P, unsigned long long spin_limit, 
 }  // namespace sa
 
 using namespace sa;
+
+extern "C" int sa_meet_selftest(int32_t blocks, int32_t expected, int32_t solves, int32_t meets, uint32_t first_epoch,
+                                uint64_t spin_limit, void* scratch, size_t scratch_bytes, int32_t* status,
+                                int32_t* passed_blocks, int32_t* early_blocks, void* stream) {
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    return SA_ERR_CUDA;
+  const size_t head = sizeof(GridSync) + 16;
+  if (blocks < 1 || blocks > sms || expected < blocks || solves < 1 || solves > 1000 || meets < 1 || meets > 1000 ||
+      spin_limit < 1 || spin_limit > kSpinLimit || !scratch || ((uintptr_t)scratch & 15) ||
+      scratch_bytes < head + 4 * (size_t)blocks || !status || !passed_blocks || !early_blocks)
+    return SA_ERR_INVALID_ARG;
+  cudaStream_t st = (cudaStream_t)stream;
+  GridSync gs = {};
+  gs.arrivals = first_epoch * (uint32_t)expected;
+  int* words = (int*)((char*)scratch + head);
+  int32_t host[1024];
+  if (cudaMemsetAsync(scratch, 0, head + 4 * (size_t)blocks, st) != cudaSuccess ||
+      cudaMemcpyAsync(scratch, &gs, sizeof(gs), cudaMemcpyHostToDevice, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    return SA_ERR_CUDA;
+  meet_selftest_kernel<<<blocks, 128, 0, st>>>((GridSync*)scratch, (unsigned int*)((char*)scratch + sizeof(GridSync)),
+                                               expected, solves, meets, spin_limit, words);
+  count_launches(1);
+  if (cudaGetLastError() != cudaSuccess ||
+      cudaMemcpyAsync(&gs, scratch, sizeof(gs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaMemcpyAsync(host, words, 4 * (size_t)blocks, cudaMemcpyDeviceToHost, st) != cudaSuccess ||
+      cudaStreamSynchronize(st) != cudaSuccess)
+    return SA_ERR_CUDA;
+  *status = gs.error;
+  *passed_blocks = *early_blocks = 0;
+  for (int b = 0; b < blocks; ++b) {
+    *passed_blocks += host[b] & 1;
+    *early_blocks += (host[b] >> 1) & 1;
+  }
+  return SA_OK;
+}
 
 extern "C" int sa_stream_selftest(const sa_stream_test* p, int32_t* words, int32_t* status, int32_t* passed_blocks,
                                   void* stream) {
