@@ -12,8 +12,11 @@ namespace {
 // A team's solves of `meets` barriers each. tick counts the CTAs that came to a barrier, words[b] says
 // whether CTA b passed them all (bit 0) and whether it left one before every CTA had come (bit 1).
 __global__ void meet_selftest_kernel(GridSync* gs, unsigned int* tick, int nb, int solves, int meets,
-                                     unsigned long long spin_limit, int* words) {
-  const TeamPolicy pol{0, nb, gs};
+                                     unsigned int first_epoch, unsigned long long spin_limit, int* words) {
+  __shared__ unsigned int s_epochs;
+  if (threadIdx.x == 0) s_epochs = first_epoch;
+  __syncthreads();
+  const TeamPolicy pol{0, nb, gs, &s_epochs};
   bool ok = true, early = false;
   unsigned int before = 0;   // CTAs that have to come before this barrier ends
   for (int s = 0; s < solves && ok; ++s) {
@@ -115,7 +118,7 @@ extern "C" int sa_meet_selftest(int32_t blocks, int32_t expected, int32_t solves
       cudaStreamSynchronize(st) != cudaSuccess)
     return SA_ERR_CUDA;
   meet_selftest_kernel<<<blocks, 128, 0, st>>>((GridSync*)scratch, (unsigned int*)((char*)scratch + sizeof(GridSync)),
-                                               expected, solves, meets, spin_limit, words);
+                                               expected, solves, meets, first_epoch, spin_limit, words);
   count_launches(1);
   if (cudaGetLastError() != cudaSuccess ||
       cudaMemcpyAsync(&gs, scratch, sizeof(gs), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
