@@ -528,8 +528,10 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
       const unsigned int flipped = __ballot_sync(0xffffffffu, cq > 0);
       if (lane == 0 && phase == 0) s_active[threadIdx.x >> 5] &= flipped;
       if (timer || pol.block() == 0) {
-        const int tot = __reduce_add_sync(0xffffffffu, cq);
-        if (lane == 0) atomicAdd(&s_total, (unsigned long long)tot);
+        // (32 candidates can flip more than 2^31 spins in a pass)
+        const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)cq & 0xffffu);
+        const unsigned hi = __reduce_add_sync(0xffffffffu, (unsigned)cq >> 16);
+        if (lane == 0) atomicAdd(&s_total, ((unsigned long long)hi << 16) + lo);
       }
     }
     const bool any = __syncthreads_or(cq > 0);

@@ -12,7 +12,7 @@ if not torch.cuda.is_available():
     pytest.skip("no CUDA device", allow_module_level=True)
 
 from oracle import specann_oracle as O  # noqa: E402
-from specann_b200 import graphs  # noqa: E402
+from specann_b200 import _lib, graphs  # noqa: E402
 from specann_b200.engine import Engine  # noqa: E402
 
 
@@ -70,4 +70,22 @@ def test_search_with_small_subsets(hubs, k, sub, final):
     assert np.array_equal(got, ref.spins)
     assert np.array_equal(ea, np.asarray(ref.energies_after, dtype=np.float64))
     assert res.iterations == ref.iterations
+    eng.close()
+
+
+def test_flip_total_beyond_32_bits():
+    # 2^25 antiferromagnetic pairs, all spins up in 32 candidates: a snapshot pass flips every spin of every
+    # candidate, 2^31 in all
+    n, k = 1 << 26, 32
+    eng = Engine(n, n, precision=32, ncv_max=2, max_candidates=k)
+    rowptr = torch.arange(n + 1, dtype=torch.int32, device="cuda")
+    col = torch.arange(n, dtype=torch.int32, device="cuda") ^ 1
+    eng.bind(rowptr, col, torch.full((n,), -1.0, device="cuda"))
+    up = torch.full((n // 32,), -1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for c in range(k):
+        _lib.check("sa_candidate_set", eng.lib.sa_candidate_set(eng.h, c, up.data_ptr()))
+    eb, ea, res = eng.local_search(k, max_iterations=1, subset_fraction=1.0, final_sweep_iters=0, semantics="snapshot")
+    assert res.total_flips == n * k
+    assert np.all(eb == n // 2) and np.all(ea == n // 2)
     eng.close()
