@@ -5,7 +5,12 @@
 
 namespace sa {
 
-constexpr int kLsCtas = 2;   // CTAs per SM: the phases wait for memory, not for the SM
+// CTAs per SM: the phases wait for memory, not for the SM, so two of them pay where there is work for both;
+// below, the second one only makes the barriers and the sums over CTAs longer. One and two CTAs in ms, by
+// n x (candidates rounded up): 5000 x 64 1.14 and 1.36, 20000 x 64 1.59 and 1.74, 40000 x 32 1.40 and 1.54,
+// 20000 x 128 2.50 and 2.23, 40000 x 64 2.26 and 2.01, 40000 x 128 3.54 and 3.17.
+constexpr int kLsCtas = 2;
+constexpr long long kLsTwoFrom = 1ll << 21;   // fields (n x candidates) from which two are launched
 
 template <typename VT, typename RP, typename GT>
 __global__ void __launch_bounds__(kThreads, kLsCtas) ls_kernel(LsArgs<VT, RP, GT> A) {
@@ -63,7 +68,8 @@ static int launch_ls(sa_handle* h, const sa_ls_params* p, char* ws, int kp, int 
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, (const void*)ls_kernel<VT, RP, GT>, kThreads, 0) != cudaSuccess ||
       per_sm < 1)
     return SA_ERR_CUDA;
-  cudaError_t e = cudaLaunchCooperativeKernel((const void*)ls_kernel<VT, RP, GT>, dim3(h->sm_count * std::min(per_sm, kLsCtas)),
+  const int ctas = h->n * kp >= kLsTwoFrom ? std::min(per_sm, kLsCtas) : 1;
+  cudaError_t e = cudaLaunchCooperativeKernel((const void*)ls_kernel<VT, RP, GT>, dim3(h->sm_count * ctas),
                                               dim3(kThreads), args, 0, h->stream);
   count_launches(1);
   return e == cudaSuccess ? SA_OK : SA_ERR_CUDA;

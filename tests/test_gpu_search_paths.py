@@ -73,6 +73,25 @@ def test_search_with_small_subsets(hubs, k, sub, final):
     eng.close()
 
 
+# one CTA per SM and two (from 2^21 fields on)
+@pytest.mark.parametrize("n", [16383, 16384])
+def test_search_on_either_side_of_the_second_cta(n):
+    J, k = graphs.barabasi_albert(n, 3, seed=8, couplings="pm1"), 128
+    S = np.where(np.random.default_rng(n).random((k, n)) < 0.5, 1, -1).astype(np.int8)
+    eng = Engine(n, J.nnz, precision=32, ncv_max=4, max_candidates=k)
+    eng.upload_csr(J.indptr, J.indices, J.data.astype(np.float32))
+    for c in range(k):
+        eng.set_candidate(c, S[c])
+    kw = dict(seed=2, max_iterations=4, num_rounds=1, final_sweep_iters=2)
+    eb, ea, res = eng.local_search(k, **kw)
+    ref = O.local_search(J, S, **kw)
+    got = np.stack([eng.candidate_spins(c, refined=True).cpu().numpy() for c in range(k)])
+    assert np.array_equal(got, ref.spins)
+    assert np.array_equal(ea, np.asarray(ref.energies_after, dtype=np.float64))
+    assert res.iterations == ref.iterations
+    eng.close()
+
+
 def test_flip_total_beyond_32_bits():
     # 2^25 antiferromagnetic pairs, all spins up in 32 candidates: a snapshot pass flips every spin of every
     # candidate, 2^31 in all
