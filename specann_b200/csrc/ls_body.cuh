@@ -160,7 +160,9 @@ __device__ __forceinline__ void ld_words(const uint32_t* p, int kw, uint32_t (&w
 }
 
 // Local fields of all candidates (cp = 32: lane c has candidate 32 t + c) for entries [e0, e1) of a row,
-// in entry order: the warp reads 32 entries at a time, then each entry's spin words, four in flight.
+// in entry order: the warp reads 32 entries at a time, then each entry's spin words, eight entries in
+// flight, or four of several words each. Eight instead of four: energies of 20
+// candidates on BA(3000, 10) 0.126 -> 0.111 ms, with real couplings 0.136 -> 0.123 ms.
 template <typename VT, typename RP, typename GT>
 __device__ __forceinline__ void row_fields(const LsArgs<VT, RP, GT>& A, long long e0, long long e1, GT (&acc)[4]) {
   const int lane = threadIdx.x & 31;
@@ -173,6 +175,23 @@ __device__ __forceinline__ void row_fields(const LsArgs<VT, RP, GT>& A, long lon
     if (lane < cnt) {
       j = __ldg(A.col + e + lane);
       v = coupling_as<GT>(__ldg(A.val + e + lane));
+    }
+    if (A.kw == 1) {
+      for (int g = 0; g < cnt; g += 8) {
+        uint32_t w[8];
+        GT vv[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int src = (g + q < cnt) ? g + q : 0;
+          const int jj = __shfl_sync(0xffffffffu, j, src);
+          vv[q] = __shfl_sync(0xffffffffu, v, src);
+          if (g + q < cnt) w[q] = __ldcg(A.sb + jj);
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (g + q < cnt) acc[0] += ((w[q] >> lane) & 1u) ? vv[q] : -vv[q];
+      }
+      continue;
     }
     for (int g = 0; g < cnt; g += 4) {
       uint32_t w[4][4];
