@@ -465,7 +465,7 @@ int sa_barrier_selftest(int32_t blocks, int32_t expected, uint64_t spin_limit, v
 /* The same for the barrier without an epilogue, at which the CTAs of an alpha solve, an adjoint, a local
  * search or a batch team meet: one launch of `blocks` CTAs (1 .. the SM count) as a team of `expected`
  * (>= blocks) goes through solves x meets barriers (1 .. 1000 each), with the team's counter at its
- * value after first_epoch barriers. Waits end after spin_limit polls (1 .. 2^25, rounded up to a
+ * value after first_epoch barriers of the first solve. Waits end after spin_limit polls (1 .. 2^25, rounded up to a
  * multiple of 64). scratch: a caller-owned device buffer of at least 32 + 4 * blocks bytes, 16-byte
  * aligned. Synchronises `stream`. *status: SA_OK, or SA_ERR_BARRIER_TIMEOUT when a wait ran out (with
  * expected > blocks); *passed_blocks: CTAs whose barriers all returned success; *early_blocks: CTAs that

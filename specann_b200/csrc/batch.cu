@@ -457,10 +457,8 @@ __device__ bool batch_problem(const BatchArgs& B, const BTeam& tm, int p, const 
 template <typename T, typename RP>
 __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(BatchArgs B) {
   __shared__ int s_team;
-  __shared__ unsigned int s_epochs;
   if (threadIdx.x == 0) {
     s_team = -1;
-    s_epochs = 0u;
     for (int t = 0; t < B.n_teams; ++t) {
       const int b0 = B.teams[t].b0, nb = B.teams[t].nb;
       if ((int)blockIdx.x >= b0 && (int)blockIdx.x < b0 + nb) { s_team = t; break; }
@@ -469,7 +467,7 @@ __global__ void __launch_bounds__(kBatchThreads, 4) batch_kernel(BatchArgs B) {
   __syncthreads();
   if (s_team < 0) return;
   const BTeam& tm = B.teams[s_team];
-  const TeamPolicy pol{tm.b0, tm.nb, B.team_gs + s_team, &s_epochs};
+  const TeamPolicy pol{tm.b0, tm.nb, B.team_gs + s_team};
   for (int q = 0; q < tm.count; ++q) {
     const int p = B.order[tm.first + q];
     if (!batch_problem<T, RP>(B, tm, p, pol)) {

@@ -41,7 +41,6 @@ struct TeamPolicy {
   static constexpr bool kShareRitz = true;
   int b0, nb;
   GridSync* gs;
-  unsigned int* epochs;   // this CTA's count of the team's barriers, in shared memory (0 with the counter)
   __device__ __forceinline__ long long tid() const { return (long long)(blockIdx.x - b0) * blockDim.x + tid_here(); }
   __device__ __forceinline__ long long nthr() const { return (long long)nb * blockDim.x; }
   __device__ __forceinline__ int block() const { return (int)blockIdx.x - b0; }
@@ -54,22 +53,23 @@ struct TeamPolicy {
       __syncthreads();
       return true;
     }
-    return grid_barrier_n(gs, (unsigned int)nb, e);
+    return grid_barrier_n(gs, (unsigned int)nb, [&] {
+      // (every CTA of the team has left its last meet)
+      if (threadIdx.x == 0) *((volatile unsigned int*)&gs->arrivals) = 0u;
+      e();
+    });
   }
   __device__ __forceinline__ bool sync(GridSync* g) const { return sync(g, [] {}); }
-  // The counter runs on from solve to solve, past 2^32 in a long run: the number of barriers cannot be had
-  // from it, so every CTA counts them. (meet writes the count behind its barrier, and a solve or a search
-  // is followed by sync before the next one reads it.)
-  __device__ __forceinline__ unsigned int first_epoch(GridSync*) const { return *((volatile unsigned int*)epochs); }
+  // A solve and a search are followed by sync, which sets the counter back (left to run on, it would pass
+  // 2^32 in a long run, and the number of barriers could not be had from it any more).
+  __device__ __forceinline__ unsigned int first_epoch(GridSync*) const { return 0; }
   __device__ __forceinline__ bool meet(GridSync*, unsigned int& epoch,
                                        unsigned long long spin_limit = kSpinLimit) const {
     if (nb == 1) {
       __syncthreads();
       return true;
     }
-    const bool ok = grid_arrive_wait(gs, (unsigned int)nb, epoch, spin_limit);
-    if (threadIdx.x == 0) *epochs = epoch;
-    return ok;
+    return grid_arrive_wait(gs, (unsigned int)nb, epoch, spin_limit);
   }
 };
 

@@ -13,14 +13,12 @@ namespace {
 // whether CTA b passed them all (bit 0) and whether it left one before every CTA had come (bit 1).
 __global__ void meet_selftest_kernel(GridSync* gs, unsigned int* tick, int nb, int solves, int meets,
                                      unsigned int first_epoch, unsigned long long spin_limit, int* words) {
-  __shared__ unsigned int s_epochs;
-  if (threadIdx.x == 0) s_epochs = first_epoch;
-  __syncthreads();
-  const TeamPolicy pol{0, nb, gs, &s_epochs};
+  const TeamPolicy pol{0, nb, gs};
   bool ok = true, early = false;
   unsigned int before = 0;   // CTAs that have to come before this barrier ends
   for (int s = 0; s < solves && ok; ++s) {
-    unsigned int epoch = pol.first_epoch(gs);
+    if (s > 0) ok = pol.sync(gs);
+    unsigned int epoch = s > 0 ? pol.first_epoch(gs) : first_epoch;
     for (int m = 0; m < meets && ok; ++m) {
       if (threadIdx.x == 0) atomicAdd(tick, 1u);
       before += (unsigned int)gridDim.x;

@@ -30,7 +30,8 @@ def test_no_cta_leaves_early(blocks):
 
 @pytest.mark.parametrize("blocks", [2, 3, 7, 100])
 def test_counter_past_its_end(blocks):
-    # a team's counter wraps after 2^32 arrivals, between two barriers of a solve or in the midst of one's
+    # a counter wraps after 2^32 arrivals, between two barriers of a solve or in the midst of one's, and the
+    # solves after it are counted anew
     for before in (0, 1, 18):
         first = ((1 << 32) // blocks - before) & 0xffffffff
         assert meet(blocks, blocks, solves=6, meets=5, first_epoch=first) == (_lib.SA_OK, _lib.SA_OK, blocks, 0)
