@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(kThreads, 2) spmv_kernel(SpmvArgs<T, RP> S, in
   const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nthreads = (long long)gridDim.x * blockDim.x;
   wait_for_previous();
-  spmv_items<T, RP, true>(S, u, gtid >> 5, nthreads >> 5, ssp, [&](long long r, T acc) {
+  spmv_items<T, RP>(S, u, gtid >> 5, nthreads >> 5, ssp, [&](long long r, T acc) {
     y[r] = rho * x[r] - sigma[r] * acc;
   });
 }

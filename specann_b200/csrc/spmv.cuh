@@ -18,11 +18,10 @@
 // neighbouring parts of col/val. Each warp runs a three-stage software pipeline: the descriptor of
 // the tile after next and the columns/values of the next tile are in flight while the current
 // tile's gathers and row sums run, so the HBM stream overlaps the gather latency.
-// col, val, rowptr and the work list are read through the read-only path. The gathered vector u
-// is read through the read-only path too when it is immutable for the whole kernel (kReadOnlyU,
-// the standalone operator); the persistent kernels rewrite u between phases, so there it is read
-// with ordinary L1-allocating loads, which see the writes of other CTAs because every phase
-// boundary is a grid barrier (gpu-scope fence by the waiting thread, then bar.sync).
+// col, val, rowptr and the work list are read through the read-only path. The gathered vector u is read
+// with ordinary L1-allocating loads: the persistent kernels rewrite u between phases (every phase
+// boundary is a barrier with a gpu-scope fence by the waiting thread, then bar.sync), and the standalone
+// operator may be launched while the kernel that writes u still runs (wait_for_previous).
 #pragma once
 #include "common.cuh"
 
@@ -91,23 +90,16 @@ __device__ __forceinline__ double ld_stream(const double* p, unsigned long long 
   return v;
 }
 
-// Gathers of the SpMV's input vector (read-only path when it is immutable for the kernel).
-__device__ __forceinline__ float ld_gather(const float* p, unsigned long long pol, bool nc) {
+// Gathers of the SpMV's input vector.
+__device__ __forceinline__ float gather(const float* u, int j, unsigned long long pol) {
   float v;
-  if (nc) asm volatile("ld.global.nc.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
-  else asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.f32 %0, [%1], %2;" : "=f"(v) : "l"(u + j), "l"(pol));
   return v;
 }
-__device__ __forceinline__ double ld_gather(const double* p, unsigned long long pol, bool nc) {
+__device__ __forceinline__ double gather(const double* u, int j, unsigned long long pol) {
   double v;
-  if (nc) asm volatile("ld.global.nc.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
-  else asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(v) : "l"(u + j), "l"(pol));
   return v;
-}
-
-template <bool kReadOnlyU, typename T>
-__device__ __forceinline__ T gather(const T* u, int j, unsigned long long pol) {
-  return ld_gather(u + j, pol, kReadOnlyU);
 }
 
 struct TileDesc {
@@ -161,7 +153,7 @@ __device__ __forceinline__ void load_tile(const SpmvArgs<T, RP>& S, const TileDe
 // fin(row, sum) is called exactly once per row with sum = sum_j val_ij * u_j (T arithmetic), by a warp
 // that follows from the work list alone; for a row of several chunks it is fin_any instead, called by
 // the warp that happens to finish last.
-template <typename T, typename RP, bool kReadOnlyU = false, int NW = kWarps, class Fin, class FinAny>
+template <typename T, typename RP, int NW = kWarps, class Fin, class FinAny>
 __device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u, long long gwarp,
                                            long long nwarps, SpmvSmem<T, NW>& sm, Fin&& fin, FinAny&& fin_any) {
   const int tid = tid_here();
@@ -188,7 +180,7 @@ __device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u,
 #pragma unroll
     for (int q = 0; q < kTileIt; ++q) {
       const int k = lane + 32 * q;
-      if (k < len) v[q] *= gather<kReadOnlyU>(u, ci[q], pol_gather);
+      if (k < len) v[q] *= gather(u, ci[q], pol_gather);
     }
     if (cur.row >= 0) {
       const int nr = item_nrows(cur.meta);
@@ -246,10 +238,10 @@ __device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u,
   }
 }
 
-template <typename T, typename RP, bool kReadOnlyU = false, int NW = kWarps, class Fin>
+template <typename T, typename RP, int NW = kWarps, class Fin>
 __device__ __forceinline__ void spmv_items(const SpmvArgs<T, RP>& S, const T* u, long long gwarp,
                                            long long nwarps, SpmvSmem<T, NW>& sm, Fin&& fin) {
-  spmv_items<T, RP, kReadOnlyU, NW>(S, u, gwarp, nwarps, sm, fin, fin);
+  spmv_items<T, RP, NW>(S, u, gwarp, nwarps, sm, fin, fin);
 }
 
 }  // namespace sa
