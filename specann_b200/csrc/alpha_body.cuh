@@ -1133,7 +1133,7 @@ __device__ __forceinline__ void items_pass(const SpmvArgs<T, RP>& S, const T* u,
     if (mode & 2) f.template fin<decltype(any)::value>(r, sum, f.pre(r));
     else __stcg(part + r, sum);
   };
-  spmv_items<T, RP, NW>(L, u, gwarp, nwarps, alpha_work<T, NW>().spmv,
+  spmv_items<T, RP, false, NW>(L, u, gwarp, nwarps, alpha_work<T, NW>().spmv,
                                [&](long long r, T s) { row(std::false_type{}, r, s); },
                                [&](long long r, T s) { row(std::true_type{}, r, s); });
   out.fixed = f.fixed;

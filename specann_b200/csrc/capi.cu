@@ -142,10 +142,11 @@ __global__ void logdeg_kernel(const double* deg, long long n, double c, double* 
 }
 
 // sigma = D^{-1/2} / sqrt(c) for this alpha and u = sigma * x.
-template <typename T>
+// kEarly: the SpMV's CTAs may come beside this kernel's, else as it ends (launch_behind).
+template <typename T, bool kEarly>
 __global__ void scale_kernel(const double* ld, long long n, double alpha, double half_log2_c, const T* x,
                              T* sigma, T* u) {
-  allow_dependent();
+  if (kEarly) allow_dependent();
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
     const double logD = (alpha == 0.0) ? 0.0 : alpha * (double)ld[i];
     const double logDc = fmax(logD, -39.86313713864835);
@@ -153,6 +154,7 @@ __global__ void scale_kernel(const double* ld, long long n, double alpha, double
     sigma[i] = s;
     u[i] = s * x[i];
   }
+  if (!kEarly) allow_dependent();
 }
 
 template <typename T, typename RP>
@@ -162,7 +164,7 @@ __global__ void __launch_bounds__(kThreads, 2) spmv_kernel(SpmvArgs<T, RP> S, in
   const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nthreads = (long long)gridDim.x * blockDim.x;
   wait_for_previous();
-  spmv_items<T, RP>(S, u, gtid >> 5, nthreads >> 5, ssp, [&](long long r, T acc) {
+  spmv_items<T, RP, true>(S, u, gtid >> 5, nthreads >> 5, ssp, [&](long long r, T acc) {
     y[r] = rho * x[r] - sigma[r] * acc;
   });
 }
@@ -563,16 +565,16 @@ int sa_spmv_scaled(sa_handle* h, double alpha, double rho, const void* x, void* 
   const int gs = h->sm_count * 2;
   if (h->panel_on || h->split_on) {
     if (h->prec == 32)
-      scale_kernel<float><<<g, 256, 0, h->stream>>>(h->ld, h->n, alpha, hl, (const float*)x, (float*)h->sigma, (float*)h->u);
+      (h->panel_on ? scale_kernel<float, true> : scale_kernel<float, false>)<<<g, 256, 0, h->stream>>>(h->ld, h->n, alpha, hl, (const float*)x, (float*)h->sigma, (float*)h->u);
     else
-      scale_kernel<double><<<g, 256, 0, h->stream>>>(h->ld, h->n, alpha, hl, (const double*)x, (double*)h->sigma, (double*)h->u);
+      (h->panel_on ? scale_kernel<double, true> : scale_kernel<double, false>)<<<g, 256, 0, h->stream>>>(h->ld, h->n, alpha, hl, (const double*)x, (double*)h->sigma, (double*)h->u);
     count_launches(1);
     SA_CUDA(cudaGetLastError());
     return h->panel_on ? panel_spmv_launch(h, h->u, x, h->sigma, rho, y) : split_spmv_launch(h, h->u, x, h->sigma, rho, y);
   }
   if (h->n_mc) SA_CUDA(cudaMemsetAsync(h->mc_count, 0, 4 * h->n_mc, h->stream));
   if (h->prec == 32) {
-    scale_kernel<float><<<g, 256, 0, h->stream>>>(h->ld, h->n, alpha, hl, (const float*)x, (float*)h->sigma, (float*)h->u);
+    scale_kernel<float, false><<<g, 256, 0, h->stream>>>(h->ld, h->n, alpha, hl, (const float*)x, (float*)h->sigma, (float*)h->u);
     count_launches(1);
     SpmvArgs<float, int> S32;
     SpmvArgs<float, long long> S64;
@@ -588,7 +590,7 @@ int sa_spmv_scaled(sa_handle* h, double alpha, double rho, const void* x, void* 
       count_launches(1);
     }
   } else {
-    scale_kernel<double><<<g, 256, 0, h->stream>>>(h->ld, h->n, alpha, hl, (const double*)x, (double*)h->sigma, (double*)h->u);
+    scale_kernel<double, false><<<g, 256, 0, h->stream>>>(h->ld, h->n, alpha, hl, (const double*)x, (double*)h->sigma, (double*)h->u);
     count_launches(1);
     if (h->rp64) {
       SpmvArgs<double, long long> S{(const long long*)h->rowptr, h->col, (const double*)h->val, h->items, h->n_items, h->mc_base, h->mc_count, (double*)h->long_part};

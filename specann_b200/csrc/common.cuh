@@ -271,7 +271,10 @@ __device__ __forceinline__ long long rp_load(const long long* rp, long long i) {
 // The standalone operator is two kernels, the scaling of x and the SpMV. The SpMV's launch (its CTAs with
 // their shared memory) runs while the scaling still works; its threads wait here before they read
 // anything that the scaling writes. Without the launch attribute both calls do nothing. Operator at
-// n = 2^20 125.2 -> 119.9 us, at n = 150,001 with values in +-1..100 28.7 -> 26.7 us.
+// n = 2^20 125.2 -> 119.9 us, at n = 150,001 with values in +-1..100 28.7 -> 26.7 us (panels, one CTA per SM:
+// launched as the scaling starts). The work list's CTAs, two per SM, are launched as it ends: earlier they
+// find room only beside the scaling's and are spread unevenly (BA(100000, 10) 20.9 us one after the
+// other, 22.2 launched early, 18.5 launched late; in FP64 26.7, 28.4 and 24.6).
 __device__ __forceinline__ void allow_dependent() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(kThreads, 2) split_spmv_kernel(SpmvArgs<T, RP>
   __shared__ SpmvSmem<T> ssp;
   const long long gtid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long nthreads = (long long)gridDim.x * blockDim.x;
-  spmv_items<T, RP>(S, u, gtid >> 5, nthreads >> 5, ssp, [&](long long r, T acc) {
+  spmv_items<T, RP, true>(S, u, gtid >> 5, nthreads >> 5, ssp, [&](long long r, T acc) {
     if (mode == 0) part[r] = acc;
     else if (mode == 1) part[r] = part[r] + acc;
     else y[r] = rho * x[r] - sigma[r] * (part[r] + acc);
