@@ -133,23 +133,52 @@ class Engine:
         check("sa_panel_workspace_size", self.lib.sa_panel_workspace_size(self.h, C.byref(nb), C.byref(blocks)))
         return int(nb.value), int(blocks.value)
 
-    def panels_pay(self) -> bool:
-        """The column-panel SpMV is chosen when every SM holds one row block and, in FP32, rows average at
-        least 16 entries (n >= 4096); in FP64, where a panel holds half the columns, rows average at least
-        32 (n >= 65536). A Lanczos step in FP64, work list against panels: BA(2^16, 20) 46.5 against
-        42.9 us, BA(2^18, 20) 120 against 98 us, BA(150000, 10) 57.0 against 62.5 us. A layout that takes
-        more than half of the free memory is left out in FP64, so that what fits without it still runs."""
-        n_min, row_min = (4096, 16) if self.precision == 32 else (65536, 32)
+    def panels_suit(self) -> bool:
+        """Whether the column-panel SpMV is the faster layout of the bound matrix: every SM holds one row
+        block and, in FP32, rows average at least 16 entries (n >= 4096). In FP64 (n >= 65536), where a panel
+        holds half the columns, rows average at least 32 entries, 36 below n = 80000, and 80 where the
+        couplings' values have to be streamed (more than one magnitude). A Lanczos step in FP64, work list
+        against panels: BA(2^16, 20) 48.9 and 45.9 us, BA(2^18, 20) 123 and 99 us; rows of 32 entries
+        at 2^16 40.6 and 42.4, at 81000 51.9 and 48.6 us; values in +-1..100, rows of 40 and 80 at 2^18 121 and
+        138, 260 and 180 us. The layout takes 2.5 ms to build at 2^16 and 4.9 ms at 2^18 (20 entries a
+        side), as much as 800 and 200 steps gain. A function of the problem and the device alone: the
+        layouts sum rows in different orders, so what else is in memory must not choose between them."""
+        return self._suited_panel_bytes() > 0
+
+    def _suited_panel_bytes(self) -> int:
+        """Bytes of the panel layout where it suits, else 0."""
+        if self.precision == 32:
+            n_min, row_min = 4096, 16
+        else:
+            one_magnitude = self.spmv_policy()["magnitude"] > 0.0
+            n_min, row_min = 65536, (36 if self.n < 80000 else 32) if one_magnitude else 80
         if self.n < n_min or self.nnz < row_min * self.n:
-            return False
-        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+            return 0
+        device = torch.cuda.get_device_properties(self.device)
         try:
             ws, blocks = self.panel_plan()
         except _lib.SpecAnnError:      # more panels than the layout supports
+            return 0
+        if blocks > device.multi_processor_count or (self.precision == 64 and 16 * ws > device.total_memory):
+            return 0
+        return ws
+
+    def panels_pay(self) -> bool:
+        """panels_suit, and in FP64 the layout takes at most half of the free memory."""
+        ws = self._suited_panel_bytes()
+        return ws > 0 and (self.precision == 32 or 2 * ws <= torch.cuda.mem_get_info(self.device)[0])
+
+    def build_suited_panels(self) -> bool:
+        """Build the panels if they suit; in FP64 the work list stays where there is no memory for them."""
+        if not self.panels_suit():
             return False
-        if self.precision == 64 and 2 * ws > torch.cuda.mem_get_info(self.device)[0]:
+        try:
+            self.build_panels()
+        except torch.cuda.OutOfMemoryError:
+            if self.precision == 32:
+                raise
             return False
-        return blocks <= sms
+        return True
 
     def build_panels(self) -> int:
         """Lay the bound matrix out for the column-panel SpMV (a device workspace owned by this

@@ -163,9 +163,8 @@ class SpectralAnnealing:
         self.tangent_tol = float(kwargs.pop("tangent_tol", 1e-2))
         # Ritz vectors kept by an implicit restart of the Lanczos basis (0: the kernel's default, 8)
         self.restart_keep = int(kwargs.pop("restart_keep", 0))
-        # operator layout: "auto" (column panels when rows average >= 16 entries, in FP64 >= 32, and the
-        # row blocks fit the SMs; L2 column splits when the gathered vector is larger than 48 MB; else
-        # the work list), "panel", "split" or "worklist"
+        # operator layout: "auto" (column panels where Engine.panels_suit, L2 column splits when the
+        # gathered vector is larger than 48 MB, else the work list), "panel", "split" or "worklist"
         self.spmv = str(kwargs.pop("spmv", "auto"))
         if self.spmv not in ("auto", "panel", "split", "worklist"):
             raise ValueError(f"spmv must be 'auto', 'panel', 'split' or 'worklist', got {self.spmv!r}")
@@ -271,11 +270,13 @@ class SpectralAnnealing:
         return self._sweep(eng, info, None, start_time)
 
     def _choose_operator(self, eng):
-        """Lay the operator out as column panels (spmv 'panel', or 'auto' when they pay) or keep
+        """Lay the operator out as column panels (spmv 'panel', or 'auto' where they suit) or keep
         the CSR work list."""
         self.operator_layout = "worklist"
-        if self.spmv == "panel" or (self.spmv == "auto" and eng.panels_pay()):
+        if self.spmv == "panel":
             eng.build_panels()
+            self.operator_layout = "panel"
+        elif self.spmv == "auto" and eng.build_suited_panels():
             self.operator_layout = "panel"
         elif self.spmv == "split" or (self.spmv == "auto" and eng.splits_pay()):
             eng.build_splits()
