@@ -8,7 +8,6 @@
 namespace sa {
 
 PanelArgs panel_args(const sa_handle* h);
-double panel_alg_bytes(const sa_handle* h);
 template <typename T, typename RP>
 SpmvArgs<T, RP> split_args(const sa_handle* h, int s);
 

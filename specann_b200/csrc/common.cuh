@@ -15,7 +15,6 @@ constexpr int kSegMax = 256;              // entries per short segment at most (
 constexpr int kSegRows = 64;              // rows per short segment at most
 constexpr int kTileIt = kSegMax / 32;     // entries per lane of a tile
 constexpr int kNcvMax = 64;               // largest Lanczos basis
-constexpr int kDotBatch = 8;              // basis vectors per register batch in the dot phase
 // Polls after which a barrier wait gives up. A poll is a round trip to L2 and, in grid_barrier_n, a sleep of
 // about 64 ns as well: some tens of seconds, well above what one CTA can make the others wait.
 constexpr unsigned long long kSpinLimit = 1ull << 25;

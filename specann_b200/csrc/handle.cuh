@@ -60,18 +60,9 @@ struct LsPass {
 // Control block of the local-search kernel.
 struct LsCtrl {
   GridSync gs;
-  int phase;                // 0 main loop, 1 final sweep, 2 done
   int it;                   // main-loop passes used
-  int round, sub;
   int final_passes;
-  int pad;
-  long long stream;         // selection stream of the current pass
-  long long m;              // nodes selected in the current pass
-  long long wl_count;       // work-list entries of the current pass
-  long long wq_count;       // wanting nodes of the current pass (priority passes)
   long long total_flips;
-  unsigned int active[4];   // candidates that have not yet had a pass without a flip
-  long long counts[128];    // flips per candidate in the current pass
   unsigned long long tph[4];  // ns by phase (set-up, decide, scatter, final)
   LsPass pass[3];
 };

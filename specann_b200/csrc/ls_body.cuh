@@ -546,7 +546,7 @@ __device__ __forceinline__ void ls_body(const LsArgs<VT, RP, GT>& A, const Pol& 
     if (threadIdx.x < 128) {
       const unsigned int flipped = __ballot_sync(0xffffffffu, cq > 0);
       if (lane == 0 && phase == 0) s_active[threadIdx.x >> 5] &= flipped;
-      if (timer || pol.block() == 0) {
+      if (pol.block() == 0) {
         // (32 candidates can flip more than 2^31 spins in a pass)
         const unsigned lo = __reduce_add_sync(0xffffffffu, (unsigned)cq & 0xffffu);
         const unsigned hi = __reduce_add_sync(0xffffffffu, (unsigned)cq >> 16);
