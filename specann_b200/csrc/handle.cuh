@@ -50,20 +50,21 @@ struct AlphaCtrl {
 
 // Counters of one local-search pass (three sets in turn: a pass counts in one, the next pass's is already
 // zero, and the last pass's may still be read).
-struct LsPass {
+struct alignas(128) LsPass {
   unsigned int wq;          // wanting nodes of ordinary rows (from the front of the queue)
   unsigned int lq;          // wanting nodes of long rows (from its back)
   unsigned long long wl;    // work-list entries
   int counts[128];          // flips per candidate
 };
 
-// Control block of the local-search kernel.
+// Control block of the local-search kernel. What is written during a search stands on other cache lines
+// than the counter that waiting CTAs poll: beside it, a search of 128 candidates took 2 % longer.
 struct LsCtrl {
   GridSync gs;
   int it;                   // main-loop passes used
   int final_passes;
   long long total_flips;
-  unsigned long long tph[4];  // ns by phase (set-up, decide, scatter, final)
+  alignas(128) unsigned long long tph[4];  // ns by phase (set-up, decide, scatter, final)
   LsPass pass[3];
 };
 
