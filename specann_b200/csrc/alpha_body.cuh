@@ -641,7 +641,7 @@ __device__ __forceinline__ double warp_sum_batch(double (&v)[N]) {
 // reorthogonalisation coefficients h_k = V_k . w' (k <= j) and of w' . w' in red[warp][0 .. j + 1].
 // Removing the dominant components explicitly first keeps the single Gram-Schmidt pass stable. w' goes to
 // u (whose gathers are over), so that w can be read by several groups of threads.
-template <typename T>
+template <typename T, bool kReadBack>
 __device__ __forceinline__ void lanczos_dots(const T* V, long long ldv, const T* w, T* u, long long nvt, int j, int pass2,
                                           double a3, double b3, double* red_all, int gtid, int nthreads) {
   constexpr int VW = 16 / sizeof(T);
@@ -652,7 +652,8 @@ __device__ __forceinline__ void lanczos_dots(const T* V, long long ldv, const T*
   for (int c = lane; c <= j + 1; c += 32) red[c] = 0.0;
   __syncwarp();
   // threads to spare: group g of them takes the batches g, g + groups, ... of basis vectors (each forms
-  // w' itself), so that a small problem waits for one batch of loads instead of all of them in turn
+  // w' itself), so that a small problem waits for one batch of loads instead of all of them in turn; with
+  // one group a thread can read the w' back that it has stored (kReadBack)
   constexpr int KB = 4;
   const int batches = (j + KB) / KB;
   const int nvw = ((int)nvt + 31) & ~31;
@@ -669,15 +670,16 @@ __device__ __forceinline__ void lanczos_dots(const T* V, long long ldv, const T*
       const long long i0 = (long long)iv * VW;
       // every load of the position before the first use or store, so that all are in flight
       T wv[VW], vj[VW], vm[VW], vk[KB][VW];
-      ld16(w + i0, wv);
-      if (!pass2) {
+      const bool form = !pass2 && (!kReadBack || kb == 0 || groups > 1);
+      ld16(form || pass2 ? w + i0 : u + i0, wv);
+      if (form) {
         ld16(Vj + i0, vj);
         ld16(Vm + i0, vm);
       }
 #pragma unroll
       for (int q = 0; q < KB; ++q)
         if (kb + q <= j) ld16(Vk + q * ldv + i0, vk[q]);
-      if (!pass2) {
+      if (form) {
 #pragma unroll
         for (int r = 0; r < VW; ++r) {
           double x = (double)wv[r] - a3 * (double)vj[r];
@@ -702,6 +704,50 @@ __device__ __forceinline__ void lanczos_dots(const T* V, long long ldv, const T*
       if (lane == 0) red[j + 1] = ww;
     }
   }
+}
+
+// P3 for a batch team, whose threads have many positions: one thread a position. The lanes' split of
+// lanczos_update, which then is one lane wide, left the update of 256 problems (n to 2^17, 145 teams) at 172 s
+// of team time; this takes 73 s and the sweep 7.0 instead of 8.2 s (with 8 vectors in flight 97 s and 7.3).
+template <typename T>
+__device__ __forceinline__ double lanczos_update_all(const T* V, long long ldv, const T* src, const T* sigma, T* w, T* u,
+                                                     long long nvt, int j, const double* h, int gtid, int nthreads) {
+  constexpr int VW = 16 / sizeof(T), KB = 4;
+  double ww = 0.0;
+  for (int iv = gtid; iv < (int)nvt; iv += nthreads) {
+    const long long i0 = (long long)iv * VW;
+    T wv[VW], sg[VW];
+    double corr[VW];
+    ld16(src + i0, wv);
+    ld16(sigma + i0, sg);
+#pragma unroll
+    for (int r = 0; r < VW; ++r) corr[r] = 0.0;
+    const T* Vk = V + i0;
+    for (int kb = 0; kb <= j; kb += KB, Vk += KB * ldv) {
+      T vk[KB][VW];
+#pragma unroll
+      for (int q = 0; q < KB; ++q)
+        if (kb + q <= j) ld16(Vk + q * ldv, vk[q]);
+#pragma unroll
+      for (int q = 0; q < KB; ++q) {
+        if (kb + q <= j) {
+          const double hk = h[kb + q];
+#pragma unroll
+          for (int r = 0; r < VW; ++r) corr[r] += hk * (double)vk[q][r];
+        }
+      }
+    }
+    T uv[VW];
+#pragma unroll
+    for (int r = 0; r < VW; ++r) {
+      wv[r] = (T)((double)wv[r] - corr[r]);
+      uv[r] = sg[r] * wv[r];
+      ww += (double)wv[r] * (double)wv[r];
+    }
+    st16(w + i0, wv);
+    st16(u + i0, uv);
+  }
+  return ww;
 }
 
 // P3: w = src - sum_k h_k V_k and u = sigma w; returns this thread's part of w . w. With threads to
@@ -1414,7 +1460,7 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
           VecStream<T, stream_bufs(sizeof(T), alpha_panels(kMode))> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
           if (!stream_dots(S, A.V, A.ldv, A.w, A.u, j, pass2, a3, b3, work.dots)) return;
         } else {
-          lanczos_dots<T>(A.V, A.ldv, A.w, A.u, nvt, j, pass2, a3, b3, work.dots, (int)pol.tid(), (int)nthreads);
+          lanczos_dots<T, Pol::kManyPositions>(A.V, A.ldv, A.w, A.u, nvt, j, pass2, a3, b3, work.dots, (int)pol.tid(), (int)nthreads);
         }
         __syncthreads();
         if (threadIdx.x <= j + 1) {
@@ -1442,7 +1488,10 @@ __device__ __forceinline__ void alpha_body(const AlphaArgs<T, RP>& A, const Pol&
           VecStream<T, stream_bufs(sizeof(T), alpha_panels(kMode))> S(stream_smem, vbars, vpar, &G->gs.error, nvt * VW, blk, nblk);
           if (!stream_update(S, A.V, A.ldv, src, A.sigma, A.w, A.u, j, C->h, v[0])) return;
         } else {
-          v[0] = lanczos_update<T>(A.V, A.ldv, src, A.sigma, A.w, A.u, nvt, j, C->h, (int)pol.tid(), (int)nthreads);
+          if (Pol::kManyPositions && 2 * nvt > nthreads)
+            v[0] = lanczos_update_all<T>(A.V, A.ldv, src, A.sigma, A.w, A.u, nvt, j, C->h, (int)pol.tid(), (int)nthreads);
+          else
+            v[0] = lanczos_update<T>(A.V, A.ldv, src, A.sigma, A.w, A.u, nvt, j, C->h, (int)pol.tid(), (int)nthreads);
         }
         sums.block_put(v);
       }

@@ -11,7 +11,8 @@ namespace sa {
 // GridPolicy: one problem on the whole grid. A cooperative grid separates phases on the control block's
 // GridSync; a grid that is one cluster (cluster = 1, only meet is used) by the cluster's barrier.
 struct GridPolicy {
-  static constexpr bool kShareRitz = false;   // every CTA runs the Ritz test itself
+  static constexpr bool kShareRitz = false;      // every CTA runs the Ritz test itself
+  static constexpr bool kManyPositions = false;  // positions of the vector phases are shared by lanes, or streamed
   int cluster = 0;
   __device__ __forceinline__ long long tid() const { return (long long)blockIdx.x * blockDim.x + tid_here(); }
   __device__ __forceinline__ long long nthr() const { return (long long)gridDim.x * blockDim.x; }
@@ -39,6 +40,7 @@ struct TeamPolicy {
   // redundant tests cost more than the barrier that hands the result over (a sweep of
   // twelve problems, n to 16,346: 104 ms with a test in every CTA, 100 ms with one a team).
   static constexpr bool kShareRitz = true;
+  static constexpr bool kManyPositions = true;   // a team of few CTAs has many positions a thread
   int b0, nb;
   GridSync* gs;
   __device__ __forceinline__ long long tid() const { return (long long)(blockIdx.x - b0) * blockDim.x + tid_here(); }
